@@ -935,7 +935,8 @@ int gwm_b200_create(const gwm_b200_grid_desc* grids, const gwm_b200_member_desc*
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return GWM_B200_ERR_NO_DEVICE;
   auto* c = new gwm_b200_ctx();
-  if (const char* t = std::getenv("GWM_B200_FAST_TILE_ROWS")) { const int r = std::atoi(t); c->fast_tile_rows = (r == 8 || r == 16) ? r : 0; }
+  const char* fast_rows = std::getenv("GWM_B200_FAST_TILE_ROWS");
+  if (fast_rows) { const int r = std::atoi(fast_rows); c->fast_tile_rows = (r == 8 || r == 16) ? r : 0; }
   cudaError_t e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return GWM_B200_ERR_CUDA; }
   c->stream = c->own_stream;
@@ -979,6 +980,15 @@ int gwm_b200_create(const gwm_b200_grid_desc* grids, const gwm_b200_member_desc*
       gwm_b200_destroy(c);
       return rc;
     }
+  }
+  // The TMA-fed kernels are the default where every member has its tensor maps: with columns
+  // split over CTAs they are the fastest form at every grid size (autotune can still choose).
+  bool tma = true;
+  for (const auto& M : c->m) tma = tma && !M.tmaps.empty();
+  if (tma) {
+    if (!fast_rows) c->fast_tile_rows = kFastTma;
+    c->slow_tile_rows = kSlowTma;
+    c->tracer_tile_rows = kTracerTma;
   }
   *out = c;
   return GWM_B200_OK;

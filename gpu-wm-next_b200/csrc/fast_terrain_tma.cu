@@ -28,6 +28,7 @@
 #include "dycore.cuh"
 #include "stencil.cuh"
 #include "tma.cuh"
+#include "zsplit.cuh"
 
 namespace gwmb {
 namespace {
@@ -91,14 +92,14 @@ struct TerrainCol {
 
 template <bool FIRST>
 __global__ void __launch_bounds__(fz::NT, 2)
-    k_fast_terrain_tma(const FastArgs a, const __grid_constant__ FastTerrainMaps m) {
+    k_fast_terrain_tma(const FastArgs a, const __grid_constant__ FastTerrainMaps m, ZSplit zs) {
   using namespace fz;
   using L = Slot<FIRST>;
   constexpr int O_RHO = L::O_RHO, O_TH = L::O_TH, O_Z = L::O_Z, O_P = L::O_P, O_DU = L::O_DU, O_DV = L::O_DV,
                 O_DW = L::O_DW, RW = L::RW, R0 = L::R0, C0 = L::C0, SLOT = L::SIZE;
   extern __shared__ unsigned char s_dyn[];
   __shared__ TerrainShared<FIRST> S;
-  float* const ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_dyn) + 127) & ~uintptr_t(127));
+  float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
 
   const Geom& g = a.g;
   const int nz = g.nz;
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(fz::NT, 2)
     S.abort[0] = 0;
     S.abort[1] = 0;
   }
-  if (blockIdx.x == 0 && blockIdx.y == 0 && a.clr_a)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && a.clr_a)
     for (int q = tid; q < nz; q += NT) { a.clr_a[q] = 0ull; a.clr_b[q] = 0ull; }
   __syncthreads();
 
@@ -140,11 +141,17 @@ __global__ void __launch_bounds__(fz::NT, 2)
   // of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
   int stall = -1;
   if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
+  // the CTA's planes are kb .. ke-1; it also loads the planes around them: the one below for
+  // its lowest Z face and dp/dz, the one above for its highest
+  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0, kl = min(ke, nz - 1);
+  if (stall >= 0) stall = kg + stall % (kl - kg + 1);  // a plane that this CTA loads
+  auto slot_of = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
   auto issue = [&](int kk) {
-    float* st = ring + (kk % NSLOT) * SLOT;
-    uint64_t* bar = &S.bar[kk % NSLOT];
-    const bool wface = kk + 1 < nz;
-    unsigned bytes = FIRST ? 3 * B_CELL : 2 * B_OWN + 2 * B_CELL + 2 * B_FACE + (wface ? B_OWN : 0u);
+    float* st = slot_of(kk);
+    uint64_t* bar = &S.bar[(kk - kg) % NSLOT];
+    const bool body = kk >= kb && kk < ke;
+    const bool wface = kk + 1 < nz && kk < ke;
+    unsigned bytes = FIRST ? 3 * B_CELL : B_OWN + 2 * B_CELL + (body ? B_OWN + 2 * B_FACE : 0u) + (wface ? B_OWN : 0u);
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(bar, bytes);
     if (kk == stall) return;  // failure-path testing: this plane's loads stay unissued
@@ -153,24 +160,25 @@ __global__ void __launch_bounds__(fz::NT, 2)
       tma_load_3d(st + O_TH, &m.th, i0 + kXOff - 4, j0, kk, bar);
     } else {
       tma_load_3d(st + O_RHO, &m.rho, i0 + kXOff, j0 + 1, kk, bar);
-      tma_load_3d(st + O_TH, &m.th, i0 + kXOff, j0 + 1, kk, bar);
       tma_load_3d(st + O_P, &m.p, i0 + kXOff - 4, j0, kk, bar);
-      tma_load_3d(st + O_DU, &m.du, i0 + kXOff, j0 + 1, kk, bar);
-      tma_load_3d(st + O_DV, &m.dv, i0 + kXOff, j0 + 1, kk, bar);
+      if (body) {
+        tma_load_3d(st + O_TH, &m.th, i0 + kXOff, j0 + 1, kk, bar);
+        tma_load_3d(st + O_DU, &m.du, i0 + kXOff, j0 + 1, kk, bar);
+        tma_load_3d(st + O_DV, &m.dv, i0 + kXOff, j0 + 1, kk, bar);
+      }
       if (wface) tma_load_3d(st + O_DW, &m.dw, i0 + kXOff, j0 + 1, kk + 1, bar);
     }
     tma_load_3d(st + O_Z, &m.z, i0 + kXOff - 4, j0, kk, bar);
   };
-  int issued = -1, waited = -1;
+  int issued = kg - 1, waited = kg - 1;
   auto wait_plane = [&](int kk, int epoch) {
-    if (!mbar_wait(&S.bar[kk % NSLOT], (kk / NSLOT) & 1)) {
+    if (!mbar_wait(&S.bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1)) {
       S.abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
     } else {
       waited = kk;  // a plane whose wait gave up stays in the drain below
     }
   };
-  auto slot_of = [&](int kk) { return ring + (kk % NSLOT) * SLOT; };
   // values of plane kk at derived-plane position (r, c)
   auto Pv = [&](int kk, int r, int c) {
     if constexpr (FIRST) return S.p[kk % 3][r][c];
@@ -221,30 +229,44 @@ __global__ void __launch_bounds__(fz::NT, 2)
     return c;
   };
 
-  if (tid == ISSUER) {
-    for (int kk = 0; kk < AHEAD && kk < nz; ++kk) { issue(kk); issued = kk; }
-  }
-  // the column reference at level 0 and the step's bottom face
+  if (tid == ISSUER)
+    for (int kk = kg; kk < kb + AHEAD && kk <= kl; ++kk) { issue(kk); issued = kk; }
+  // the column reference at the chunk's lowest level and the step's bottom face
   float prc0 = 0.f, rrc0 = 0.f, prc1 = 0.f, rrc1 = 0.f, bwz0 = 0.f, bwz1 = 0.f;
+  float dwc0 = 0.f, dwc1 = 0.f;  // increment at face k (face 0 never changes)
   if (own0) {
-    const int o = gidx(g, gi, gj0, 0);
+    const int o = gidx(g, gi, gj0, kb);
     prc0 = __ldg(a.col_pref + o); rrc0 = __ldg(a.col_rref + o);
-    if (final_step) bwz0 = __ldg(a.bw + o);
+    if (final_step && kb == 0) bwz0 = __ldg(a.bw + o);
   }
   if (own1) {
-    const int o = gidx(g, gi, gj1, 0);
+    const int o = gidx(g, gi, gj1, kb);
     prc1 = __ldg(a.col_pref + o); rrc1 = __ldg(a.col_rref + o);
-    if (final_step) bwz1 = __ldg(a.bw + o);
+    if (final_step && kb == 0) bwz1 = __ldg(a.bw + o);
   }
-  TerrainCol c0 = load_col(own0, gj0, 0), c1 = load_col(own1, gj1, 0);
-  wait_plane(0, 0);
-  derive_p(0);
-  if (nz > 1) {
-    wait_plane(1, 0);
-    derive_p(1);
+  TerrainCol c0 = load_col(own0, gj0, kb), c1 = load_col(own1, gj1, kb);
+  wait_plane(kg, kb);
+  derive_p(kg);
+  if (kb > 0) {  // the chunk's lowest Z face, from the plane below
+    wait_plane(kb, kb);
+    derive_p(kb);
+    const float* s0 = slot_of(kg);
+    const float* s1 = slot_of(kb);
+    auto face = [&](bool own, int row, int gj, float pru, float rru) {
+      if (!own) return 0.f;
+      const int o = gidx(g, gi, gj, kg), q = O_RHO + (row + R0) * RW + tx + C0;
+      return fp::wmom(FIRST ? 0.f : s0[O_DW + row * OBW + tx], Pv(kb, row + 1, tx + 1), pru, Pv(kg, row + 1, tx + 1),
+                      __ldg(a.col_pref + o), s0[q], __ldg(a.col_rref + o), s1[q], rru, __ldg(a.idz_f + o + g.plane),
+                      a.gravity, dtf);
+    };
+    dwc0 = face(own0, ty, gj0, prc0, rrc0);
+    dwc1 = face(own1, ty + RY, gj1, prc1, rrc1);
   }
-  derive_dz(0);
-  float dwc0 = 0.f, dwc1 = 0.f;  // increment at face k (face 0 never changes)
+  if (kb + 1 <= kl) {
+    wait_plane(kb + 1, kb);
+    derive_p(kb + 1);
+  }
+  derive_dz(kb);
   __syncthreads();
 
   // Interior tiles (full, away from every periodic edge ring and open side) run a copy
@@ -258,17 +280,17 @@ __global__ void __launch_bounds__(fz::NT, 2)
       if (IN) f[gidx(gg, i, j, kk)] = v;
       else store_tile(f, gg, o, i, j, kk, v, edge);
     };
-    for (int k = 0; k < nz; ++k) {
+    for (int k = kb; k < ke; ++k) {
       const int pb = k & 1;
       const float* st = slot_of(k);
       const float* stn = slot_of(k + 1);
       const TerrainCol n0 = load_col(o0, gj0, k + 1), n1 = load_col(o1, gj1, k + 1);
       // ---- dp/dz of plane k+1 (plane k+2 arrives first)
-      if (k + 2 < nz) {
+      if (k + 2 <= kl) {
         wait_plane(k + 2, k);
         derive_p(k + 2);
       }
-      if (k + 1 < nz) derive_dz(k + 1);
+      if (k + 1 < ke) derive_dz(k + 1);
       // ---- faces of plane k: K12/K13 horizontal momenta, K14 vertical momentum at face k+1
       auto P0 = [&](int r, int c) { return Pv(k, r, c); };
       auto Z0 = [&](int r, int c) { return st[O_Z + r * CBW + c + 3]; };
@@ -332,12 +354,12 @@ __global__ void __launch_bounds__(fz::NT, 2)
       __syncthreads();  // publishes dz(k+1), p(k+2), du(k), dv(k); the slot of plane k-1 is free
       if (S.abort[pb]) return true;
       if (tid == ISSUER) {
-        if (acc_mode && k > 0) {  // level sums of plane k-1 (warp totals published above)
+        if (acc_mode && k > kb) {  // level sums of plane k-1 (warp totals published above)
           long long sa = 0;
           for (int q = 0; q < NW; ++q) sa += S.red[pb ^ 1][q][0];
           acc_add(a.acc_a + k - 1, sa);
         }
-        if (k + AHEAD < nz) { issue(k + AHEAD); issued = k + AHEAD; }
+        if (k + AHEAD <= kl) { issue(k + AHEAD); issued = k + AHEAD; }
       }
       // ---- K15 density of plane k, K10 rho*theta, stores
       FxAcc sa;
@@ -383,16 +405,16 @@ __global__ void __launch_bounds__(fz::NT, 2)
   if (aborted) {
     // drain the tiles still in flight (bounded) before the CTA's shared memory goes away
     if (tid == ISSUER)
-      for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&S.bar[kk % NSLOT], (kk / NSLOT) & 1);
+      for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&S.bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1);
     return;
   }
   if (acc_mode) {
     __syncthreads();  // the last plane's warp totals
     if (tid == ISSUER) {
-      const int pb = (nz - 1) & 1;
+      const int pb = (ke - 1) & 1;
       long long sa = 0;
       for (int q = 0; q < NW; ++q) sa += S.red[pb][q][0];
-      acc_add(a.acc_a + nz - 1, sa);
+      acc_add(a.acc_a + ke - 1, sa);
     }
   }
 }
@@ -413,9 +435,11 @@ cudaError_t launch_fast_terrain_tma(const FastArgs& a, const FastTerrainMaps& m,
       (a.final_kind == 0 && !a.p_out) || (a.final_kind == 2 && (!a.bu || !a.bv || !a.bw)))
     return cudaErrorInvalidValue;
   const dim3 block(fz::TX, fz::RY);
-  const dim3 grid((a.g.nx + fz::TX - 1) / fz::TX, (a.g.ny + fz::TY - 1) / fz::TY);
-  if (first) k_fast_terrain_tma<true><<<grid, block, fz::dyn_smem<true>(), s>>>(a, m);
-  else k_fast_terrain_tma<false><<<grid, block, fz::dyn_smem<false>(), s>>>(a, m);
+  dim3 grid((a.g.nx + fz::TX - 1) / fz::TX, (a.g.ny + fz::TY - 1) / fz::TY);
+  const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 2, 3.0f);
+  grid.z = zs.chunks;
+  if (first) k_fast_terrain_tma<true><<<grid, block, fz::dyn_smem<true>(), s>>>(a, m, zs);
+  else k_fast_terrain_tma<false><<<grid, block, fz::dyn_smem<false>(), s>>>(a, m, zs);
   return cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@
 #include "dycore.cuh"
 #include "stencil.cuh"
 #include "tma.cuh"
+#include "zsplit.cuh"
 
 namespace gwmb {
 namespace {
@@ -134,13 +135,17 @@ __device__ __forceinline__ void fast_substep_setup(const FastArgs& a, const Fast
 // One tile (bx, by) of one acoustic substep: K9-K15 plane by plane over the TMA ring.
 // FIRST: the first substep of a stage (no increments in).  PIN: p' of the input (with its
 // ring) is loaded; otherwise (first substep only) it is derived from rho and theta.
+// The tile's planes are kb .. ke-1 of the column (all of them, or one chunk of a column
+// split over several CTAs).  A chunk that starts above the ground also loads plane kb-1,
+// from which it computes the increment of its lowest Z face, a face the chunk below
+// stores; every value is computed by the same operations in either form.
 // The ring's planes are counted across the tiles a CTA runs: plane kk of this tile is
-// ring plane base + kk (its slot and barrier phase).  stall >= 0 (failure-path tests
-// only) leaves that plane's loads unissued.  Returns true when a bounded wait gave up;
-// the tile's loads in flight are drained first.
+// ring plane base + kk - kg, kg the first plane loaded (its slot and barrier phase).
+// stall >= 0 (failure-path tests only) leaves the loads of a plane unissued.  Returns true
+// when a bounded wait gave up; the tile's loads in flight are drained first.
 template <bool FIRST, bool PIN>
-__device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, int bx, int by, FastShared& S,
-                                          float* ring, const FastTables& T, unsigned base, int stall) {
+__device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, int bx, int by, int kb, int ke,
+                                          FastShared& S, float* ring, const FastTables& T, unsigned base, int stall) {
   using namespace ft;
   using L = Slot<FIRST, PIN>;
   constexpr int O_RHO = L::O_RHO, O_TH = L::O_TH, O_DU = L::O_DU, O_DV = L::O_DV, O_DW = L::O_DW, O_P = L::O_P,
@@ -172,15 +177,21 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
   const int acc_mode = a.acc_off ? 0 : (a.final_kind == 0 ? 1 : 2);
   const bool hm = a.hmom != 0, dn = a.dens != 0;
 
-  // producer: all tiles of plane kk into slot (base + kk) % NSLOT, completing on its barrier
+  const int kg = kb > 0 ? kb - 1 : 0;  // first plane loaded
+  const int kl = min(ke, nz - 1);      // last plane loaded: the one above the chunk, if any
+  if (stall >= 0) stall = kg + stall % (kl - kg + 1);  // a plane that this tile loads
+  const unsigned rb = base - (unsigned)kg;  // ring plane of plane kk: rb + kk
+  // producer: all tiles of plane kk into slot (rb + kk) % NSLOT, completing on its barrier.
+  // The planes below and above the chunk carry only what the Z faces between need.
   auto issue = [&](int kk) {
-    float* st = ring + ((base + kk) % NSLOT) * slot;
-    uint64_t* bar = &S.bar[(base + kk) % NSLOT];
-    const bool wface = kk + 1 < nz;
-    unsigned bytes = (FIRST && !PIN) ? 2 * B_CELL : 2 * B_OWN;
-    if (!FIRST) bytes += 2 * B_FACE + (wface ? B_OWN : 0u);
+    float* st = ring + ((rb + kk) % NSLOT) * slot;
+    uint64_t* bar = &S.bar[(rb + kk) % NSLOT];
+    const bool body = kk >= kb && kk < ke;
+    const bool wface = kk + 1 < nz && kk < ke;
+    unsigned bytes = (FIRST && !PIN) ? 2 * B_CELL : (body ? 2 * B_OWN : B_OWN);
+    if (!FIRST) bytes += (body ? 2 * B_FACE : 0u) + (wface ? B_OWN : 0u);
     if (PIN) bytes += B_CELL;
-    if (final_step) bytes += 3 * B_OWN;
+    if (final_step && body) bytes += 3 * B_OWN;
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(bar, bytes);
     if (kk == stall) return;  // failure-path testing: this plane's loads stay unissued
@@ -189,23 +200,25 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
       tma_load_3d(st + O_TH, &m.th, i0 + kXOff - 4, j0, kk, bar);
     } else {  // owned cells
       tma_load_3d(st + O_RHO, &m.rho, i0 + kXOff, j0 + 1, kk, bar);
-      tma_load_3d(st + O_TH, &m.th, i0 + kXOff, j0 + 1, kk, bar);
+      if (body) tma_load_3d(st + O_TH, &m.th, i0 + kXOff, j0 + 1, kk, bar);
     }
     if (!FIRST) {
-      tma_load_3d(st + O_DU, &m.du, i0 + kXOff, j0 + 1, kk, bar);
-      tma_load_3d(st + O_DV, &m.dv, i0 + kXOff, j0 + 1, kk, bar);
+      if (body) {
+        tma_load_3d(st + O_DU, &m.du, i0 + kXOff, j0 + 1, kk, bar);
+        tma_load_3d(st + O_DV, &m.dv, i0 + kXOff, j0 + 1, kk, bar);
+      }
       if (wface) tma_load_3d(st + O_DW, &m.dw, i0 + kXOff, j0 + 1, kk + 1, bar);
     }
     if (PIN) tma_load_3d(st + O_P, &m.p, i0 + kXOff - 4, j0, kk, bar);
-    if (final_step) {
+    if (final_step && body) {
       tma_load_3d(st + O_BU, &m.bu, i0 + kXOff, j0 + 1, kk, bar);
       tma_load_3d(st + O_BV, &m.bv, i0 + kXOff, j0 + 1, kk, bar);
       tma_load_3d(st + O_BW, &m.bw, i0 + kXOff, j0 + 1, kk + 1, bar);
     }
   };
-  int issued = -1, waited = -1;  // planes issued / waited for (producer bookkeeping)
+  int issued = kg - 1, waited = kg - 1;  // planes issued / waited for (producer bookkeeping)
   auto wait_plane = [&](int kk, int epoch) {
-    if (!mbar_wait(&S.bar[(base + kk) % NSLOT], ((base + kk) / NSLOT) & 1)) {
+    if (!mbar_wait(&S.bar[(rb + kk) % NSLOT], ((rb + kk) / NSLOT) & 1)) {
       S.abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
     } else {
@@ -218,25 +231,44 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
     return eos_pprime_ref(rho, fp::mul(rho, th), T.binv[kk], T.bpr[kk]);
   };
   auto plane_p = [&](int kk) {
-    const float* st = ring + ((base + kk) % NSLOT) * slot;
+    const float* st = ring + ((rb + kk) % NSLOT) * slot;
     float(*sp)[TX + 2] = S.p[kk & 1];
     if (own0) sp[ty + 1][tx + 1] = cell_p(st, ty + 1, tx + 1, kk);
     if (own1) sp[ty + RY + 1][tx + 1] = cell_p(st, ty + RY + 1, tx + 1, kk);
     if (role >= 0) sp[hr][hc] = cell_p(st, hr, hc, kk);
   };
 
-  if (tid == ISSUER) {
-    issue(0);
-    issued = 0;
-    for (int kk = 1; kk < AHEAD && kk < nz; ++kk) { issue(kk); issued = kk; }
-  }
-  wait_plane(0, 0);
-  if (FIRST && !PIN) plane_p(0);
+  if (tid == ISSUER)
+    for (int kk = kg; kk < kb + AHEAD && kk <= kl; ++kk) { issue(kk); issued = kk; }
+  // K14 vertical momentum increment at face kk+1 of an owned cell (row of the tile), from
+  // p' of planes kk, kk+1 and the increment before the substep
+  auto face_w = [&](int kk, int row, float pc, float pn, float dw) {
+    const float* s0 = ring + ((rb + kk) % NSLOT) * slot;
+    const float* s1 = ring + ((rb + kk + 1) % NSLOT) * slot;
+    const int o = O_RHO + (row + R0) * RW + tx + C0;
+    return fp::wmom(dw, pn, T.pref[kk + 1], pc, T.pref[kk], s0[o], T.rref[kk], s1[o], T.rref[kk + 1], T.idzf[kk + 1],
+                    a.gravity, dtf);
+  };
   float dwc0 = 0.f, dwc1 = 0.f;  // increment at face k (face 0 never changes)
   float bwz0 = 0.f, bwz1 = 0.f;  // base momentum at face 0 (last substep of the step)
-  if (final_step) {
-    if (own0) bwz0 = __ldg(a.bw + gidx(g, gi, gj0, 0));
-    if (own1) bwz1 = __ldg(a.bw + gidx(g, gi, gj1, 0));
+  if (kb > 0) {  // the chunk's lowest Z face, from the plane below
+    wait_plane(kg, kb);
+    wait_plane(kb, kb);
+    const float* s0 = ring + ((rb + kg) % NSLOT) * slot;
+    const float* s1 = ring + ((rb + kb) % NSLOT) * slot;
+    if (FIRST && !PIN) { plane_p(kg); plane_p(kb); }
+    auto P = [&](const float* st, int kk, int row) {
+      return PIN ? st[O_P + (row + 1) * CBW + tx + 4] : S.p[kk & 1][row + 1][tx + 1];
+    };
+    dwc0 = face_w(kg, ty, P(s0, kg, ty), P(s1, kb, ty), FIRST ? 0.f : s0[O_DW + ty * OBW + tx]);
+    dwc1 = face_w(kg, ty + RY, P(s0, kg, ty + RY), P(s1, kb, ty + RY), FIRST ? 0.f : s0[O_DW + (ty + RY) * OBW + tx]);
+  } else {
+    wait_plane(0, 0);
+    if (FIRST && !PIN) plane_p(0);
+    if (final_step) {
+      if (own0) bwz0 = __ldg(a.bw + gidx(g, gi, gj0, 0));
+      if (own1) bwz1 = __ldg(a.bw + gidx(g, gi, gj1, 0));
+    }
   }
   __syncthreads();
 
@@ -253,10 +285,10 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
       if (IN) f[gidx(gg, i, j, kk)] = v;
       else store_tile(f, gg, o, i, j, kk, v, edge);
     };
-    for (int k = 0; k < nz; ++k) {
+    for (int k = kb; k < ke; ++k) {
       const int pb = k & 1;
-      const float* st = ring + ((base + k) % NSLOT) * slot;
-      const float* stn = ring + ((base + k + 1) % NSLOT) * slot;
+      const float* st = ring + ((rb + k) % NSLOT) * slot;
+      const float* stn = ring + ((rb + k + 1) % NSLOT) * slot;
       // ---- pressure perturbation of plane k+1 (its tiles were issued a plane ago)
       if (k + 1 < nz) {
         wait_plane(k + 1, k);
@@ -308,23 +340,19 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
       const float rc0 = st[O_RHO + (ty + R0) * RW + tx + C0], rc1 = st[O_RHO + (ty + RY + R0) * RW + tx + C0];
       float wn0 = dw0, wn1 = dw1;
       if (k + 1 < nz) {
-        const float prl = T.pref[k], pru = T.pref[k + 1], rrl = T.rref[k], rru = T.rref[k + 1];
-        const float idzf = T.idzf[k + 1];
-        const float pn0 = P1(ty + 1, tx + 1), pn1 = P1(ty + RY + 1, tx + 1);
-        const float rn0 = stn[O_RHO + (ty + R0) * RW + tx + C0], rn1 = stn[O_RHO + (ty + RY + R0) * RW + tx + C0];
-        wn0 = fp::wmom(dw0, pn0, pru, pc0, prl, rc0, rrl, rn0, rru, idzf, a.gravity, dtf);
-        wn1 = fp::wmom(dw1, pn1, pru, pc1, prl, rc1, rrl, rn1, rru, idzf, a.gravity, dtf);
+        wn0 = face_w(k, ty, pc0, P1(ty + 1, tx + 1), dw0);
+        wn1 = face_w(k, ty + RY, pc1, P1(ty + RY + 1, tx + 1), dw1);
       }
       __syncthreads();  // publishes s_p(k+1), s_du(k), s_dv(k); the slot of plane k-1 is free
       if (S.abort[pb]) return true;
       if (tid == ISSUER) {
-        if (acc_mode && k > 0) {  // level sums of plane k-1 (warp totals published above)
+        if (acc_mode && k > kb) {  // level sums of plane k-1 (warp totals published above)
           long long sa = 0, sb = 0;
           for (int q = 0; q < NW; ++q) { sa += S.red[pb ^ 1][q][0]; sb += S.red[pb ^ 1][q][1]; }
           acc_add(a.acc_a + k - 1, sa);
           if (acc_mode == 1) acc_add(a.acc_b + k - 1, sb);
         }
-        if (k + AHEAD < nz) { issue(k + AHEAD); issued = k + AHEAD; }
+        if (k + AHEAD <= kl) { issue(k + AHEAD); issued = k + AHEAD; }
       }
       // ---- K15 density of plane k, K10 rho*theta, stores
       const float idzc = T.idzc[k];
@@ -398,16 +426,16 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
     // drain the tiles still in flight (bounded) before the CTA's shared memory goes away
     if (tid == ISSUER)
       for (int kk = waited + 1; kk <= issued; ++kk)
-        mbar_wait(&S.bar[(base + kk) % NSLOT], ((base + kk) / NSLOT) & 1);
+        mbar_wait(&S.bar[(rb + kk) % NSLOT], ((rb + kk) / NSLOT) & 1);
     return true;
   }
   __syncthreads();  // the last plane's warp totals; every thread is done with the tile
   if (acc_mode && tid == ISSUER) {  // level sums of the last plane
-    const int pb = (nz - 1) & 1;
+    const int pb = (ke - 1) & 1;
     long long sa = 0, sb = 0;
     for (int q = 0; q < NW; ++q) { sa += S.red[pb][q][0]; sb += S.red[pb][q][1]; }
-    acc_add(a.acc_a + nz - 1, sa);
-    if (acc_mode == 1) acc_add(a.acc_b + nz - 1, sb);
+    acc_add(a.acc_a + ke - 1, sa);
+    if (acc_mode == 1) acc_add(a.acc_b + ke - 1, sb);
   }
   return false;
 }
@@ -430,18 +458,20 @@ __device__ __forceinline__ int fast_stall_plane(const FastArgs& a) {
   return -1;
 }
 
-// One acoustic substep: one CTA per tile.
+// One acoustic substep: one CTA per tile and chunk of levels.
 template <bool FIRST, bool PIN>
-__global__ void __launch_bounds__(ft::NT, 3) k_fast_tma(const FastArgs a, const __grid_constant__ FastMaps m) {
+__global__ void __launch_bounds__(ft::NT, 3) k_fast_tma(const FastArgs a, const __grid_constant__ FastMaps m,
+                                                        ZSplit zs) {
   extern __shared__ unsigned char s_dyn[];
   __shared__ FastShared S;
   using L = ft::Slot<FIRST, PIN>;
   const int slot = a.final_kind == 2 ? L::LONG : L::SHORT;
-  float* const ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_dyn) + 127) & ~uintptr_t(127));
+  float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
   const FastTables T = fast_tables(ring, slot, a.g.nz);
   fast_cta_init(S);
-  fast_substep_setup(a, T, blockIdx.x == 0 && blockIdx.y == 0);
-  fast_tile<FIRST, PIN>(a, m, blockIdx.x, blockIdx.y, S, ring, T, 0u, fast_stall_plane(a));
+  fast_substep_setup(a, T, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0);
+  fast_tile<FIRST, PIN>(a, m, blockIdx.x, blockIdx.y, zs.first(blockIdx.z), zs.last(blockIdx.z, a.g.nz), S, ring, T,
+                        0u, fast_stall_plane(a));
 }
 
 // Grid-wide barrier of a cooperative launch: arrive on count, the last arrival resets it
@@ -483,7 +513,7 @@ __global__ void __launch_bounds__(ft::NT, 3) k_fast_stage_tma(const __grid_const
   using namespace ft;
   extern __shared__ unsigned char s_dyn[];
   __shared__ FastShared S;
-  float* const ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_dyn) + 127) & ~uintptr_t(127));
+  float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
   const int nz = st.a[0].g.nz;
   const int ntx = (st.a[0].g.nx + TX - 1) / TX, nty = (st.a[0].g.ny + TY - 1) / TY, ntiles = ntx * nty;
   fast_cta_init(S);
@@ -498,9 +528,9 @@ __global__ void __launch_bounds__(ft::NT, 3) k_fast_stage_tma(const __grid_const
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       const int bx = t % ntx, by = t / ntx;
       bool aborted;
-      if (q > 0) aborted = fast_tile<false, true>(a, st.m[q], bx, by, S, ring, T, base, t == blockIdx.x ? stall : -1);
-      else if (PIN_FIRST) aborted = fast_tile<true, true>(a, st.m[q], bx, by, S, ring, T, base, t == blockIdx.x ? stall : -1);
-      else aborted = fast_tile<true, false>(a, st.m[q], bx, by, S, ring, T, base, t == blockIdx.x ? stall : -1);
+      if (q > 0) aborted = fast_tile<false, true>(a, st.m[q], bx, by, 0, nz, S, ring, T, base, t == blockIdx.x ? stall : -1);
+      else if (PIN_FIRST) aborted = fast_tile<true, true>(a, st.m[q], bx, by, 0, nz, S, ring, T, base, t == blockIdx.x ? stall : -1);
+      else aborted = fast_tile<true, false>(a, st.m[q], bx, by, 0, nz, S, ring, T, base, t == blockIdx.x ? stall : -1);
       if (aborted) {
         // the other CTAs find out at the next grid barrier, which this CTA never reaches
         return;
@@ -533,11 +563,13 @@ cudaError_t init_fast_tma() {
 cudaError_t launch_fast_tma(const FastArgs& a, const FastMaps& m, bool first, bool p_ready, cudaStream_t s) {
   if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err) return cudaErrorInvalidValue;
   const dim3 block(ft::TX, ft::RY);
-  const dim3 grid((a.g.nx + ft::TX - 1) / ft::TX, (a.g.ny + ft::TY - 1) / ft::TY);
+  dim3 grid((a.g.nx + ft::TX - 1) / ft::TX, (a.g.ny + ft::TY - 1) / ft::TY);
+  const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 3, 1.0f);
+  grid.z = zs.chunks;
   const bool fin = a.final_kind == 2;
-  if (first && p_ready) k_fast_tma<true, true><<<grid, block, ft::dyn_smem<true, true>(fin, a.g.nz), s>>>(a, m);
-  else if (first) k_fast_tma<true, false><<<grid, block, ft::dyn_smem<true, false>(fin, a.g.nz), s>>>(a, m);
-  else k_fast_tma<false, true><<<grid, block, ft::dyn_smem<false, true>(fin, a.g.nz), s>>>(a, m);
+  if (first && p_ready) k_fast_tma<true, true><<<grid, block, ft::dyn_smem<true, true>(fin, a.g.nz), s>>>(a, m, zs);
+  else if (first) k_fast_tma<true, false><<<grid, block, ft::dyn_smem<true, false>(fin, a.g.nz), s>>>(a, m, zs);
+  else k_fast_tma<false, true><<<grid, block, ft::dyn_smem<false, true>(fin, a.g.nz), s>>>(a, m, zs);
   return cudaGetLastError();
 }
 

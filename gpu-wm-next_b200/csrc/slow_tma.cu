@@ -22,6 +22,7 @@
 #include "dycore.cuh"
 #include "stencil.cuh"
 #include "tma.cuh"
+#include "zsplit.cuh"
 
 namespace gwmb {
 namespace {
@@ -61,7 +62,8 @@ struct SlowBlend {
 };
 
 template <bool INC>
-__global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const __grid_constant__ SlowMaps m) {
+__global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const __grid_constant__ SlowMaps m,
+                                                        ZSplit zs) {
   using namespace sl;
   extern __shared__ unsigned char s_dyn[];
   __shared__ float s_thref[kMaxNz];
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   __shared__ __align__(8) uint64_t s_bar[NSLOT];
   __shared__ int s_abort[2];
   constexpr int slot = INC ? SLOT : SLOT_SHORT;
-  float* const ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_dyn) + 127) & ~uintptr_t(127));
+  float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
   float* const der = ring + NSLOT * slot;
 
   const Geom& g = a.g;
@@ -96,7 +98,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     s_abort[0] = 0;
     s_abort[1] = 0;
   }
-  if (blockIdx.x == 0 && blockIdx.y == 0 && a.clr_a)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && a.clr_a)
     for (int q = tid; q < nz; q += NT) { a.clr_a[q] = 0ull; a.clr_b[q] = 0ull; }
   for (int q = tid; q < nz; q += NT) {
     s_thref[q] = (float)(acc_read(a.th_acc + q, kScaleTheta) * a.inv_count);
@@ -109,9 +111,14 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   // of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
   int stall = -1;
   if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
-  auto issue = [&](int kk) {  // plane kk in [0, nz] into slot kk % NSLOT
-    float* sr = ring + (kk % NSLOT) * slot;
-    uint64_t* bar = &s_bar[kk % NSLOT];
+  // the CTA's planes are kb .. ke-1; it also loads plane ke and (above the ground) the plane
+  // below, kb-1, whose derived values its lowest faces read
+  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0;
+  if (stall >= 0) stall = kg + stall % (ke - kg + 1);  // a plane that this CTA loads
+  auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * slot; };
+  auto issue = [&](int kk) {  // plane kk in [kg, ke] into its slot
+    float* sr = slot_at(kk);
+    uint64_t* bar = &s_bar[(kk - kg) % NSLOT];
     const bool cells = kk < nz;
     unsigned bytes = (INC ? 2u : 1u) * B_BOX;
     if (cells) bytes += 3 * B_BOX + B_BOXV + (INC ? B_BOX + B_BOXV : 0u);
@@ -132,9 +139,9 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
       }
     }
   };
-  int issued = -1, waited = -1;
+  int issued = kg - 1, waited = kg - 1;
   auto wait_plane = [&](int kk, int epoch) {
-    if (!mbar_wait(&s_bar[kk % NSLOT], (kk / NSLOT) & 1)) {
+    if (!mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1)) {
       s_abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
     } else {
@@ -163,14 +170,11 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     return q;
   };
 
-  if (tid == ISSUER) {
-    issue(0);
-    issue(1);
-    issued = 1;
-  }
-  SlowBlend q0a = load_q0(gj0, own0, 0), q0b = load_q0(gj1, own1, 0);
+  if (tid == ISSUER)
+    for (int kk = kg; kk <= kb + 1; ++kk) { issue(kk); issued = kk; }
+  SlowBlend q0a = load_q0(gj0, own0, kb), q0b = load_q0(gj1, own1, kb);
   SlowCarry ca{0.f, 0.f, 0.f, 0.f, 0.f}, cb{0.f, 0.f, 0.f, 0.f, 0.f};
-  wait_plane(0, 0);
+  wait_plane(kg, kb);
 
   // one owned column: cell, X face, Y face and Z face of plane k (+ the top face)
   // per-plane constants, loaded at the top of the plane so the derive phase covers their latency
@@ -197,8 +201,8 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
                     const PlaneConst& kc) {
     constexpr bool IN = decltype(tile_class)::value;  // an interior tile
     const bool own = IN || own_rt;
-    const float* sr = ring + (k % NSLOT) * slot;
-    const float* sn = ring + ((k + 1) % NSLOT) * slot;
+    const float* sr = slot_at(k);
+    const float* sn = slot_at(k + 1);
     const float* uc = der + D_UC + (k % 3) * DN;
     const float* vc = der + D_VC + (k % 3) * DN;
     const float* wc = der + D_WC + (k % 3) * DN;
@@ -337,63 +341,76 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     cy.wf = wf;
   };
 
+  // derive plane k: theta, p', uc, vc, wc at the 34 x 18 positions
+  auto derive = [&](int k) {
+    const float* sr = slot_at(k);
+    const float* sn = slot_at(k + 1);
+    float* uc = der + D_UC + (k % 3) * DN;
+    float* vc = der + D_VC + (k % 3) * DN;
+    float* wc = der + D_WC + (k % 3) * DN;
+    float* th = der + D_TH + (k & 1) * DN;
+    float* pp = der + D_P + (k & 1) * DN;
+    for (int q = tid; q < DN; q += NT) {
+      const int r = q / DW, c = q - r * DW;
+      const int b = r * BW + c + 3;
+      const float rho = sr[R_RHO + b], rt = RT(sr, b);
+      th[q] = fp::theta(rho, rt);
+      pp[q] = eos_pprime_ref(rho, rt, s_binv[k], s_bpr[k]);
+      // cell-centred velocities: dry_momentum_flux.cu:36-73
+      const float rr = fmaxf(rho, 1.0e-6f);
+      uc[q] = fp::centred(U(sr, b), U(sr, b + 1), rr);
+      vc[q] = fp::centred(V(sr, b), V(sr, b + BW), rr);
+      wc[q] = fp::centred(W(sr, b), W(sn, b), rr);
+    }
+  };
+  if (kb > 0) {  // the plane below the chunk: its derived values, and the column's own
+    wait_plane(kb, kb);
+    derive(kg);
+    const float* sr = slot_at(kg);
+    auto carry = [&](int r) {
+      const int b = r * BW + tx + 4;
+      return SlowCarry{sr[R_RHO + b], fp::theta(sr[R_RHO + b], RT(sr, b)), U(sr, b), V(sr, b), W(sr, b)};
+    };
+    ca = carry(ty + 1);
+    cb = carry(ty + RY + 1);
+  }
+
   // Interior tiles (full, away from every periodic edge ring and open side) run a copy
   // of the plane loop compiled without the edge logic: plain stores, none of the
   // open-boundary flux tests.  Both copies do the same arithmetic on the same values.
   const bool interior = !edge && (g.per_x || (i0 > 0 && i0 + TX < nx)) && (g.per_y || (j0 > 0 && j0 + TY < ny));
   auto plane_loop = [&](auto tile_class) -> bool {  // true when a bounded wait gave up
     constexpr bool IN = decltype(tile_class)::value;
-    for (int k = 0; k < nz; ++k) {
+    for (int k = kb; k < ke; ++k) {
       const int pb = k & 1;
       const PlaneConst kc = plane_const(k);
-      // ---- derive plane k: theta, p', uc, vc, wc at the 34 x 18 positions
       wait_plane(k + 1, k);
-      {
-        const float* sr = ring + (k % NSLOT) * slot;
-        const float* sn = ring + ((k + 1) % NSLOT) * slot;
-        float* uc = der + D_UC + (k % 3) * DN;
-        float* vc = der + D_VC + (k % 3) * DN;
-        float* wc = der + D_WC + (k % 3) * DN;
-        float* th = der + D_TH + pb * DN;
-        float* pp = der + D_P + pb * DN;
-        for (int q = tid; q < DN; q += NT) {
-          const int r = q / DW, c = q - r * DW;
-          const int b = r * BW + c + 3;
-          const float rho = sr[R_RHO + b], rt = RT(sr, b);
-          th[q] = fp::theta(rho, rt);
-          pp[q] = eos_pprime_ref(rho, rt, s_binv[k], s_bpr[k]);
-          // cell-centred velocities: dry_momentum_flux.cu:36-73
-          const float rr = fmaxf(rho, 1.0e-6f);
-          uc[q] = fp::centred(U(sr, b), U(sr, b + 1), rr);
-          vc[q] = fp::centred(V(sr, b), V(sr, b + BW), rr);
-          wc[q] = fp::centred(W(sr, b), W(sn, b), rr);
-        }
-      }
+      derive(k);
       const SlowBlend n0a = load_q0(gj0, own0, k + 1), n0b = load_q0(gj1, own1, k + 1);
       __syncthreads();  // publishes plane k's derived values; slot (k-1) is free
       if (s_abort[pb]) return true;
       if (tid == ISSUER) {
-        if (a.acc_mode && k > 0) {
+        if (a.acc_mode && k > kb) {
           long long sa = 0, sb = 0;
           for (int q = 0; q < NW; ++q) { sa += s_red[pb ^ 1][q][0]; sb += s_red[pb ^ 1][q][1]; }
           acc_add(a.acc_a + k - 1, sa);
           if (a.acc_mode == 1) acc_add(a.acc_b + k - 1, sb);
         }
-        if (k + 2 <= nz) { issue(k + 2); issued = k + 2; }
+        if (k + 2 <= ke) { issue(k + 2); issued = k + 2; }
       }
       // ---- cells and faces of plane k
       FxAcc ra, rb;
       column(tile_class, k, ty + 1, gj0, own0, ca, q0a, ra, rb, kc);
       column(tile_class, k, ty + RY + 1, gj1, own1, cb, q0b, ra, rb, kc);
       if (!IN && xf) {  // open east boundary: X face nx of row j0+tx
-        const float* sr = ring + (k % NSLOT) * slot;
+        const float* sr = slot_at(k);
         const float uf = U(sr, (tx + 1) * BW + w + 4);
         float u1 = fp::update(uf, dt, 0.0f, -1.0e30f);
         if (blend) u1 = fp::blend(a.wa, __ldg(a.u0 + gidx(g, nx, j0 + tx, k)), a.wb, u1);
         put(false, a.o_u, g, kFaceX, nx, j0 + tx, k, u1);
       }
       if (!IN && yf) {  // open north boundary: Y face ny of column i0+tx
-        const float* sr = ring + (k % NSLOT) * slot;
+        const float* sr = slot_at(k);
         const float vf = V(sr, (h + 1) * BW + tx + 4);
         float v1 = fp::update(vf, dt, 0.0f, -1.0e30f);
         if (blend) v1 = fp::blend(a.wa, __ldg(a.v0 + gidx(g, i0 + tx, ny, k)), a.wb, v1);
@@ -411,17 +428,17 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   const bool aborted = interior ? plane_loop(std::true_type{}) : plane_loop(std::false_type{});
   if (aborted) {
     if (tid == ISSUER)
-      for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&s_bar[kk % NSLOT], (kk / NSLOT) & 1);
+      for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1);
     return;
   }
   if (a.acc_mode) {
     __syncthreads();
     if (tid == ISSUER) {
-      const int pb = (nz - 1) & 1;
+      const int pb = (ke - 1) & 1;
       long long sa = 0, sb = 0;
       for (int q = 0; q < NW; ++q) { sa += s_red[pb][q][0]; sb += s_red[pb][q][1]; }
-      acc_add(a.acc_a + nz - 1, sa);
-      if (a.acc_mode == 1) acc_add(a.acc_b + nz - 1, sb);
+      acc_add(a.acc_a + ke - 1, sa);
+      if (a.acc_mode == 1) acc_add(a.acc_b + ke - 1, sb);
     }
   }
 }
@@ -439,9 +456,11 @@ cudaError_t init_slow_tma() {
 cudaError_t launch_slow_tma(const SlowArgs& a, const SlowMaps& m, cudaStream_t s) {
   if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || a.tend_only) return cudaErrorInvalidValue;
   const dim3 block(sl::TX, sl::RY);
-  const dim3 grid((a.g.nx + sl::TX - 1) / sl::TX, (a.g.ny + sl::TY - 1) / sl::TY);
-  if (a.du) k_slow_tma<true><<<grid, block, sl::smem_bytes(true), s>>>(a, m);
-  else k_slow_tma<false><<<grid, block, sl::smem_bytes(false), s>>>(a, m);
+  dim3 grid((a.g.nx + sl::TX - 1) / sl::TX, (a.g.ny + sl::TY - 1) / sl::TY);
+  const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 2, 1.0f);
+  grid.z = zs.chunks;
+  if (a.du) k_slow_tma<true><<<grid, block, sl::smem_bytes(true), s>>>(a, m, zs);
+  else k_slow_tma<false><<<grid, block, sl::smem_bytes(false), s>>>(a, m, zs);
   return cudaGetLastError();
 }
 

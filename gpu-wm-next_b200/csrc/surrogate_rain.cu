@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_rain_net(const RainArgs a, cons
   __shared__ __align__(8) uint64_t s_mma;           // tcgen05.commit of one layer
   __shared__ unsigned s_tmem;
   __shared__ int s_tail, s_consumed, s_prod_done, s_fail, s_cmd, s_cfail;
-  unsigned char* const base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(s_dyn) + 127) & ~uintptr_t(127));
+  unsigned char* const base = align_smem_128(s_dyn);
   unsigned char* const sw = base;                       // weights, canonical layout
   unsigned char* const sa1 = base + kWBytes;            // layer-1 input ring, kTiles tiles
   unsigned char* const sah = base + kWBytes + kA1Bytes; // hidden-layer operand

@@ -46,6 +46,14 @@ __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
 
+// The first 128-byte boundary of a kernel's dynamic shared memory (its allocation carries
+// 128 bytes of slack).  The offset is added to the array itself: rounding the address up as
+// an integer would hide from the compiler that the result is shared memory, and every ring
+// access would become a generic load with 64-bit address arithmetic.
+__device__ __forceinline__ unsigned char* align_smem_128(unsigned char* dyn) {
+  return dyn + (-smem_u32(dyn) & 127u);
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
@@ -66,14 +74,21 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned by
                : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// The thread may sleep this long in one try_wait before it polls again, so that waiting warps
+// leave the issue slots to the others.
+constexpr unsigned kSuspendNs = 20000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
   unsigned ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
       : "memory");
   return ok != 0;
 }

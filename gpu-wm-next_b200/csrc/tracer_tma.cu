@@ -17,6 +17,7 @@
 #include "physics.cuh"
 #include "stencil.cuh"
 #include "tma.cuh"
+#include "zsplit.cuh"
 
 namespace gwmb {
 namespace {
@@ -39,13 +40,14 @@ static_assert(O_Q - O_RHO >= CBW * CBH && O_U - O_Q >= NTR * 736 && O_V - O_U >=
 }  // namespace tt
 
 template <bool TERRAIN>
-__global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, const __grid_constant__ TracerMaps m) {
+__global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, const __grid_constant__ TracerMaps m,
+                                                          ZSplit zs) {
   using namespace tt;
   extern __shared__ unsigned char s_dyn[];
   __shared__ float s_q[NTR][2][QH][QW];
   __shared__ __align__(8) uint64_t s_bar[NSLOT];
   __shared__ int s_abort[2];
-  float* const ring = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(s_dyn) + 127) & ~uintptr_t(127));
+  float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
 
   const Geom& g = a.g;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
@@ -77,9 +79,14 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
   // of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
   int stall = -1;
   if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
-  auto issue = [&](int kk) {  // plane kk in [0, nz]; plane nz holds the top faces only
-    float* st = ring + (kk % NSLOT) * SLOT;
-    uint64_t* bar = &s_bar[kk % NSLOT];
+  // the CTA's planes are kb .. ke-1; it also loads plane ke and (above the ground) the plane
+  // below, kb-1, whose mixing ratios its lowest faces read
+  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0;
+  if (stall >= 0) stall = kg + stall % (ke - kg + 1);  // a plane that this CTA loads
+  auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
+  auto issue = [&](int kk) {  // plane kk in [kg, ke]; plane nz holds the top faces only
+    float* st = slot_at(kk);
+    uint64_t* bar = &s_bar[(kk - kg) % NSLOT];
     const bool cells = kk < nz;
     unsigned bytes = B_OWN;
     if (cells) bytes += (1 + a.ntracers) * B_CELL + 2 * B_FACE;
@@ -94,9 +101,9 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
       tma_load_3d(st + O_V, &m.v, i0 + kXOff, j0 + 1, kk, bar);
     }
   };
-  int issued = -1, waited = -1;
+  int issued = kg - 1, waited = kg - 1;
   auto wait_plane = [&](int kk, int epoch) {
-    if (!mbar_wait(&s_bar[kk % NSLOT], (kk / NSLOT) & 1)) {
+    if (!mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1)) {
       s_abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
     } else {
@@ -105,7 +112,7 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
   };
   // mixing ratios of plane kk (dry_transport.cu:91-94) at the owned cells and the ring
   auto mix = [&](int kk) {
-    const float* st = ring + (kk % NSLOT) * SLOT;
+    const float* st = slot_at(kk);
     auto one = [&](int r, int c) {
       const int b = r * CBW + c + 3;
       const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
@@ -118,16 +125,26 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
     if (hr >= 0) one(hr, hc);
   };
 
-  if (tid == ISSUER) {
-    issue(0);
-    issue(1);
-    issued = 1;
-    if (nz >= 2) { issue(2); issued = 2; }
-  }
-  wait_plane(0, 0);
-  mix(0);
+  if (tid == ISSUER)
+    for (int kk = kg; kk < kg + NSLOT && kk <= ke; ++kk) { issue(kk); issued = kk; }
   float qb0[NTR] = {0.f, 0.f, 0.f}, qb1[NTR] = {0.f, 0.f, 0.f};  // own mixing ratios at k-1
+  wait_plane(kg, kb);
+  if (kb > 0) {  // those of the plane below the chunk
+    const float* st = slot_at(kg);
+    auto below = [&](int row, float* qb) {
+      const int b = (row + 1) * CBW + tx + 4;
+      const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
+#pragma unroll
+      for (int t = 0; t < NTR; ++t)
+        if (t < a.ntracers) qb[t] = st[O_Q + t * 736 + b] / rr;
+    };
+    below(ty, qb0);
+    below(ty + RY, qb1);
+    wait_plane(kb, kb);
+  }
+  mix(kb);
   __syncthreads();
+  if (kb > 0 && tid == ISSUER && kb + 2 <= ke) { issue(kb + 2); issued = kb + 2; }  // into plane kg's slot
 
   // blend partner of plane kk at the thread's owned cells (prefetched a plane ahead)
   auto load_q0 = [&](int gj, bool own, int kk, float* q0v) {
@@ -140,15 +157,15 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
       if (t < a.ntracers) q0v[t] = __ldg(a.q0[t] + o);
   };
   float q0a[NTR], q0b[NTR];
-  load_q0(gj0, own0, 0, q0a);
-  load_q0(gj1, own1, 0, q0b);
+  load_q0(gj0, own0, kb, q0a);
+  load_q0(gj1, own1, kb, q0b);
 
   // one owned column of plane k
   auto column = [&](auto tile_class, int k, int r, int gj, bool own_rt, float* qb, const float* q0v, float idz) {
     constexpr bool IN = decltype(tile_class)::value;  // interior tile: plain stores
     const bool own = IN || own_rt;
-    const float* st = ring + (k % NSLOT) * SLOT;
-    const float* sn = ring + ((k + 1) % NSLOT) * SLOT;
+    const float* st = slot_at(k);
+    const float* sn = slot_at(k + 1);
     const int c = tx + 1;
     const int pb = k & 1;
     const float fw = st[O_U + (r - 1) * FBW + tx], fe = st[O_U + (r - 1) * FBW + tx + 1];
@@ -181,7 +198,7 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
   const bool interior = !edge && i0 + TX <= nx && j0 + TY <= ny;
   auto plane_loop = [&](auto tile_class) -> bool {  // true when a bounded wait gave up
     [[maybe_unused]] constexpr bool IN = decltype(tile_class)::value;
-    for (int k = 0; k < nz; ++k) {
+    for (int k = kb; k < ke; ++k) {
       // mixing ratios of plane k+1 (the own ones are this thread's, the ring published
       // by the barrier below for the next plane)
       // inverse layer depth (per level on flat terrain, per cell on terrain), loaded ahead
@@ -204,13 +221,13 @@ __global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, co
       for (int t = 0; t < NTR; ++t) { q0a[t] = n0a[t]; q0b[t] = n0b[t]; }
       __syncthreads();  // publishes plane k+1's ring; slot k is free
       if (s_abort[k & 1]) return true;
-      if (tid == ISSUER && k + 3 <= nz) { issue(k + 3); issued = k + 3; }
+      if (tid == ISSUER && k + 3 <= ke) { issue(k + 3); issued = k + 3; }
     }
     return false;
   };
   const bool aborted = interior ? plane_loop(std::true_type{}) : plane_loop(std::false_type{});
   if (aborted && tid == ISSUER)
-    for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&s_bar[kk % NSLOT], (kk / NSLOT) & 1);
+    for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1);
 }
 
 }  // namespace
@@ -225,9 +242,11 @@ cudaError_t init_tracer_tma() {
 cudaError_t launch_tracer_tma(const TracerArgs& a, const TracerMaps& m, cudaStream_t s) {
   if (a.g.nz < 1 || !a.err || a.ntracers < 1 || a.ntracers > tt::NTR) return cudaErrorInvalidValue;
   const dim3 block(tt::TX, tt::RY);
-  const dim3 grid((a.g.nx + tt::TX - 1) / tt::TX, (a.g.ny + tt::TY - 1) / tt::TY);
-  if (a.terrain) k_tracer_tma<true><<<grid, block, tt::kDynSmem, s>>>(a, m);
-  else k_tracer_tma<false><<<grid, block, tt::kDynSmem, s>>>(a, m);
+  dim3 grid((a.g.nx + tt::TX - 1) / tt::TX, (a.g.ny + tt::TY - 1) / tt::TY);
+  const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 3, 1.2f);
+  grid.z = zs.chunks;
+  if (a.terrain) k_tracer_tma<true><<<grid, block, tt::kDynSmem, s>>>(a, m, zs);
+  else k_tracer_tma<false><<<grid, block, tt::kDynSmem, s>>>(a, m, zs);
   return cudaGetLastError();
 }
 
