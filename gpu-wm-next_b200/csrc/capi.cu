@@ -537,6 +537,8 @@ cudaError_t launch_substep(gwm_b200_ctx* c, const Member& M, const FastArgs& f, 
   if (!terr && fast_tma_path(c)) {
     FastMaps m{};
     if (!fast_maps(M, f, first, p_ready, m)) return cudaErrorInvalidValue;
+    // the standard substep with its p' at hand runs on independent warps
+    if ((!first || p_ready) && f.hmom && f.dens) return launch_fast_rows(f, m, first, c->stream);
     return launch_fast_tma(f, m, first, p_ready, c->stream);
   }
   return launch_fast(f, first, terr, c->stream, c->fast_tile_rows);
@@ -940,7 +942,7 @@ int gwm_b200_create(const gwm_b200_grid_desc* grids, const gwm_b200_member_desc*
   cudaError_t e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return GWM_B200_ERR_CUDA; }
   c->stream = c->own_stream;
-  if (init_fast_tma() != cudaSuccess || init_fast_terrain_tma() != cudaSuccess || init_slow_tma() != cudaSuccess ||
+  if (init_fast_tma() != cudaSuccess || init_fast_rows() != cudaSuccess || init_fast_terrain_tma() != cudaSuccess || init_slow_tma() != cudaSuccess ||
       init_slow_terrain_tma() != cudaSuccess || init_tracer_tma() != cudaSuccess) {
     cudaStreamDestroy(c->own_stream);
     delete c;

@@ -78,6 +78,11 @@ __device__ __forceinline__ float column_dpdz(int k, int nz, float pm, float pc, 
 // real arithmetic (the base is constant on a level) but keep ~1e-5 Pa resolution
 // instead of the ~1e-2 Pa of an FP32 pressure near 1e5 Pa.
 // base layout: [rt_ref(nz) | 1/rt_ref(nz) | p_ref(nz)], FP64.
+// The rare far-from-base form is a call: inlined at every use it would multiply the code of
+// the unrolled plane loops.
+static __noinline__ __device__ float eos_pprime_full(float rho, float rt, double pref) {
+  return (float)((double)eos_pressure(rho, rt) - pref);
+}
 // Core form with the level's 1/rt_ref and p_ref already at hand.
 __device__ __forceinline__ float eos_pprime_ref(float rho, float rt, double inv_rt_ref, double pref) {
   const double d = fma((double)rt, inv_rt_ref, -1.0);
@@ -93,7 +98,7 @@ __device__ __forceinline__ float eos_pprime_ref(float rho, float rt, double inv_
     const double s = fma(hi, d4, lo);
     return (float)(pref * (s * d));
   }
-  return (float)((double)eos_pressure(rho, rt) - pref);
+  return eos_pprime_full(rho, rt, pref);
 }
 __device__ __forceinline__ float eos_pprime(float rho, float rt, const double* __restrict__ base, int k,
                                             int nz) {
@@ -194,6 +199,14 @@ struct FxAcc {
     return (long long)sh * 16777216LL + (long long)sl;
   }
 };
+
+// The warp total of int64 fixed-point values (sums of fx() over a thread's few cells), split
+// as in FxAcc but once per thread.
+__device__ __forceinline__ long long warp_total_fx(long long x) {
+  const int sh = __reduce_add_sync(0xffffffffu, (int)(x >> 24));
+  const unsigned sl = __reduce_add_sync(0xffffffffu, (unsigned)(x & 0xffffffLL));
+  return (long long)sh * 16777216LL + (long long)sl;
+}
 
 __device__ __forceinline__ long long warp_sum_ll(long long v) {
 #pragma unroll

@@ -131,6 +131,10 @@ cudaError_t init_slow_terrain_tma();
 // first: the first substep of a stage (no increments in); p_ready: its p' (with the
 // halo ring) is in a.p_in, written by the slow stage, instead of derived from rho, theta
 cudaError_t launch_fast_tma(const FastArgs& a, const FastMaps& m, bool first, bool p_ready, cudaStream_t s);
+// The same substep with independent warps (fast_rows.cu), for a substep that loads p' of its
+// input (not first, or p_ready) and updates momenta and density (a.hmom, a.dens).
+cudaError_t launch_fast_rows(const FastArgs& a, const FastMaps& m, bool first, cudaStream_t s);
+cudaError_t init_fast_rows();
 // Acoustic substep on terrain fed by TMA tile loads (owned 32 x 16 tiles): the
 // arithmetic of the overlapped-tile terrain kernel.  Needs a.col_pref / a.col_rref
 // (launch_column_reference of a.rho_in first); inner substeps (final_kind 0) store the

@@ -82,13 +82,18 @@ __device__ __forceinline__ V hmom_terrain(V d, V pr, V pl, V zr, V zl, V dpdz_l,
 }
 // K14 vertical momentum increment at a face: dw + dtf (-(p'_u - p'_l) idzf - g rho'_f),
 // with p'_u = pn - pru, p'_l = pc - prl and rho'_f = 0.5 ((rc - rrl) + (rn - rru)).
+// wmom_pert takes the perturbations p'_u, p'_l, rho'_l, rho'_u themselves.
+template <class V>
+__device__ __forceinline__ V wmom_pert(V dw, V pu, V pl, V rl, V ru, float idzf, float gravity, float dtf) {
+  const V dp = sub(pu, pl);
+  const V rf = mul(sc<V>(0.5f), add(rl, ru));
+  const V tend = fma(neg(dp), sc<V>(idzf), neg(mul(sc<V>(gravity), rf)));
+  return fma(sc<V>(dtf), tend, dw);
+}
 template <class V>
 __device__ __forceinline__ V wmom(V dw, V pn, V pru, V pc, V prl, V rc, V rrl, V rn, V rru, float idzf, float gravity,
                                   float dtf) {
-  const V dp = sub(sub(pn, pru), sub(pc, prl));
-  const V rf = mul(sc<V>(0.5f), add(sub(rc, rrl), sub(rn, rru)));
-  const V tend = fma(neg(dp), sc<V>(idzf), neg(mul(sc<V>(gravity), rf)));
-  return fma(sc<V>(dtf), tend, dw);
+  return wmom_pert(dw, sub(pn, pru), sub(pc, prl), sub(rc, rrl), sub(rn, rru), idzf, gravity, dtf);
 }
 // K15 density from the perturbation mass-flux divergence: max(1e-6, rho - dtf div).
 template <class V>
