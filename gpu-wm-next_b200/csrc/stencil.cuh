@@ -29,6 +29,20 @@ __device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b);
 __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ float div(float a, float b) { return __fdiv_rn(a, b); }
+// Quotients of several values by one b.  With y = 1/b rounded to nearest, one residual step
+// makes q = a y faithful and a second one gives a / b rounded to nearest (P. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34, 1990, theorem 8.3): the value of div(a, b), five operations each instead of a
+// division.  It holds where the residuals neither overflow nor underflow; for b in [1e-6,
+// 1e6] that is a = 0 or 2^-79 <= |a| <= 2^100.  Smaller |a| may be one ulp off (of values
+// below 1e-18); the callers send quotients that are not finite to div().
+__device__ __forceinline__ float recip(float b) { return __frcp_rn(b); }
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+  const float q0 = __fmul_rn(a, y);
+  const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+  return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+}
+__device__ __forceinline__ bool finite(float a) { return fabsf(a) < __int_as_float(0x7f800000); }
 __device__ __forceinline__ float neg(float a) { return -a; }
 __device__ __forceinline__ float vmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float select_ge0(float a, float x, float y) { return a >= 0.0f ? x : y; }
@@ -126,6 +140,16 @@ __device__ __forceinline__ V add_buoyancy(V t, V th_l, V th_u, float tref_l, flo
   const float trf = __fmul_rn(0.5f, __fadd_rn(tref_l, tref_u));
   const V tf = avg(th_l, th_u);
   const V b = div(mul(sc<V>(gravity), sub(tf, sc<V>(trf))), sc<V>(fmaxf(trf, 1.0e-6f)));
+  return fma(avg(rho_l, rho_u), b, t);
+}
+
+// The same with the face mean of the level means, trf, and the reciprocal of its floored
+// value at hand (one pair per level).
+__device__ __forceinline__ float add_buoyancy_ref(float t, float th_l, float th_u, float trf, float ytrf, float rho_l,
+                                                  float rho_u, float gravity) {
+  const float n = mul(gravity, sub(avg(th_l, th_u), trf)), d = fmaxf(trf, 1.0e-6f);
+  float b = div_by(n, d, ytrf);
+  if (!finite(b)) b = div(n, d);
   return fma(avg(rho_l, rho_u), b, t);
 }
 
