@@ -107,108 +107,145 @@ __global__ void __launch_bounds__(BX * TBY) k_tracer_stage(const TracerArgs a) {
 }
 
 
-constexpr int RB = 128;  // columns per warm-rain block (one row segment)
+// Warm rain and fallout.  A warp takes 32 columns of one row; a CTA's kRW warps are WX along
+// the row and kRW / WX up the levels.  What falls out of a cell depends on that cell alone, so
+// only the top cell of a warp's levels waits for its inflow, from the warp above through
+// shared memory.  Small grids take all warps up the levels: a column sweep is a serial chain
+// of nz cells there (109 us at 128 x 128 x 64; 33 us in eight chunks).  Large grids take long
+// rows, whose loads are contiguous (1024 x 1024 x 64: 948 us with 32 columns per CTA).
+constexpr int kRW = 8;  // warps per CTA
 
 // MICRO = false: fallout only, on a state whose microphysics was already applied
 // (the surrogate's network kernel); the reference applies each cell's microphysics
 // before the rain from above arrives, so the split is exact.
-template <bool MICRO>
-__global__ void __launch_bounds__(RB) k_warm_rain(const RainArgs a) {
+template <bool MICRO, int WX>
+__global__ void __launch_bounds__(32 * kRW) k_warm_rain(const RainArgs a) {
+  constexpr int WZ = kRW / WX;
   const Geom& g = a.g;
-  const int gi = blockIdx.x * RB + threadIdx.x;
-  const int gj = blockIdx.y;
-  const bool active = gi < g.nx && gj < g.ny;
-  const int ilo = blockIdx.x * RB;
-  const bool edge = (g.per_x && (ilo <= 1 || ilo + RB - 1 >= g.nx - 1)) ||
-                    (g.per_y && (gj <= 1 || gj >= g.ny - 1));
-  __shared__ long long s_th[kMaxNz][RB / 32];
-  float incoming = 0.0f;
-  // one-cell-ahead prefetch down the column
-  float n_rho = 0.f, n_rt = 0.f, n_qv = 0.f, n_qc = 0.f, n_qr = 0.f;
-  const bool need_rt = MICRO || a.th_acc;
-  if (active) {
-    const int o = gidx(g, gi, gj, g.nz - 1);
-    n_rho = __ldg(a.rho + o); n_qr = a.qr[o];
-    if (need_rt) n_rt = a.rt[o];
-    if (MICRO) { n_qv = a.qv[o]; n_qc = a.qc[o]; }
-  }
-  for (int k = g.nz - 1; k >= 0; --k) {
-    FxAcc th_sum;
-    const float c_rho = n_rho, c_rt = n_rt, c_qv = n_qv, c_qc = n_qc, c_qr = n_qr;
-    if (active && k > 0) {
-      const int o1 = gidx(g, gi, gj, k - 1);
-      n_rho = __ldg(a.rho + o1); n_qr = a.qr[o1];
-      if (need_rt) n_rt = a.rt[o1];
-      if (MICRO) { n_qv = a.qv[o1]; n_qc = a.qc[o1]; }
-    }
-    if (active) {
-      const int o = gidx(g, gi, gj, k);
-      const float rho_d = c_rho;
-      float rho = 0.0f, th = 0.0f, qv = 0.0f, qc = 0.0f, rqr = c_qr;
-      if (MICRO) {  // warm_rain_kernel: warm_rain.cu:36-120
-        MicroCell mc;
-        if (a.thr >= 0.0f && surely_quiet(rho_d, c_rt, c_qv, c_qc, c_qr)) {
-          // micro_step leaves the cell as micro_state derives it: only the mixing ratios
-          // and theta are needed, not the temperature, pressure or saturation
-          mc.rho = fmaxf(rho_d, 1.0e-6f);
-          mc.th = c_rt / mc.rho;
-          mc.qv = fmaxf(c_qv / mc.rho, 0.0f);
-          mc.qc = fmaxf(c_qc / mc.rho, 0.0f);
-          mc.qr = fmaxf(c_qr / mc.rho, 0.0f);
-        } else {
-          mc = micro_state(rho_d, c_rt, c_qv, c_qc, c_qr);
-          micro_step(mc, MicroParams{a.dt, a.relax, a.thr, a.rate, a.evap, a.latent});
-        }
-        rho = mc.rho; th = mc.th; qv = mc.qv; qc = mc.qc;
-        rqr = rho * mc.qr;
-      }
-      // fallout of this cell, fed by the cell above
-      if (a.fallout_mode == 1) {  // rain_fallout_metric_kernel: warm_rain.cu:156-191
-        const float idz = fmaxf(a.terrain ? __ldg(a.idz_c + o) : __ldg(a.idz_c + k), 1.0e-6f);
-        const float dz = 1.0f / idz;
-        const float frac = fminf(fmaxf(a.vt * a.dt * idz, 0.0f), 1.0f);
-        const float old_a = fmaxf(rqr, 0.0f) * dz;
-        const float out = frac * old_a;
-        rqr = ((old_a - out) + incoming) * idz;
-        incoming = out;
-      } else if (a.fallout_mode == 2) {  // rain_fallout_nominal_kernel: warm_rain.cu:122-154
-        const float dz = fmaxf(a.layer_depth, 1.0e-3f);
-        const float frac = fminf(fmaxf(a.vt * a.dt / dz, 0.0f), 1.0f);
-        if (frac > 0.0f) {
-          const float old_a = fmaxf(rqr, 0.0f) * dz;
-          const float out = frac * old_a;
-          rqr = ((old_a - out) + incoming) / dz;
-          incoming = out;
-        }
-      }
-      const float rt_new = MICRO ? rho * th : c_rt;
-      if (MICRO) {
-        store_tile(a.qv, g, kCell, gi, gj, k, rho * qv, edge);
-        store_tile(a.qc, g, kCell, gi, gj, k, rho * qc, edge);
-        store_tile(a.rt, g, kCell, gi, gj, k, rt_new, edge);
-      }
-      if (MICRO || a.fallout_mode) store_tile(a.qr, g, kCell, gi, gj, k, rqr, edge);
-      if (a.th_acc) th_sum.add(theta_of(rho_d, rt_new), kFxTheta);
-    }
-    if (a.th_acc) {
-      const long long t = th_sum.warp_total();
-      if ((threadIdx.x & 31) == 0) s_th[k][threadIdx.x >> 5] = t;
-    }
-  }
-  if (active && a.fallout_mode && a.precip) {  // compensated FP64 surface accumulation
-    const int q = gj * g.nx + gi;
-    const double s = a.precip[q], x = (double)incoming, t = s + x;
-    a.precip_comp[q] += (fabs(s) >= fabs(x)) ? (s - t) + x : (x - t) + s;
-    a.precip[q] = t;
-  }
-  if (a.th_acc) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wx = wid % WX, wz = wid / WX;
+  const int per = (g.nz + WZ - 1) / WZ;
+  const int k0 = wz * per, k1 = min(k0 + per, g.nz);  // the warp's levels (none when k0 >= nz)
+  __shared__ long long s_th[kMaxNz][WX];
+  __shared__ float s_out[kRW][32];  // outflow of each warp's lowest cell
+  // fallout of a layer: its floored inverse depth, its depth, the fraction that falls out
+  struct Layer {
+    float idz, dz, frac;
+  };
+  __shared__ Layer s_layer[kMaxNz];  // flat terrain: one per level
+  auto layer = [&](float v) {
+    const float idz = fmaxf(v, 1.0e-6f);
+    return Layer{idz, 1.0f / idz, fminf(fmaxf(a.vt * a.dt * idz, 0.0f), 1.0f)};
+  };
+  if (a.fallout_mode == 1 && !a.terrain) {
+    for (int k = threadIdx.x; k < g.nz; k += 32 * kRW) s_layer[k] = layer(__ldg(a.idz_c + k));
     __syncthreads();
-    for (int k = threadIdx.x; k < g.nz; k += RB) {
+  }
+  const bool need_rt = MICRO || a.th_acc;
+  {
+    const int gj = blockIdx.y, ilo = (blockIdx.x * WX + wx) * 32, gi = ilo + lane;
+    const bool active = gi < g.nx;
+    const bool edge = (g.per_x && (ilo <= 1 || ilo + 31 >= g.nx - 1)) || (g.per_y && (gj <= 1 || gj >= g.ny - 1));
+    float out = 0.0f;                     // falling out of the cell above
+    float top_kept = 0.0f, top_f = 0.0f;  // top cell: water kept, and the factor to a density
+    const bool waits = k1 < g.nz && k0 < k1 && a.fallout_mode != 0;  // its inflow comes from another warp
+    // one-cell-ahead prefetch down the levels
+    float n_rho = 0.f, n_rt = 0.f, n_qv = 0.f, n_qc = 0.f, n_qr = 0.f;
+    auto fetch = [&](int k) {
+      const int o = gidx(g, gi, gj, k);
+      n_rho = __ldg(a.rho + o);
+      n_qr = a.qr[o];
+      if (need_rt) n_rt = a.rt[o];
+      if (MICRO) { n_qv = a.qv[o]; n_qc = a.qc[o]; }
+    };
+    if (active && k0 < k1) fetch(k1 - 1);
+    for (int k = k1 - 1; k >= k0; --k) {
+      long long th_sum = 0;
+      const float c_rho = n_rho, c_rt = n_rt, c_qv = n_qv, c_qc = n_qc, c_qr = n_qr;
+      if (active && k > k0) fetch(k - 1);
+      if (active) {
+        const float rho_d = c_rho;
+        float rho = 0.0f, th = 0.0f, qv = 0.0f, qc = 0.0f, rqr = c_qr;
+        // a / max(rho, 1e-6) of several a by one reciprocal
+        const float rr = fmaxf(rho_d, 1.0e-6f), y = fp::recip(rr);
+        auto quotient = [&](float v) {
+          const float t = fp::div_by(v, rr, y);
+          return fp::finite(t) ? t : fp::div(v, rr);
+        };
+        if (MICRO) {  // warm_rain_kernel: warm_rain.cu:36-120
+          MicroCell mc;
+          if (a.thr >= 0.0f && surely_quiet(rho_d, c_rt, c_qv, c_qc, c_qr)) {
+            // micro_step leaves the cell as micro_state derives it: only the mixing ratios
+            // and theta are needed, not the temperature, pressure or saturation
+            mc.rho = rr;
+            mc.th = quotient(c_rt);
+            mc.qv = fmaxf(quotient(c_qv), 0.0f);
+            mc.qc = 0.0f;  // no cloud or rain water above zero: clipped at zero
+            mc.qr = 0.0f;
+          } else {
+            mc = micro_state(rho_d, c_rt, c_qv, c_qc, c_qr);
+            micro_step(mc, MicroParams{a.dt, a.relax, a.thr, a.rate, a.evap, a.latent});
+          }
+          rho = mc.rho; th = mc.th; qv = mc.qv; qc = mc.qc;
+          rqr = rho * mc.qr;
+        }
+        // fallout of this cell, fed by the cell above
+        const bool top = waits && k == k1 - 1;
+        if (a.fallout_mode == 1) {  // rain_fallout_metric_kernel: warm_rain.cu:156-191
+          const Layer l = a.terrain ? layer(__ldg(a.idz_c + gidx(g, gi, gj, k))) : s_layer[k];
+          const float idz = l.idz, dz = l.dz, frac = l.frac;
+          const float old_a = fmaxf(rqr, 0.0f) * dz;
+          const float fall = frac * old_a;
+          rqr = ((old_a - fall) + out) * idz;
+          if (top) { top_kept = old_a - fall; top_f = idz; }
+          out = fall;
+        } else if (a.fallout_mode == 2) {  // rain_fallout_nominal_kernel: warm_rain.cu:122-154
+          const float dz = fmaxf(a.layer_depth, 1.0e-3f);
+          const float frac = fminf(fmaxf(a.vt * a.dt / dz, 0.0f), 1.0f);
+          if (frac > 0.0f) {
+            const float old_a = fmaxf(rqr, 0.0f) * dz;
+            const float fall = frac * old_a;
+            rqr = ((old_a - fall) + out) / dz;
+            if (top) { top_kept = old_a - fall; top_f = dz; }
+            out = fall;
+          } else if (top) {
+            top_kept = rqr;
+            top_f = 0.0f;  // nothing falls: the cell keeps its water
+          }
+        }
+        const float rt_new = MICRO ? rho * th : c_rt;
+        if (MICRO) {
+          store_tile(a.qv, g, kCell, gi, gj, k, rho * qv, edge);
+          store_tile(a.qc, g, kCell, gi, gj, k, rho * qc, edge);
+          store_tile(a.rt, g, kCell, gi, gj, k, rt_new, edge);
+        }
+        if ((MICRO || a.fallout_mode) && !top) store_tile(a.qr, g, kCell, gi, gj, k, rqr, edge);
+        if (a.th_acc) th_sum = fx(quotient(rt_new), kFxTheta);
+      }
+      if (a.th_acc) {
+        const long long t = warp_total_fx(th_sum);
+        if (lane == 0) s_th[k][wx] = t;
+      }
+    }
+    s_out[wid][lane] = out;
+    __syncthreads();
+    if (active && waits) {  // the top cell's inflow: what fell out of the warp above
+      const float in = s_out[wid + WX][lane];
+      const float rqr = a.fallout_mode == 1 ? (top_kept + in) * top_f : (top_f > 0.0f ? (top_kept + in) / top_f : top_kept);
+      store_tile(a.qr, g, kCell, gi, gj, k1 - 1, rqr, edge);
+    }
+    if (wz == 0 && active && a.fallout_mode && a.precip) {  // compensated FP64 surface accumulation
+      const int o = gj * g.nx + gi;
+      const double s = a.precip[o], x = (double)out, t = s + x;
+      a.precip_comp[o] += (fabs(s) >= fabs(x)) ? (s - t) + x : (x - t) + s;
+      a.precip[o] = t;
+    }
+  }
+  if (a.th_acc)
+    for (int k = threadIdx.x; k < g.nz; k += 32 * kRW) {
       long long t = 0;
-      for (int w = 0; w < RB / 32; ++w) t += s_th[k][w];
+      for (int v = 0; v < WX; ++v) t += s_th[k][v];
       acc_add(a.th_acc + k, t);
     }
-  }
 }
 
 }  // namespace
@@ -226,9 +263,16 @@ cudaError_t launch_tracer_stage(const TracerArgs& a, cudaStream_t s, int tile_ro
 
 cudaError_t launch_warm_rain(const RainArgs& a, cudaStream_t s, bool micro) {
   if (a.g.nz > kMaxNz) return cudaErrorInvalidValue;
-  const dim3 grid((a.g.nx + RB - 1) / RB, a.g.ny);
-  if (micro) k_warm_rain<true><<<grid, RB, 0, s>>>(a);
-  else if (a.fallout_mode || a.th_acc) k_warm_rain<false><<<grid, RB, 0, s>>>(a);
+  // enough CTAs for two waves of four per SM decide how much of the CTA goes along the row
+  const int nseg = (a.g.nx + 31) / 32 * a.g.ny;
+  const int wx = nseg >= 4 * 148 * 8 ? 4 : nseg >= 2 * 148 * 8 ? 2 : 1;
+  const dim3 grid((a.g.nx + 32 * wx - 1) / (32 * wx), a.g.ny);
+  if (!micro && !a.fallout_mode && !a.th_acc) return cudaSuccess;
+  switch (wx) {
+    case 4: micro ? k_warm_rain<true, 4><<<grid, 32 * kRW, 0, s>>>(a) : k_warm_rain<false, 4><<<grid, 32 * kRW, 0, s>>>(a); break;
+    case 2: micro ? k_warm_rain<true, 2><<<grid, 32 * kRW, 0, s>>>(a) : k_warm_rain<false, 2><<<grid, 32 * kRW, 0, s>>>(a); break;
+    default: micro ? k_warm_rain<true, 1><<<grid, 32 * kRW, 0, s>>>(a) : k_warm_rain<false, 1><<<grid, 32 * kRW, 0, s>>>(a);
+  }
   return cudaGetLastError();
 }
 
