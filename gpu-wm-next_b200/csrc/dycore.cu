@@ -377,9 +377,16 @@ __global__ void __launch_bounds__(128) k_column_reference(const FastArgs a) {
   if (i >= g.nx || j >= g.ny) return;
   const int base = gidx(g, i, j, 0);
   float pref = 0.f, rref = 0.f, zb = 0.f;
+  // the next level's values are loaded while this one's chain runs
+  float n_rho = __ldg(a.rho_in + base), n_th = __ldg(a.th + base), n_z = __ldg(a.zc + base);
   for (int k = 0; k < g.nz; ++k) {
     const int o = base + k * g.plane;
-    const float rho = __ldg(a.rho_in + o), th = __ldg(a.th + o), z = __ldg(a.zc + o);
+    const float rho = n_rho, th = n_th, z = n_z;
+    if (k + 1 < g.nz) {
+      n_rho = __ldg(a.rho_in + o + g.plane);
+      n_th = __ldg(a.th + o + g.plane);
+      n_z = __ldg(a.zc + o + g.plane);
+    }
     fp::column_reference_level(k, rho, fp::mul(rho, th), z, a.gravity, pref, rref, zb);
     a.col_pref[o] = pref;
     a.col_rref[o] = rref;

@@ -158,30 +158,35 @@ __device__ __forceinline__ float add_buoyancy_ref(float t, float th_l, float th_
 // rho, rho*theta and height z, given those of the level below (pref, rref at height zb);
 // updates pref, rref and zb.  Four fixed-point iterations, then the density of the result.
 // An iteration that returns its own input is a fixed point that every later iteration
-// repeats, and the final density is then the one just evaluated, so the loop stops there
-// with the same result (the iterations contract by about g dz / (2 c^2) ~ 1e-2).
+// repeats, and the final density is then the one just evaluated, so the third iteration and
+// the fourth stop there with the same result (the iterations contract by about
+// g dz / (2 c^2) ~ 1e-2, so the first two are never the last).
+__device__ __forceinline__ float eos_rho_of(float p, float rdth) {  // eos_rho with Rd*theta at hand
+  const float x = div_by(p, kP0, 1.0f / kP0);
+  return p / fmaxf(rdth * powf(fmaxf(x, 1.0e-6f), kKappa), 1.0e-6f);
+}
 __device__ __forceinline__ void column_reference_level(int k, float rho, float rt, float z, float gravity,
                                                        float& pref, float& rref, float& zb) {
-  const float thp = theta(rho, rt);
+  const float rdth = kRd * theta(rho, rt);
   if (k == 0) {
     pref = eos_pressure(rho, rt);
-    rref = eos_rho(pref, thp);
+    rref = eos_rho_of(pref, rdth);
   } else {
-    const float dzk = z - zb;
+    const float dzk = z - zb, hg = mul(gravity, 0.5f);
+    auto next = [&](float rn) { return fmaxf(fma(-mul(hg, add(rref, rn)), dzk, pref), 1.0f); };
     float pn = fmaxf(1.0f, fma(-mul(gravity, rref), dzk, pref));
-    float rn = 0.0f;
-    bool fixed = false;
-    for (int it = 0; it < 4; ++it) {
-      rn = eos_rho(pn, thp);
-      const float pq = fmaxf(fma(-mul(mul(gravity, 0.5f), add(rref, rn)), dzk, pref), 1.0f);
-      if (pq == pn) {
-        fixed = true;
-        break;
-      }
+    pn = next(eos_rho_of(pn, rdth));
+    pn = next(eos_rho_of(pn, rdth));
+    float rn = eos_rho_of(pn, rdth);
+    float pq = next(rn);
+    if (pq != pn) {
       pn = pq;
+      rn = eos_rho_of(pn, rdth);
+      pq = next(rn);
+      if (pq != pn) rn = eos_rho_of(pq, rdth);
     }
-    pref = pn;
-    rref = fixed ? rn : eos_rho(pn, thp);
+    pref = pq;
+    rref = rn;
   }
   zb = z;
 }
