@@ -537,8 +537,11 @@ cudaError_t launch_substep(gwm_b200_ctx* c, const Member& M, const FastArgs& f, 
   if (!terr && fast_tma_path(c)) {
     FastMaps m{};
     if (!fast_maps(M, f, first, p_ready, m)) return cudaErrorInvalidValue;
-    // the standard substep with its p' at hand runs on independent warps
-    if ((!first || p_ready) && f.hmom && f.dens) return launch_fast_rows(f, m, first, c->stream);
+    // The standard substep with its p' at hand runs on independent warps; a handful of tiles is
+    // done sooner by eight warps of two rows (32 x 32 x 40, two tiles: 12.8 against 13.9 us; 12
+    // tiles: 13.2 against 13.0).
+    const int tiles = ((f.g.nx + 31) / 32) * ((f.g.ny + 15) / 16);
+    if ((!first || p_ready) && f.hmom && f.dens && tiles >= 8) return launch_fast_rows(f, m, first, c->stream);
     return launch_fast_tma(f, m, first, p_ready, c->stream);
   }
   return launch_fast(f, first, terr, c->stream, c->fast_tile_rows);
