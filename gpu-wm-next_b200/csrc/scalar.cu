@@ -2,56 +2,146 @@
 // scalar field under a constant advection velocity with first-order upwind differences
 // (upwind_stage_kernel, :13-37), on the global owned array (nz, ny, nx) in device memory.
 //
-// One kernel per stage with the stage's blend fused in (blend_stage_kernel, :39-46):
-//   stage 1: q1 = L(q)
-//   stage 2: q2 = 0.75 q + 0.25 L(q1)
-//   stage 3: q  = 1/3 q + 2/3 L(q2)        (in place: each cell reads only its own q)
+// One kernel per step: a warp marches down the rows of 32 columns in the direction of the
+// wind and computes the three stages
+//   q1 = L(q),  q2 = 0.75 q + 0.25 L(q1),  q' = 1/3 q + 2/3 L(q2)
+// of a row together: the upwind row's values stay in registers, the upwind column's come from
+// the neighbouring lane, and each stage is valid one column and one row further downwind, so
+// 29 columns and all but the first three rows of a segment are written.  A step reads q and
+// writes q' once, 8 B per cell, where a kernel per stage moved 32.  The steps alternate
+// between q and one scratch array.
 // with L(x) = x - dt (u dx/dx + v dx/dy).  The roundings are the reference build's: the
 // divisions, fma(-dt, fma(u, dqx, v*dqy), q) for the stage and fma(wa, a, wb*b) for the
 // blend (the contractions its compiler makes of the written expressions, identified on
 // its golden vectors), written out so that no compiler choice can change them.  The
 // stencil's halo is the periodic image, or zero beyond an open side: what the
 // reference's halo exchange gives its virtual ranks (an absent neighbour sends zeros).
+#include <map>
+#include <mutex>
+
 #include "../../include/gwm_b200.h"
 #include "common.cuh"
+#include "stencil.cuh"
 
 namespace gwmb {
 namespace {
 
-struct ScalarStage {
-  int nx, ny, nz, px, py;
+struct ScalarStep {
+  int nx, ny, px, py;
   float u, v, dt, dx, dy;
   const float* in;
-  const float* q0;  // blend partner (null: no blend)
   float* out;
-  float wa, wb;
 };
 
-constexpr int kSX = 32, kSY = 8;
+constexpr int kSLanes = 29;  // columns a warp writes: 32 less one per stage
+constexpr int kSRows = 32;   // rows it writes
+constexpr int kSWarps = 4;
 
-__global__ void __launch_bounds__(kSX * kSY) k_scalar_stage(const ScalarStage a) {
-  const int i = blockIdx.x * kSX + threadIdx.x, j = blockIdx.y * kSY + threadIdx.y, k = blockIdx.z;
-  if (i >= a.nx || j >= a.ny) return;
-  const size_t plane = (size_t)a.nx * a.ny;
-  const float* in = a.in + (size_t)k * plane;
-  auto at = [&](int ii, int jj) -> float {
-    if (ii < 0 || ii >= a.nx) {
-      if (!a.px) return 0.0f;
-      ii = ii < 0 ? ii + a.nx : ii - a.nx;
-    }
-    if (jj < 0 || jj >= a.ny) {
-      if (!a.py) return 0.0f;
-      jj = jj < 0 ? jj + a.ny : jj - a.ny;
-    }
-    return __ldg(in + (size_t)jj * a.nx + ii);
+// NEAR: dx and dy lie in [2^-20, 2^20], so a quotient by them may take the residual steps of
+// fp::div_by, which give the division's value for the differences tested here (the others
+// divide); six IEEE divisions per cell and step were most of the kernel.
+template <bool NEAR>
+__global__ void __launch_bounds__(32 * kSWarps) k_scalar_step(const ScalarStep a) {
+  const int lane = threadIdx.x & 31, seg = blockIdx.y * kSWarps + (threadIdx.x >> 5);
+  const int j0 = seg * kSRows, j1 = min(j0 + kSRows, a.ny);
+  if (j0 >= a.ny) return;  // the whole warp
+  const size_t level = (size_t)blockIdx.z * ((size_t)a.nx * a.ny);
+  const bool west = a.u >= 0.0f, south = a.v >= 0.0f;  // where the wind comes from
+  const int i = blockIdx.x * kSLanes + lane - (west ? 3 : 0);
+  const bool own = (west ? lane >= 3 : lane < kSLanes) && i < a.nx;
+  const bool in_x = a.px || (i >= 0 && i < a.nx);
+  auto wrap = [](int q, int n) {
+    if (q >= 0 && q < n) return q;
+    q %= n;
+    return q < 0 ? q + n : q;
   };
-  const float q = at(i, j);
-  const float dqx = (a.u >= 0.0f) ? (q - at(i - 1, j)) / a.dx : (at(i + 1, j) - q) / a.dx;
-  const float dqy = (a.v >= 0.0f) ? (q - at(i, j - 1)) / a.dy : (at(i, j + 1) - q) / a.dy;
+  const float* col = a.in + level + wrap(i, a.nx);
+  // row n of the march: three rows upwind of the segment first
+  const int rows = j1 - j0 + 3;
+  auto row = [&](int n) { return south ? j0 - 3 + n : j1 + 2 - n; };
+  auto inside = [&](int j) { return in_x && (a.py || (j >= 0 && j < a.ny)); };
+  auto load = [&](int n) {
+    const int j = row(n);
+    return n < rows && inside(j) ? __ldg(col + (size_t)wrap(j, a.ny) * a.nx) : 0.0f;
+  };
+  const float ydx = fp::recip(a.dx), ydy = fp::recip(a.dy);
+  // 0, or a magnitude in [2^-79, 2^100]
+  auto residual_safe = [](float e) {
+    const unsigned x = __float_as_uint(e) & 0x7fffffffu;
+    return x == 0u || x - 0x18000000u <= 0x71800000u - 0x18000000u;
+  };
   // the reference build's contractions of q - dt*(u*dqx + v*dqy) and wa*a + wb*b
-  const float t = __fmaf_rn(-a.dt, __fmaf_rn(a.u, dqx, __fmul_rn(a.v, dqy)), q);
-  const size_t o = (size_t)k * plane + (size_t)j * a.nx + i;
-  a.out[o] = a.q0 ? __fmaf_rn(a.wa, a.q0[o], __fmul_rn(a.wb, t)) : t;
+  auto stage = [&](float q, float qy) {
+    const float qx = west ? __shfl_up_sync(0xffffffffu, q, 1) : __shfl_down_sync(0xffffffffu, q, 1);
+    const float ex = west ? q - qx : qx - q, ey = south ? q - qy : qy - q;
+    float dqx, dqy;
+    if (NEAR && residual_safe(ex) && residual_safe(ey)) {
+      dqx = fp::div_by(ex, a.dx, ydx);
+      dqy = fp::div_by(ey, a.dy, ydy);
+    } else {
+      dqx = ex / a.dx;
+      dqy = ey / a.dy;
+    }
+    return __fmaf_rn(-a.dt, __fmaf_rn(a.u, dqx, __fmul_rn(a.v, dqy)), q);
+  };
+  float n0 = load(0), n1 = load(1);        // two rows ahead
+  float p0 = 0.0f, p1 = 0.0f, p2 = 0.0f;   // the upwind row's q, q1, q2
+  for (int n = 0; n < rows; ++n) {
+    const float q = n0;
+    n0 = n1;
+    n1 = load(n + 2);
+    const int j = row(n);
+    const bool in = inside(j);  // beyond an open side every stage reads zeros
+    float q1 = stage(q, p0);
+    if (!in) q1 = 0.0f;
+    float q2 = __fmaf_rn(0.75f, q, __fmul_rn(0.25f, stage(q1, p1)));
+    if (!in) q2 = 0.0f;
+    const float out = __fmaf_rn(1.0f / 3.0f, q, __fmul_rn(2.0f / 3.0f, stage(q2, p2)));
+    if (own && n >= 3) a.out[level + (size_t)j * a.nx + i] = out;
+    p0 = q;
+    p1 = q1;
+    p2 = q2;
+  }
+}
+
+// Scratch of the calls, from a pool of the library per device that keeps up to 256 MB between
+// calls (larger scratch goes back to the device at the next synchronisation): the default
+// pool gives everything back at each call's end, and mapping it again cost more than the
+// steps.  Allocations are stream-ordered, so threads and streams share the pool safely.
+constexpr uint64_t kKeptScratch = 256ull << 20;
+cudaError_t scratch_alloc(float** p, size_t bytes, cudaStream_t s) {
+  static std::mutex lock;
+  static std::map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> hold(lock);
+    auto it = pools.find(dev);
+    if (it == pools.end()) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      uint64_t keep = kKeptScratch;
+      if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+          cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+        pools[dev] = pool;
+      else
+        pool = nullptr;
+    } else {
+      pool = it->second;
+    }
+  }
+  if (pool) {
+    e = cudaMallocFromPoolAsync((void**)p, bytes, pool, s);
+    if (e == cudaSuccess || e == cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();  // a pool of a context that is gone (cudaDeviceReset): forget it
+    std::lock_guard<std::mutex> hold(lock);
+    pools.erase(dev);
+  }
+  return cudaMallocAsync((void**)p, bytes, s);
 }
 
 }  // namespace
@@ -65,27 +155,23 @@ extern "C" int gwm_b200_scalar_ssprk3(const gwm_b200_scalar_desc* d, float* q, i
   if (nsteps == 0) return GWM_B200_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t n = (size_t)d->nx * d->ny * d->nz;
-  float *q1 = nullptr, *q2 = nullptr;
-  if (cudaMallocAsync(&q1, n * sizeof(float), s) != cudaSuccess) return GWM_B200_ERR_CUDA;
-  if (cudaMallocAsync(&q2, n * sizeof(float), s) != cudaSuccess) {
-    cudaFreeAsync(q1, s);
-    return GWM_B200_ERR_CUDA;
+  float* tmp = nullptr;
+  if (scratch_alloc(&tmp, n * sizeof(float), s) != cudaSuccess) return GWM_B200_ERR_CUDA;
+  ScalarStep a{d->nx, d->ny, d->periodic_x, d->periodic_y, d->u_adv, d->v_adv, d->dt, d->dx, d->dy, q, tmp};
+  auto mid = [](float x) { return x >= 9.5367431640625e-7f && x <= 1048576.0f; };
+  const bool near = mid(d->dx) && mid(d->dy);
+  const int segs = (d->ny + kSRows - 1) / kSRows;
+  const dim3 grid((d->nx + kSLanes - 1) / kSLanes, (segs + kSWarps - 1) / kSWarps, d->nz);
+  for (int step = 0; step < nsteps; ++step) {
+    if (near) k_scalar_step<true><<<grid, 32 * kSWarps, 0, s>>>(a);
+    else k_scalar_step<false><<<grid, 32 * kSWarps, 0, s>>>(a);
+    a.in = a.out;
+    a.out = a.out == q ? tmp : q;
   }
-  ScalarStage a{d->nx, d->ny, d->nz, d->periodic_x, d->periodic_y, d->u_adv, d->v_adv, d->dt, d->dx, d->dy,
-                nullptr, nullptr, nullptr, 0.0f, 0.0f};
-  const dim3 block(kSX, kSY), grid((d->nx + kSX - 1) / kSX, (d->ny + kSY - 1) / kSY, d->nz);
-  cudaError_t e = cudaSuccess;
-  for (int step = 0; step < nsteps && e == cudaSuccess; ++step) {
-    a.in = q; a.q0 = nullptr; a.out = q1;
-    k_scalar_stage<<<grid, block, 0, s>>>(a);
-    a.in = q1; a.q0 = q; a.out = q2; a.wa = 0.75f; a.wb = 0.25f;
-    k_scalar_stage<<<grid, block, 0, s>>>(a);
-    a.in = q2; a.q0 = q; a.out = q; a.wa = 1.0f / 3.0f; a.wb = 2.0f / 3.0f;
-    k_scalar_stage<<<grid, block, 0, s>>>(a);
-    e = cudaGetLastError();
-  }
-  cudaFreeAsync(q2, s);
-  cudaFreeAsync(q1, s);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && nsteps % 2)  // the result is in the scratch
+    e = cudaMemcpyAsync(q, tmp, n * sizeof(float), cudaMemcpyDeviceToDevice, s);
+  cudaFreeAsync(tmp, s);
   if (e != cudaSuccess) return GWM_B200_ERR_CUDA;
   return cudaStreamSynchronize(s) == cudaSuccess ? GWM_B200_OK : GWM_B200_ERR_CUDA;
 }
