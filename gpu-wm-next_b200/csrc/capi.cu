@@ -1367,45 +1367,35 @@ int gwm_b200_mlp_train(const float* x, const float* y, long long n, const gwm_b2
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return GWM_B200_ERR_NO_DEVICE;
   const int batch = (int)std::min<long long>(cfg->batch, n);
   cudaStream_t s = nullptr;
-  std::vector<void*> owned;
-  auto alloc = [&](size_t bytes) -> void* {
-    void* p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
-    owned.push_back(p);
-    return p;
+  // one device block for everything; a loss per batch of the epoch, read back at its end
+  const size_t nbatch = (size_t)(n / batch);
+  size_t total = 0;
+  auto place = [&](size_t bytes) {
+    const size_t at = total;
+    total += (bytes + 255) / 256 * 256;
+    return at;
   };
+  const size_t o_stats = place((2 * kMlpIn + 2 * kMlpIn + 2 * kMlpOut) * sizeof(double)), o_p = place(kMlpParams * 4),
+               o_n = place(kMlpNorm * 4), o_g = place(kMlpParams * 4), o_m = place(kMlpParams * 4),
+               o_v = place(kMlpParams * 4), o_scr = place(mlp_scratch_floats(batch) * 4),
+               o_part = place(mlp_partial_floats(batch) * 4), o_l = place(nbatch * sizeof(double)),
+               o_idx = place((size_t)n * sizeof(int));
+  char* block = nullptr;
+  if (cudaMalloc(&block, total) != cudaSuccess) return GWM_B200_ERR_CUDA;
   auto cleanup = [&](int rc) {
-    for (void* p : owned) cudaFree(p);
+    cudaFree(block);
     return rc;
   };
-  double* stats = (double*)alloc((2 * kMlpIn + 2 * kMlpIn + 2 * kMlpOut) * sizeof(double));
-  float* dp = (float*)alloc(kMlpParams * 4);
-  float* dn = (float*)alloc(kMlpNorm * 4);
-  float* dg = (float*)alloc(kMlpParams * 4);
-  float* dm = (float*)alloc(kMlpParams * 4);
-  float* dv = (float*)alloc(kMlpParams * 4);
-  float* scr = (float*)alloc(mlp_scratch_floats(batch) * 4);
-  float* part = (float*)alloc(mlp_partial_floats(batch) * 4);
-  double* dl = (double*)alloc(sizeof(double));
-  int* didx = (int*)alloc((size_t)n * sizeof(int));
-  if (!stats || !dp || !dn || !dg || !dm || !dv || !scr || !part || !dl || !didx) return cleanup(GWM_B200_ERR_CUDA);
+  double* stats = (double*)(block + o_stats);
+  float *dp = (float*)(block + o_p), *dn = (float*)(block + o_n), *dg = (float*)(block + o_g),
+        *dm = (float*)(block + o_m), *dv = (float*)(block + o_v), *scr = (float*)(block + o_scr),
+        *part = (float*)(block + o_part);
+  double* dl = (double*)(block + o_l);
+  int* didx = (int*)(block + o_idx);
   // normalisation: FP64 means and standard deviations of inputs and targets; input range
   if (mlp_column_stats(x, n, kMlpIn, stats, stats + 2 * kMlpIn, s) != cudaSuccess ||
       mlp_column_stats(y, n, kMlpOut, stats + 4 * kMlpIn, nullptr, s) != cudaSuccess)
     return cleanup(GWM_B200_ERR_CUDA);
-  double hs[4 * kMlpIn + 2 * kMlpOut];
-  if (cudaMemcpy(hs, stats, sizeof(hs), cudaMemcpyDeviceToHost) != cudaSuccess) return cleanup(GWM_B200_ERR_CUDA);
-  for (int f = 0; f < kMlpIn; ++f) {
-    norm[f] = (float)hs[f];
-    norm[kMlpIn + f] = hs[kMlpIn + f] > 1e-30 ? (float)hs[kMlpIn + f] : 1.0f;  // constant input (dt)
-    if (range) { range[f] = (float)hs[2 * kMlpIn + f]; range[kMlpIn + f] = (float)hs[3 * kMlpIn + f]; }
-  }
-  for (int o = 0; o < kMlpOut; ++o) {
-    norm[2 * kMlpIn + o] = (float)hs[4 * kMlpIn + o];
-    const double sd = hs[4 * kMlpIn + kMlpOut + o];
-    // a target that never varies gets scale 0: inference reproduces its mean exactly
-    norm[2 * kMlpIn + kMlpOut + o] = sd > 1e-30 ? (float)sd : 0.0f;
-  }
   uint64_t rng = cfg->seed ? cfg->seed : 0x5EED5EEDull;
   if (cfg->init) {  // Xavier-uniform weights, zero biases
     auto uni = [&]() { return (double)(splitmix(rng) >> 11) * (1.0 / 9007199254740992.0) * 2.0 - 1.0; };
@@ -1419,25 +1409,45 @@ int gwm_b200_mlp_train(const float* x, const float* y, long long n, const gwm_b2
     fill_w(kOffW3, kMlpHid, kMlpHid);
     fill_w(kOffW4, kMlpOut, kMlpHid);
   }
+  std::vector<int> perm((size_t)n);
+  for (long long q = 0; q < n; ++q) perm[(size_t)q] = (int)q;
+  auto shuffle = [&] {
+    for (long long q = n - 1; q > 0; --q) std::swap(perm[(size_t)q], perm[(size_t)(splitmix(rng) % (uint64_t)(q + 1))]);
+  };
+  shuffle();  // the first epoch's order, while the device reduces the statistics
+  double hs[4 * kMlpIn + 2 * kMlpOut];
+  if (cudaMemcpy(hs, stats, sizeof(hs), cudaMemcpyDeviceToHost) != cudaSuccess) return cleanup(GWM_B200_ERR_CUDA);
+  for (int f = 0; f < kMlpIn; ++f) {
+    norm[f] = (float)hs[f];
+    norm[kMlpIn + f] = hs[kMlpIn + f] > 1e-30 ? (float)hs[kMlpIn + f] : 1.0f;  // constant input (dt)
+    if (range) { range[f] = (float)hs[2 * kMlpIn + f]; range[kMlpIn + f] = (float)hs[3 * kMlpIn + f]; }
+  }
+  for (int o = 0; o < kMlpOut; ++o) {
+    norm[2 * kMlpIn + o] = (float)hs[4 * kMlpIn + o];
+    const double sd = hs[4 * kMlpIn + kMlpOut + o];
+    // a target that never varies gets scale 0: inference reproduces its mean exactly
+    norm[2 * kMlpIn + kMlpOut + o] = sd > 1e-30 ? (float)sd : 0.0f;
+  }
   cudaMemcpy(dp, params, kMlpParams * 4, cudaMemcpyHostToDevice);
   cudaMemcpy(dn, norm, kMlpNorm * 4, cudaMemcpyHostToDevice);
   cudaMemset(dm, 0, kMlpParams * 4);
   cudaMemset(dv, 0, kMlpParams * 4);
-  std::vector<int> perm((size_t)n);
-  for (long long q = 0; q < n; ++q) perm[(size_t)q] = (int)q;
+  std::vector<double> losses(nbatch);
   int t = 0;
   for (int ep = 0; ep < cfg->epochs; ++ep) {
-    for (long long q = n - 1; q > 0; --q) std::swap(perm[(size_t)q], perm[(size_t)(splitmix(rng) % (uint64_t)(q + 1))]);
+    if (ep > 0) shuffle();
     if (cudaMemcpy(didx, perm.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+      return cleanup(GWM_B200_ERR_CUDA);
+    for (size_t k = 0; k < nbatch; ++k) {
+      MlpBatch b{dp, dn, x, y, didx + k * batch, batch, scr, part, dg, dl + k};
+      if (mlp_loss_grad(b, s) != cudaSuccess || mlp_adam(dp, dg, dm, dv, cfg->lr, ++t, s) != cudaSuccess)
+        return cleanup(GWM_B200_ERR_CUDA);
+    }
+    if (cudaMemcpy(losses.data(), dl, nbatch * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
       return cleanup(GWM_B200_ERR_CUDA);
     double ep_loss = 0.0;
     long long seen = 0;
-    for (long long b0 = 0; b0 + batch <= n; b0 += batch) {
-      MlpBatch b{dp, dn, x, y, didx + b0, batch, scr, part, dg, dl};
-      if (mlp_loss_grad(b, s) != cudaSuccess || mlp_adam(dp, dg, dm, dv, cfg->lr, ++t, s) != cudaSuccess)
-        return cleanup(GWM_B200_ERR_CUDA);
-      double l = 0.0;
-      if (cudaMemcpy(&l, dl, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) return cleanup(GWM_B200_ERR_CUDA);
+    for (double l : losses) {
       ep_loss += l * batch;
       seen += batch;
     }

@@ -4,7 +4,7 @@
 //    rain_cell.cuh): features (T, p, rho_d, qv, qc, qr, dt) of a state and the targets
 //    (the three process fractions, dtheta, dqv), written in cell order.
 //  * mlp_loss_grad: mean squared error of the normalised targets and its exact gradient,
-//    deterministic: one thread per sample for the forward and backward sweeps, then the
+//    deterministic: four threads per sample for the forward and backward sweeps, then the
 //    weight gradients as tiled products over fixed chunks of samples reduced in a
 //    fixed order (no floating-point atomics).
 //  * mlp_adam: the optimiser step.
@@ -157,6 +157,7 @@ __global__ void k_stats1(const float* __restrict__ a, long long n, int d, double
 __global__ void k_stats2(const double* __restrict__ part, int nb, long long n, int d, double* out, double* rng) {
   for (int f = threadIdx.x; f < d; f += blockDim.x) {
     double t0 = 0.0, t1 = 0.0, t2 = 1e300, t3 = -1e300;
+#pragma unroll 16  // the loads go ahead of the ordered sums
     for (int b = 0; b < nb; ++b) {
       const double* p = part + ((size_t)b * d + f) * 4;
       t0 += p[0]; t1 += p[1]; t2 = fmin(t2, p[2]); t3 = fmax(t3, p[3]);
@@ -169,7 +170,7 @@ __global__ void k_stats2(const double* __restrict__ part, int nb, long long n, i
   }
 }
 
-// ---- forward and backward sweeps, one thread per sample
+// ---- forward and backward sweeps
 constexpr float kGeluC = 0.7978845608028654f;  // sqrt(2/pi)
 __device__ __forceinline__ float gelu_t(float z, float& dg) {
   const float u = kGeluC * (z + 0.044715f * z * z * z);
@@ -184,9 +185,15 @@ constexpr int kScrX0 = 0, kScrZ1 = kScrX0 + kMlpIn, kScrA1 = kScrZ1 + kMlpHid, k
               kScrA2 = kScrZ2 + kMlpHid, kScrZ3 = kScrA2 + kMlpHid, kScrA3 = kScrZ3 + kMlpHid,
               kScrD1 = kScrA3 + kMlpHid, kScrD2 = kScrD1 + kMlpHid, kScrD3 = kScrD2 + kMlpHid,
               kScrD4 = kScrD3 + kMlpHid, kScrRows = kScrD4 + kMlpOut;
-constexpr int kFbThreads = 128;
+constexpr int kFbThreads = 128;  // samples per block
+constexpr int kFbGroups = 4;     // threads per sample: a quarter of each layer's outputs each
+constexpr int kFbOut = kMlpHid / kFbGroups;
 
-__global__ void __launch_bounds__(kFbThreads) k_mlp_fwd_bwd(const MlpBatch bt, double* loss_part) {
+// Four threads share a sample, each computing 16 of a layer's 64 outputs (every output's sum
+// keeps its order); a layer's values pass through the scratch rows that the gradients read
+// anyway.  One thread per sample put four warps on an SM, each a chain of 64 x 64 products:
+// 104 us per 16384 samples.
+__global__ void __launch_bounds__(kFbThreads * kFbGroups) k_mlp_fwd_bwd(const MlpBatch bt, double* loss_part) {
   __shared__ float w[kMlpParams];
   __shared__ float nrm[kMlpNorm];
   __shared__ double s_loss[kFbThreads];
@@ -194,20 +201,23 @@ __global__ void __launch_bounds__(kFbThreads) k_mlp_fwd_bwd(const MlpBatch bt, d
   for (int q = threadIdx.x; q < kMlpNorm; q += blockDim.x) nrm[q] = bt.norm[q];
   __syncthreads();
   const int n = bt.n;
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int sample = threadIdx.x % kFbThreads, group = threadIdx.x / kFbThreads;
+  const int b = blockIdx.x * kFbThreads + sample;
+  const bool live = b < n;
+  const int j0 = group * kFbOut;
+  float* S = bt.scratch;
+  auto at = [&](int row) -> float& { return S[(size_t)row * n + b]; };
+  const long long src = live ? (bt.index ? bt.index[b] : b) : 0;
+  float in[kMlpHid];
   double l = 0.0;
-  if (b < n) {
-    float* S = bt.scratch;
-    auto at = [&](int row) -> float& { return S[(size_t)row * n + b]; };
-    const long long src = bt.index ? bt.index[b] : b;
-    float in[kMlpHid];
+  if (live) {
 #pragma unroll
     for (int f = 0; f < kMlpIn; ++f) {
       in[f] = (bt.x[src * kMlpIn + f] - nrm[f]) / nrm[kMlpIn + f];
-      at(kScrX0 + f) = in[f];
+      if (group == 0) at(kScrX0 + f) = in[f];
     }
     // layer 1 (7 -> 64)
-    for (int j = 0; j < kMlpHid; ++j) {
+    for (int j = j0; j < j0 + kFbOut; ++j) {
       float z = w[kOffB1 + j];
 #pragma unroll
       for (int f = 0; f < kMlpIn; ++f) z += w[kOffW1 + j * kMlpIn + f] * in[f];
@@ -215,13 +225,16 @@ __global__ void __launch_bounds__(kFbThreads) k_mlp_fwd_bwd(const MlpBatch bt, d
       at(kScrZ1 + j) = z;
       at(kScrA1 + j) = gelu_t(z, dg);
     }
-    // layers 2 and 3 (64 -> 64)
-    const int offw[2] = {kOffW2, kOffW3}, offb[2] = {kOffB2, kOffB3};
-    const int rin[2] = {kScrA1, kScrA2}, rz[2] = {kScrZ2, kScrZ3}, ra[2] = {kScrA2, kScrA3};
-    for (int L = 0; L < 2; ++L) {
+  }
+  __syncthreads();
+  // layers 2 and 3 (64 -> 64)
+  const int offw[2] = {kOffW2, kOffW3}, offb[2] = {kOffB2, kOffB3};
+  const int rin[2] = {kScrA1, kScrA2}, rz[2] = {kScrZ2, kScrZ3}, ra[2] = {kScrA2, kScrA3};
+  for (int L = 0; L < 2; ++L) {
+    if (live) {
 #pragma unroll
       for (int f = 0; f < kMlpHid; ++f) in[f] = at(rin[L] + f);
-      for (int j = 0; j < kMlpHid; ++j) {
+      for (int j = j0; j < j0 + kFbOut; ++j) {
         float z = w[offb[L] + j];
 #pragma unroll
         for (int f = 0; f < kMlpHid; ++f) z += w[offw[L] + j * kMlpHid + f] * in[f];
@@ -230,10 +243,12 @@ __global__ void __launch_bounds__(kFbThreads) k_mlp_fwd_bwd(const MlpBatch bt, d
         at(ra[L] + j) = gelu_t(z, dg);
       }
     }
-    // output layer (64 -> 5) and the loss gradient
+    __syncthreads();
+  }
+  // output layer (64 -> 5) and the loss gradient
+  if (live && group == 0) {
 #pragma unroll
     for (int f = 0; f < kMlpHid; ++f) in[f] = at(kScrA3 + f);
-    float d4[kMlpOut];
 #pragma unroll
     for (int o = 0; o < kMlpOut; ++o) {
       float y = w[kOffB4 + o];
@@ -243,88 +258,117 @@ __global__ void __launch_bounds__(kFbThreads) k_mlp_fwd_bwd(const MlpBatch bt, d
       const float t = sd > 0.0f ? (bt.y[src * kMlpOut + o] - nrm[2 * kMlpIn + o]) / sd : 0.0f;
       const float e = y - t;
       l += (double)e * (double)e;
-      d4[o] = 2.0f * e / ((float)n * (float)kMlpOut);
-      at(kScrD4 + o) = d4[o];
+      at(kScrD4 + o) = 2.0f * e / ((float)n * (float)kMlpOut);
     }
-    // backward: delta3 = (W4^T d4) * gelu'(z3)
-    float dnext[kMlpHid];
+  }
+  if (group == 0) s_loss[sample] = l;
+  __syncthreads();
+  // backward: delta3 = (W4^T d4) * gelu'(z3)
+  if (live) {
+    float d4[kMlpOut];
 #pragma unroll
-    for (int f = 0; f < kMlpHid; ++f) {
+    for (int o = 0; o < kMlpOut; ++o) d4[o] = at(kScrD4 + o);
+#pragma unroll
+    for (int f = j0; f < j0 + kFbOut; ++f) {
       float s = 0.0f;
 #pragma unroll
       for (int o = 0; o < kMlpOut; ++o) s += w[kOffW4 + o * kMlpHid + f] * d4[o];
       float dg;
       gelu_t(at(kScrZ3 + f), dg);
-      dnext[f] = s * dg;
-      at(kScrD3 + f) = dnext[f];
-    }
-    // delta2 = (W3^T delta3) * gelu'(z2); delta1 = (W2^T delta2) * gelu'(z1)
-    const int bw[2] = {kOffW3, kOffW2}, bz[2] = {kScrZ2, kScrZ1}, bd[2] = {kScrD2, kScrD1};
-    for (int L = 0; L < 2; ++L) {
-      float dcur[kMlpHid];
-      for (int f = 0; f < kMlpHid; ++f) {
-        float s = 0.0f;
-#pragma unroll
-        for (int j = 0; j < kMlpHid; ++j) s += w[bw[L] + j * kMlpHid + f] * dnext[j];
-        float dg;
-        gelu_t(at(bz[L] + f), dg);
-        dcur[f] = s * dg;
-        at(bd[L] + f) = dcur[f];
-      }
-#pragma unroll
-      for (int f = 0; f < kMlpHid; ++f) dnext[f] = dcur[f];
+      at(kScrD3 + f) = s * dg;
     }
   }
-  s_loss[threadIdx.x] = l;
   __syncthreads();
+  // delta2 = (W3^T delta3) * gelu'(z2); delta1 = (W2^T delta2) * gelu'(z1)
+  const int bw[2] = {kOffW3, kOffW2}, bz[2] = {kScrZ2, kScrZ1}, bi[2] = {kScrD3, kScrD2}, bd[2] = {kScrD2, kScrD1};
+  for (int L = 0; L < 2; ++L) {
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < kMlpHid; ++j) in[j] = at(bi[L] + j);
+      for (int f = j0; f < j0 + kFbOut; ++f) {
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kMlpHid; ++j) s += w[bw[L] + j * kMlpHid + f] * in[j];
+        float dg;
+        gelu_t(at(bz[L] + f), dg);
+        at(bd[L] + f) = s * dg;
+      }
+    }
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int q = 0; q < (int)blockDim.x; ++q) t += s_loss[q];
+    for (int q = 0; q < kFbThreads; ++q) t += s_loss[q];
     loss_part[blockIdx.x] = t;
   }
 }
 
-// Gradient of one layer over one chunk of samples: part[o][i] = sum_b D[o][b] A[i][b]
-// (i < I) and part[o][I] = sum_b D[o][b], for O <= 64 outputs and I <= 64 inputs.
-__global__ void __launch_bounds__(256) k_mlp_grad_chunk(const float* __restrict__ S, int n, int rowD, int O,
-                                                       int rowA, int I, int off_w, int off_b,
-                                                       float* __restrict__ partial) {
-  __shared__ float Ds[64][33], As[65][33];
+// Gradients of the four layers over one chunk of samples: for each layer
+// part[o][i] = sum_b D[o][b] A[i][b] (i < I) and part[o][I] = sum_b D[o][b], for O <= 64 outputs
+// and I <= 64 inputs.  Each sum runs over its chunk's samples in order, in one thread; the sums
+// are spread over blockIdx = (chunk, layer, quarter of the input columns), and the next 32
+// samples are loaded while the current ones are summed.  (One block per chunk and layer, one
+// launch per layer, left 132 SMs idle: 927 us per 16384 samples.)
+struct GradLayer {
+  int rowD, O, rowA, I, off_w, off_b;
+};
+constexpr int kGradSplit = 4, kGradCols = 5, kGradRows = 4 * kGradCols;  // column i = g + 16 q, g = 4 split + t / 64
+__global__ void __launch_bounds__(256) k_mlp_grad_chunk(const float* __restrict__ S, int n, float* __restrict__ partial) {
+  constexpr GradLayer layers[4] = {{kScrD1, kMlpHid, kScrX0, kMlpIn, kOffW1, kOffB1},
+                                   {kScrD2, kMlpHid, kScrA1, kMlpHid, kOffW2, kOffB2},
+                                   {kScrD3, kMlpHid, kScrA2, kMlpHid, kOffW3, kOffB3},
+                                   {kScrD4, kMlpOut, kScrA3, kMlpHid, kOffW4, kOffB4}};
+  const GradLayer y = layers[blockIdx.y];
+  __shared__ float Ds[64][33], As[kGradRows][33];
+  const int split = blockIdx.z;
+  if (4 * split > y.I) return;  // none of the layer's columns
   const int c = blockIdx.x;
   const int b0 = c * kChunk, b1 = min(n, b0 + kChunk);
-  const int t = threadIdx.x, o = t & 63, jg = t >> 6;  // 4 groups of input columns
-  float acc[17];
+  const int t = threadIdx.x, o = t & 63, jg = t >> 6, g = 4 * split + jg;
+  const int lr = t >> 5, ls = t & 31;  // loads: row lr + 8 q, sample ls
+  constexpr int ND = 64 / 8, NA = (kGradRows + 7) / 8;
+  auto load_d = [&](int q, int s0, int m) {
+    const int r = lr + 8 * q;
+    return r < y.O && ls < m ? S[(size_t)(y.rowD + r) * n + s0 + ls] : 0.0f;
+  };
+  auto load_a = [&](int q, int s0, int m) {  // row r of As: column 4 split + r / kGradCols + 16 (r % kGradCols)
+    const int r = lr + 8 * q, i = 4 * split + r / kGradCols + 16 * (r % kGradCols);
+    if (r >= kGradRows || ls >= m) return 0.0f;
+    return i < y.I ? S[(size_t)(y.rowA + i) * n + s0 + ls] : (i == y.I ? 1.0f : 0.0f);
+  };
+  float nd[ND], na[NA], acc[kGradCols];
 #pragma unroll
-  for (int q = 0; q < 17; ++q) acc[q] = 0.0f;
-  for (int s0 = b0; s0 < b1; s0 += 32) {
+  for (int q = 0; q < kGradCols; ++q) acc[q] = 0.0f;
+  auto fetch = [&](int s0) {
     const int m = min(32, b1 - s0);
-    for (int q = t; q < 64 * 32; q += 256) {
-      const int r = q >> 5, sidx = q & 31;
-      Ds[r][sidx] = (r < O && sidx < m) ? S[(size_t)(rowD + r) * n + s0 + sidx] : 0.0f;
-    }
-    for (int q = t; q < 65 * 32; q += 256) {
-      const int r = q >> 5, sidx = q & 31;
-      float v = 0.0f;
-      if (sidx < m) v = r < I ? S[(size_t)(rowA + r) * n + s0 + sidx] : (r == I ? 1.0f : 0.0f);
-      As[r][sidx] = v;
-    }
-    __syncthreads();
-    for (int sidx = 0; sidx < 32; ++sidx) {
-      const float d = Ds[o][sidx];
 #pragma unroll
-      for (int q = 0; q < 17; ++q) {
-        const int i = jg * 17 + q;
-        if (i <= 64) acc[q] += d * As[i][sidx];
-      }
+    for (int q = 0; q < ND; ++q) nd[q] = load_d(q, s0, m);
+#pragma unroll
+    for (int q = 0; q < NA; ++q) na[q] = load_a(q, s0, m);
+  };
+  fetch(b0);
+  for (int s0 = b0; s0 < b1; s0 += 32) {
+#pragma unroll
+    for (int q = 0; q < ND; ++q) Ds[lr + 8 * q][ls] = nd[q];
+#pragma unroll
+    for (int q = 0; q < NA; ++q)
+      if (lr + 8 * q < kGradRows) As[lr + 8 * q][ls] = na[q];
+    __syncthreads();
+    if (s0 + 32 < b1) fetch(s0 + 32);
+#pragma unroll 8
+    for (int s = 0; s < 32; ++s) {
+      const float d = Ds[o][s];
+#pragma unroll
+      for (int q = 0; q < kGradCols; ++q) acc[q] += d * As[jg * kGradCols + q][s];
     }
     __syncthreads();
   }
-  if (o < O) {
+  if (o < y.O) {
 #pragma unroll
-    for (int q = 0; q < 17; ++q) {
-      const int i = jg * 17 + q;
-      if (i < I) partial[(size_t)c * kMlpParams + off_w + o * I + i] = acc[q];
-      else if (i == I) partial[(size_t)c * kMlpParams + off_b + o] = acc[q];
+    for (int q = 0; q < kGradCols; ++q) {
+      const int i = g + 16 * q;
+      if (i < y.I) partial[(size_t)c * kMlpParams + y.off_w + o * y.I + i] = acc[q];
+      else if (i == y.I) partial[(size_t)c * kMlpParams + y.off_b + o] = acc[q];
     }
   }
 }
@@ -401,12 +445,8 @@ cudaError_t mlp_loss_grad(const MlpBatch& bt, cudaStream_t s) {
   size_t off = (size_t)chunks * kMlpParams;
   off = (off + 1) & ~size_t(1);
   double* loss_part = reinterpret_cast<double*>(bt.partial + off);
-  k_mlp_fwd_bwd<<<nlb, kFbThreads, 0, s>>>(bt, loss_part);
-  // (layer: delta rows, outputs, activation rows, inputs, weight and bias offsets)
-  k_mlp_grad_chunk<<<chunks, 256, 0, s>>>(bt.scratch, bt.n, kScrD1, kMlpHid, kScrX0, kMlpIn, kOffW1, kOffB1, bt.partial);
-  k_mlp_grad_chunk<<<chunks, 256, 0, s>>>(bt.scratch, bt.n, kScrD2, kMlpHid, kScrA1, kMlpHid, kOffW2, kOffB2, bt.partial);
-  k_mlp_grad_chunk<<<chunks, 256, 0, s>>>(bt.scratch, bt.n, kScrD3, kMlpHid, kScrA2, kMlpHid, kOffW3, kOffB3, bt.partial);
-  k_mlp_grad_chunk<<<chunks, 256, 0, s>>>(bt.scratch, bt.n, kScrD4, kMlpOut, kScrA3, kMlpHid, kOffW4, kOffB4, bt.partial);
+  k_mlp_fwd_bwd<<<nlb, kFbThreads * kFbGroups, 0, s>>>(bt, loss_part);
+  k_mlp_grad_chunk<<<dim3(chunks, 4, kGradSplit), 256, 0, s>>>(bt.scratch, bt.n, bt.partial);
   k_mlp_grad_reduce<<<(kMlpParams + 255) / 256, 256, 0, s>>>(bt.partial, chunks, bt.grad, loss_part, nlb, bt.loss,
                                                               1.0 / ((double)bt.n * kMlpOut));
   return cudaGetLastError();
