@@ -4,14 +4,17 @@
 // Same operator and per-cell arithmetic as k_tracer_stage: the upwind mixing-ratio
 // flux divergence with frozen end-of-step dry mass fluxes
 // (passive_tracer_stage_kernel, src/dycore/dry_transport.cu:49-125; clip at zero) and
-// the SSPRK3 blend of advance_passive_tracers_ssprk3 (:440-518).  A CTA owns a
-// 32 x 16 tile, two columns per thread; one elected thread fetches each plane's boxes
-// with cp.async.bulk.tensor.3d into a three-slot shared-memory ring:
-//   rho, rho*q (three tracers)   40 x 18 boxes: the tile and its halo ring
-//   u, v                         36 x 17 boxes: owned faces + the east/north face
-//   w                            32 x 16 box: owned Z faces (plane nz: w only)
-// Per plane the mixing ratios of the tile and its ring (no corners) go to shared
-// memory; one barrier per plane publishes them.
+// the SSPRK3 blend of advance_passive_tracers_ssprk3 (:440-518).  As in fast_rows.cu a warp
+// owns 32 x 4 cells, four rows per thread, an extra warp issues the TMA loads into a
+// three-slot ring with full and empty barriers, and the plane loop has no block barrier:
+//   rho, rho*q (up to three tracers)  40 x 18 boxes: the tile and its halo ring
+//   u, v                              36 x 17 boxes: owned faces + the east/north face
+//   w                                 32 x 16 box: owned Z faces (plane nz: w only)
+// A thread computes the mixing ratios of its rows one plane ahead and those of the rows around
+// them, lanes 0-7 those of the warp's two ring columns, with one reciprocal per position; the
+// Y fluxes between its rows are computed once, and the flux out of a plane's top is carried as
+// the next plane's bottom flux.  The kernel is issue-bound: 426 instructions per cell with one
+// row per eight and a block barrier per plane.
 #include <type_traits>
 
 #include "physics.cuh"
@@ -23,230 +26,267 @@ namespace gwmb {
 namespace {
 
 namespace tt {
-constexpr int TX = 32, TY = 16, RY = 8, NT = 256, NTR = 3;
-// the thread that issues the TMA loads: lane 0 of the last warp, which has no halo-ring
-// role (warps 0-2 carry those)
-constexpr int ISSUER = NT - 32;
+constexpr int TX = 32, ROWS = 4, NW = 4, TY = ROWS * NW;  // consumer warps: 4 rows each
+constexpr int NT = 32 * (NW + 1);                         // and the producer warp
+constexpr int MIN_CTAS = 3, NTR = 3;
 constexpr int CBW = 40, CBH = 18, FBW = 36, FBH = 17, OBW = 32, OBH = 16;
-constexpr int O_RHO = 0, O_Q = 736, O_U = 2944, O_V = 3584, O_W = 4224, SLOT = 4736, NSLOT = 3;
+constexpr int O_RHO = 0, O_U = 736, O_V = 1376, O_W = 2016, O_Q = 2528, Q_STRIDE = 736, NSLOT = 3;
+template <int N> constexpr int kSlot = O_Q + N * Q_STRIDE;  // floats, N tracers
 constexpr unsigned B_CELL = CBW * CBH * 4, B_FACE = FBW * FBH * 4, B_OWN = OBW * OBH * 4;
-constexpr int QW = TX + 2, QH = TY + 2;  // mixing-ratio plane: 34 x 18
-constexpr size_t kDynSmem = size_t(SLOT) * NSLOT * sizeof(float) + 128;
-static_assert(O_Q % 32 == 0 && O_U % 32 == 0 && O_V % 32 == 0 && O_W % 32 == 0 && SLOT % 32 == 0,
-              "128-byte aligned sub-buffers");
-static_assert(O_Q - O_RHO >= CBW * CBH && O_U - O_Q >= NTR * 736 && O_V - O_U >= FBW * FBH &&
-                  O_W - O_V >= FBW * FBH && SLOT - O_W >= OBW * OBH,
-              "boxes fit their sub-buffers");
+constexpr size_t smem_bytes(int ntr) { return size_t(O_Q + ntr * Q_STRIDE) * NSLOT * sizeof(float) + 128; }
+static_assert(O_U % 32 == 0 && O_V % 32 == 0 && O_W % 32 == 0 && O_Q % 32 == 0 && Q_STRIDE % 32 == 0 &&
+                  O_U - O_RHO >= CBW * CBH && O_V - O_U >= FBW * FBH && O_W - O_V >= FBW * FBH &&
+                  O_Q - O_W >= OBW * OBH && Q_STRIDE >= CBW * CBH,
+              "128-byte aligned boxes that fit");
 }  // namespace tt
 
-template <bool TERRAIN>
-__global__ void __launch_bounds__(tt::NT, 3) k_tracer_tma(const TracerArgs a, const __grid_constant__ TracerMaps m,
-                                                          ZSplit zs) {
+template <bool TERRAIN, int N>  // N: tracers
+__global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
+    k_tracer_tma(const TracerArgs a, const __grid_constant__ TracerMaps m, ZSplit zs) {
   using namespace tt;
+  constexpr int SLOT = kSlot<N>;
   extern __shared__ unsigned char s_dyn[];
-  __shared__ float s_q[NTR][2][QH][QW];
-  __shared__ __align__(8) uint64_t s_bar[NSLOT];
-  __shared__ int s_abort[2];
+  __shared__ __align__(8) uint64_t s_full[NSLOT], s_empty[NSLOT];
+  __shared__ float s_q[2][NW][N][ROWS][TX + 2];  // a warp's mixing ratios with its ring columns
   float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
 
   const Geom& g = a.g;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
+  // planes kb .. ke-1 are the CTA's; it also loads plane ke and (above the ground) the plane
+  // below, whose mixing ratios its lowest faces read
+  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0;
+
+  if (tid == 0) {
+    for (int s = 0; s < NSLOT; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&s_empty[s], NW);
+    }
+    mbar_fence_init();
+  }
+  __syncthreads();
+
+  if (wid == NW) {  // ---- producer
+    if (lane == 0) {
+      // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads
+      // of one of its planes unissued, so that CTA's bounded waits run out
+      int stall = -1;
+      if (*(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
+      if (stall >= 0) stall = kg + stall % (ke - kg + 1);
+      int issued = kg - 1;
+      for (int kk = kg; kk <= ke; ++kk) {  // plane nz holds the top faces only
+        const int q = kk - kg, s = q % NSLOT;
+        if (q >= NSLOT && !mbar_wait(&s_empty[s], (q / NSLOT - 1) & 1)) {
+          atomicExch(a.err, 1);
+          break;
+        }
+        float* st = ring + s * SLOT;
+        uint64_t* bar = &s_full[s];
+        const bool cells = kk < nz, body = kk >= kb && kk < ke;
+        mbar_arrive_expect_tx(bar, B_OWN + (cells ? (1 + N) * B_CELL : 0u) + (body ? 2 * B_FACE : 0u));
+        issued = kk;
+        if (kk == stall) continue;  // failure-path testing
+        const int x = i0 + kXOff, y = j0 + 1;
+        tma_load_3d(st + O_W, &m.w, x, y, kk, bar);
+        if (cells) {
+          tma_load_3d(st + O_RHO, &m.rho, x - 4, j0, kk, bar);
+#pragma unroll
+          for (int t = 0; t < N; ++t) tma_load_3d(st + O_Q + t * Q_STRIDE, &m.q[t], x - 4, j0, kk, bar);
+        }
+        if (body) {
+          tma_load_3d(st + O_U, &m.u, x, y, kk, bar);
+          tma_load_3d(st + O_V, &m.v, x, y, kk, bar);
+        }
+      }
+      // the loads in flight end before the CTA's shared memory goes away
+      for (int kk = max(kg, issued - NSLOT + 1); kk <= issued; ++kk) {
+        const int q = kk - kg;
+        mbar_wait(&s_full[q % NSLOT], (q / NSLOT) & 1);
+      }
+    }
+    return;
+  }
+  // ---- consumers
+  const int r0 = wid * ROWS;  // the warp's first row in the tile
   const int w = min(TX, nx - i0), h = min(TY, ny - j0);
-  const bool own0 = tx < w && ty < h, own1 = tx < w && ty + RY < h;
-  const int gi = i0 + tx, gj0 = j0 + ty, gj1 = j0 + ty + RY;
+  const int gi = i0 + lane, gj = j0 + r0;  // the thread's column and first row
   const bool edge = (g.per_x && (i0 <= 1 || i0 + w >= nx - 1)) || (g.per_y && (j0 <= 1 || j0 + h >= ny - 1));
   const float idx = g.inv_dx, idy = g.inv_dy;
   const bool blend = a.q0[0] != nullptr;
-  // halo ring (threads 0-95, whole warps): west, east columns, south, north rows;
-  // (hr, hc) are mixing-ratio plane coordinates (row 0 = j0-1, column 0 = i0-1)
-  int hr = -1, hc = 0;
-  if (tid < TY) { if (tid < h) { hr = tid + 1; hc = 0; } }
-  else if (tid < 2 * TY) { if (tid - TY < h) { hr = tid - TY + 1; hc = w + 1; } }
-  else if (tid < 2 * TY + TX) { if (tid - 2 * TY < w) { hr = 0; hc = tid - 2 * TY + 1; } }
-  else if (tid < 2 * TY + 2 * TX) { if (tid - 2 * TY - TX < w) { hr = h + 1; hc = tid - 2 * TY - TX + 1; } }
-
-  if (tid == 0) {
-    for (int s = 0; s < NSLOT; ++s) mbar_init(&s_bar[s], 1);
-    mbar_fence_init();
-    s_abort[0] = 0;
-    s_abort[1] = 0;
-  }
-  __syncthreads();
-
-  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads
-  // of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
-  int stall = -1;
-  if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
-  // the CTA's planes are kb .. ke-1; it also loads plane ke and (above the ground) the plane
-  // below, kb-1, whose mixing ratios its lowest faces read
-  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0;
-  if (stall >= 0) stall = kg + stall % (ke - kg + 1);  // a plane that this CTA loads
-  auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
-  auto issue = [&](int kk) {  // plane kk in [kg, ke]; plane nz holds the top faces only
-    float* st = slot_at(kk);
-    uint64_t* bar = &s_bar[(kk - kg) % NSLOT];
-    const bool cells = kk < nz;
-    unsigned bytes = B_OWN;
-    if (cells) bytes += (1 + a.ntracers) * B_CELL + 2 * B_FACE;
-    fence_proxy_async_smem();
-    mbar_arrive_expect_tx(bar, bytes);
-    if (kk == stall) return;  // failure-path testing: this plane's loads stay unissued
-    tma_load_3d(st + O_W, &m.w, i0 + kXOff, j0 + 1, kk, bar);
-    if (cells) {
-      tma_load_3d(st + O_RHO, &m.rho, i0 + kXOff - 4, j0, kk, bar);
-      for (int t = 0; t < a.ntracers; ++t) tma_load_3d(st + O_Q + t * 736, &m.q[t], i0 + kXOff - 4, j0, kk, bar);
-      tma_load_3d(st + O_U, &m.u, i0 + kXOff, j0 + 1, kk, bar);
-      tma_load_3d(st + O_V, &m.v, i0 + kXOff, j0 + 1, kk, bar);
-    }
-  };
-  int issued = kg - 1, waited = kg - 1;
-  auto wait_plane = [&](int kk, int epoch) {
-    if (!mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1)) {
-      s_abort[epoch & 1] = 1;
-      atomicExch(a.err, 1);
-    } else {
-      waited = kk;  // a plane whose wait gave up stays in the drain below
-    }
-  };
-  // mixing ratios of plane kk (dry_transport.cu:91-94) at the owned cells and the ring
-  auto mix = [&](int kk) {
-    const float* st = slot_at(kk);
-    auto one = [&](int r, int c) {
-      const int b = r * CBW + c + 3;
-      const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
-#pragma unroll
-      for (int t = 0; t < NTR; ++t)
-        if (t < a.ntracers) s_q[t][kk & 1][r][c] = st[O_Q + t * 736 + b] / rr;
-    };
-    if (own0) one(ty + 1, tx + 1);
-    if (own1) one(ty + RY + 1, tx + 1);
-    if (hr >= 0) one(hr, hc);
-  };
-
-  if (tid == ISSUER)
-    for (int kk = kg; kk < kg + NSLOT && kk <= ke; ++kk) { issue(kk); issued = kk; }
-  float qb0[NTR] = {0.f, 0.f, 0.f}, qb1[NTR] = {0.f, 0.f, 0.f};  // own mixing ratios at k-1
-  wait_plane(kg, kb);
-  if (kb > 0) {  // those of the plane below the chunk
-    const float* st = slot_at(kg);
-    auto below = [&](int row, float* qb) {
-      const int b = (row + 1) * CBW + tx + 4;
-      const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
-#pragma unroll
-      for (int t = 0; t < NTR; ++t)
-        if (t < a.ntracers) qb[t] = st[O_Q + t * 736 + b] / rr;
-    };
-    below(ty, qb0);
-    below(ty + RY, qb1);
-    wait_plane(kb, kb);
-  }
-  mix(kb);
-  __syncthreads();
-  if (kb > 0 && tid == ISSUER && kb + 2 <= ke) { issue(kb + 2); issued = kb + 2; }  // into plane kg's slot
-
-  // blend partner of plane kk at the thread's owned cells (prefetched a plane ahead)
-  auto load_q0 = [&](int gj, bool own, int kk, float* q0v) {
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) q0v[t] = 0.f;
-    if (!own || !blend || kk >= nz) return;
-    const int o = gidx(g, gi, gj, kk);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t)
-      if (t < a.ntracers) q0v[t] = __ldg(a.q0[t] + o);
-  };
-  float q0a[NTR], q0b[NTR];
-  load_q0(gj0, own0, kb, q0a);
-  load_q0(gj1, own1, kb, q0b);
-
-  // one owned column of plane k
-  auto column = [&](auto tile_class, int k, int r, int gj, bool own_rt, float* qb, const float* q0v, float idz) {
-    constexpr bool IN = decltype(tile_class)::value;  // interior tile: plain stores
-    const bool own = IN || own_rt;
-    const float* st = slot_at(k);
-    const float* sn = slot_at(k + 1);
-    const int c = tx + 1;
-    const int pb = k & 1;
-    const float fw = st[O_U + (r - 1) * FBW + tx], fe = st[O_U + (r - 1) * FBW + tx + 1];
-    const float fs = st[O_V + (r - 1) * FBW + tx], fn = st[O_V + r * FBW + tx];
-    const float fb = st[O_W + (r - 1) * OBW + tx], ft = sn[O_W + (r - 1) * OBW + tx];
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) {
-      if (t >= a.ntracers) break;
-      const float qc = s_q[t][pb][r][c];
-      const float qw = s_q[t][pb][r][c - 1], qe = s_q[t][pb][r][c + 1];
-      const float qs = s_q[t][pb][r - 1][c], qn = s_q[t][pb][r + 1][c];
-      const float qbt = (k > 0) ? qb[t] : qc;
-      const float qt = (k + 1 < nz) ? s_q[t][pb ^ 1][r][c] : qc;
-      const float gw = fp::upwind(fw, qw, qc), ge = fp::upwind(fe, qc, qe);
-      const float gs = fp::upwind(fs, qs, qc), gn = fp::upwind(fn, qc, qn);
-      const float gb = fp::upwind(fb, qbt, qc), gt = fp::upwind(ft, qc, qt);
-      const float div = fp::divergence(ge, gw, gn, gs, gt, gb, idx, idy, idz);
-      float out = fp::update(st[O_Q + t * 736 + r * CBW + c + 3], -a.dt, div, 0.0f);
-      if (blend) out = fp::blend(a.wa, q0v[t], a.wb, out);
-      if (own) {
-        if (IN) a.q_out[t][gidx(g, gi, gj, k)] = out;
-        else store_tile(a.q_out[t], g, kCell, gi, gj, k, out, edge);
-      }
-      qb[t] = qc;
-    }
-  };
-
-  // Interior tiles (full, away from every periodic edge ring) run a copy of the plane
-  // loop with plain stores instead of the periodic mirror stores; the arithmetic is the same.
+  // Interior tiles (full, away from every periodic edge ring) run a copy of the plane loop
+  // with plain stores instead of the periodic mirror stores; the arithmetic is the same.
   const bool interior = !edge && i0 + TX <= nx && j0 + TY <= ny;
-  auto plane_loop = [&](auto tile_class) -> bool {  // true when a bounded wait gave up
-    [[maybe_unused]] constexpr bool IN = decltype(tile_class)::value;
-    for (int k = kb; k < ke; ++k) {
-      // mixing ratios of plane k+1 (the own ones are this thread's, the ring published
-      // by the barrier below for the next plane)
-      // inverse layer depth (per level on flat terrain, per cell on terrain), loaded ahead
-      // of the mixing-ratio work
-      float idz0, idz1;
-      if constexpr (TERRAIN) {
-        idz0 = (IN || own0) ? __ldg(a.idz_c + gidx(g, gi, gj0, k)) : 0.f;
-        idz1 = (IN || own1) ? __ldg(a.idz_c + gidx(g, gi, gj1, k)) : 0.f;
-      } else {
-        idz0 = idz1 = __ldg(a.idz_c + k);
-      }
-      float n0a[NTR], n0b[NTR];
-      load_q0(gj0, own0, k + 1, n0a);
-      load_q0(gj1, own1, k + 1, n0b);
-      wait_plane(k + 1, k);
-      if (k + 1 < nz) mix(k + 1);
-      column(tile_class, k, ty + 1, gj0, own0, qb0, q0a, idz0);
-      column(tile_class, k, ty + RY + 1, gj1, own1, qb1, q0b, idz1);
-  #pragma unroll
-      for (int t = 0; t < NTR; ++t) { q0a[t] = n0a[t]; q0b[t] = n0b[t]; }
-      __syncthreads();  // publishes plane k+1's ring; slot k is free
-      if (s_abort[k & 1]) return true;
-      if (tid == ISSUER && k + 3 <= ke) { issue(k + 3); issued = k + 3; }
-    }
-    return false;
+  auto wait_full = [&](int kk) -> bool {
+    const int q = kk - kg;
+    const bool ok = mbar_wait(&s_full[q % NSLOT], (q / NSLOT) & 1);
+    return __all_sync(0xffffffffu, ok);
   };
-  const bool aborted = interior ? plane_loop(std::true_type{}) : plane_loop(std::false_type{});
-  if (aborted && tid == ISSUER)
-    for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1);
+  auto release = [&](int kk) {  // the warp is done with plane kk's slot
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&s_empty[(kk - kg) % NSLOT]);
+  };
+  auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
+  // mixing ratios (dry_transport.cu:91-94) at position b of a plane's cell boxes
+  auto mix = [&](const float* st, int b, float* q) {
+    const float rr = fmaxf(st[O_RHO + b], 1.0e-6f), y = fp::recip(rr);
+    float sum = 0.0f;
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      q[t] = fp::div_by(st[O_Q + t * Q_STRIDE + b], rr, y);
+      sum += fabsf(q[t]);
+    }
+    if (!fp::finite(sum)) {
+#pragma unroll
+      for (int t = 0; t < N; ++t) q[t] = fp::div(st[O_Q + t * Q_STRIDE + b], rr);
+    }
+  };
+
+  auto run = [&](auto tile_class) -> bool {  // false when a bounded wait gave up
+    constexpr bool IN = decltype(tile_class)::value;  // interior tile: plain stores
+    int off[ROWS];  // the owned cells of the current plane
+    bool own[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      off[r] = gidx(g, gi, gj + r, kb);
+      own[r] = IN || (lane < w && r0 + r < h);
+    }
+    const int b0 = (r0 + 1) * CBW + lane + 4;  // box position of the thread's first row
+    const int ring_row = lane & 3, ring_col = (lane & 4) ? TX : -1;
+    const int ring_b = (r0 + ring_row + 1) * CBW + ring_col + 4;
+    float qc[ROWS][N], fz[ROWS][N];  // mixing ratios of plane k, fluxes through its bottom faces
+    if (!wait_full(kg)) return false;
+    {
+      const float* st = slot_at(kg);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) mix(st, b0 + r * CBW, qc[r]);
+    }
+    if (kb > 0) {
+      if (!wait_full(kb)) return false;
+      const float* st = slot_at(kb);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        float qn[N];
+        mix(st, b0 + r * CBW, qn);
+        const float f = st[O_W + (r0 + r) * OBW + lane];
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          fz[r][t] = fp::upwind(f, qc[r][t], qn[t]);
+          qc[r][t] = qn[t];
+        }
+      }
+      release(kg);
+    } else {
+      const float* st = slot_at(0);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int t = 0; t < N; ++t) fz[r][t] = fp::upwind(st[O_W + (r0 + r) * OBW + lane], qc[r][t], qc[r][t]);
+    }
+    for (int k = kb; k < ke; ++k) {
+      const float* st = slot_at(k);
+      const int pb = k & 1;
+      // blend partner and inverse depths of the plane: used at the end
+      float q0[ROWS][N], idz[ROWS];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        idz[r] = TERRAIN ? (own[r] ? __ldg(a.idz_c + off[r]) : 0.f) : __ldg(a.idz_c + k);
+#pragma unroll
+        for (int t = 0; t < N; ++t) q0[r][t] = blend && own[r] ? __ldg(a.q0[t] + off[r]) : 0.f;
+      }
+      // the warp's ring columns, and its rows for the neighbouring lanes
+      if (lane < 2 * ROWS) {
+        float q[N];
+        mix(st, ring_b, q);
+#pragma unroll
+        for (int t = 0; t < N; ++t) s_q[pb][wid][t][ring_row][ring_col + 1] = q[t];
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+        for (int t = 0; t < N; ++t) s_q[pb][wid][t][r][lane + 1] = qc[r][t];
+      float qs[N], qn[N];  // the rows around the warp's
+      mix(st, b0 - CBW, qs);
+      mix(st, b0 + ROWS * CBW, qn);
+      if (!wait_full(k + 1)) return false;
+      const float* sn = slot_at(k + 1);
+      __syncwarp();
+      const float* su = st + O_U + r0 * FBW + lane;
+      const float* sv = st + O_V + r0 * FBW + lane;
+      float gy[N];  // Y fluxes below the row
+#pragma unroll
+      for (int t = 0; t < N; ++t) gy[t] = fp::upwind(sv[0], qs[t], qc[0][t]);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const float fw = su[r * FBW], fe = su[r * FBW + 1], fn = sv[(r + 1) * FBW];
+        const float ft = sn[O_W + (r0 + r) * OBW + lane];
+        float qt[N];
+        if (k + 1 < nz) {
+          mix(sn, b0 + r * CBW, qt);
+        } else {
+#pragma unroll
+          for (int t = 0; t < N; ++t) qt[t] = qc[r][t];
+        }
+#pragma unroll
+        for (int t = 0; t < N; ++t) {
+          const float c = qc[r][t];
+          const float gw = fp::upwind(fw, s_q[pb][wid][t][r][lane], c);
+          const float ge = fp::upwind(fe, c, s_q[pb][wid][t][r][lane + 2]);
+          const float gn = fp::upwind(fn, c, r + 1 < ROWS ? qc[r + 1 < ROWS ? r + 1 : r][t] : qn[t]);
+          const float gt = fp::upwind(ft, c, qt[t]);
+          const float div = fp::divergence(ge, gw, gn, gy[t], gt, fz[r][t], idx, idy, idz[r]);
+          float out = fp::update(st[O_Q + t * Q_STRIDE + b0 + r * CBW], -a.dt, div, 0.0f);
+          if (blend) out = fp::blend(a.wa, q0[r][t], a.wb, out);
+          if (IN) a.q_out[t][off[r]] = out;
+          else if (own[r]) store_tile(a.q_out[t], g, kCell, gi, gj + r, k, out, edge);
+          gy[t] = gn;
+          fz[r][t] = gt;
+        }
+#pragma unroll
+        for (int t = 0; t < N; ++t) qc[r][t] = qt[t];
+        off[r] += g.plane;
+      }
+      release(k);
+    }
+    return true;
+  };
+  const bool ok = interior ? run(std::true_type{}) : run(std::false_type{});
+  if (!ok && lane == 0) atomicExch(a.err, 1);
+}
+
+template <bool TERRAIN, int N>
+cudaError_t allow_smem() {
+  return cudaFuncSetAttribute(k_tracer_tma<TERRAIN, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)tt::smem_bytes(N));
+}
+
+template <bool TERRAIN>
+void launch(const TracerArgs& a, const TracerMaps& m, dim3 grid, const ZSplit& zs, cudaStream_t s) {
+  const size_t smem = tt::smem_bytes(a.ntracers);
+  if (a.ntracers == 1) k_tracer_tma<TERRAIN, 1><<<grid, tt::NT, smem, s>>>(a, m, zs);
+  else if (a.ntracers == 2) k_tracer_tma<TERRAIN, 2><<<grid, tt::NT, smem, s>>>(a, m, zs);
+  else k_tracer_tma<TERRAIN, 3><<<grid, tt::NT, smem, s>>>(a, m, zs);
 }
 
 }  // namespace
 
 cudaError_t init_tracer_tma() {
-  const cudaError_t e =
-      cudaFuncSetAttribute(k_tracer_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tt::kDynSmem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_tracer_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tt::kDynSmem);
+  cudaError_t e = allow_smem<false, 1>();
+  if (e == cudaSuccess) e = allow_smem<false, 2>();
+  if (e == cudaSuccess) e = allow_smem<false, 3>();
+  if (e == cudaSuccess) e = allow_smem<true, 1>();
+  if (e == cudaSuccess) e = allow_smem<true, 2>();
+  if (e == cudaSuccess) e = allow_smem<true, 3>();
+  return e;
 }
 
 cudaError_t launch_tracer_tma(const TracerArgs& a, const TracerMaps& m, cudaStream_t s) {
   if (a.g.nz < 1 || !a.err || a.ntracers < 1 || a.ntracers > tt::NTR) return cudaErrorInvalidValue;
-  const dim3 block(tt::TX, tt::RY);
   dim3 grid((a.g.nx + tt::TX - 1) / tt::TX, (a.g.ny + tt::TY - 1) / tt::TY);
-  const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 3, 1.2f);
+  const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, tt::MIN_CTAS, 1.0f);
   grid.z = zs.chunks;
-  if (a.terrain) k_tracer_tma<true><<<grid, block, tt::kDynSmem, s>>>(a, m, zs);
-  else k_tracer_tma<false><<<grid, block, tt::kDynSmem, s>>>(a, m, zs);
+  if (a.terrain) launch<true>(a, m, grid, zs, s);
+  else launch<false>(a, m, grid, zs, s);
   return cudaGetLastError();
 }
 
