@@ -84,21 +84,25 @@ static __noinline__ __device__ float eos_pprime_full(float rho, float rt, double
   return (float)((double)eos_pressure(rho, rt) - pref);
 }
 // Core form with the level's 1/rt_ref and p_ref already at hand.
-__device__ __forceinline__ float eos_pprime_ref(float rho, float rt, double inv_rt_ref, double pref) {
+// eos_pprime_near clears `near` where the series does not hold and the full form is due.
+__device__ __forceinline__ float eos_pprime_near(float rho, float rt, double inv_rt_ref, double pref, bool& near) {
   const double d = fma((double)rt, inv_rt_ref, -1.0);
-  if (rho >= 1.0e-6f && fabs(d) < 0.0625) {
-    // C(g, n), n = 1 .. 7, for g = 1.0f / (1.0f - 0.2854f); Estrin's scheme keeps the
-    // dependent FP64 chain three operations deep instead of seven (Horner)
-    const double d2 = d * d, d4 = d2 * d2;
-    const double a = fma(0.2794461309425813, d, 1.3993843793869019);
-    const double b = fma(0.022387238647368683, d, -0.055946570454669185);
-    const double c = fma(0.0069876670302162856, d, -0.011644120505748048);
-    const double lo = fma(b, d2, a);
-    const double hi = fma(-0.0045925100129794545, d2, c);
-    const double s = fma(hi, d4, lo);
-    return (float)(pref * (s * d));
-  }
-  return eos_pprime_full(rho, rt, pref);
+  near = near && rho >= 1.0e-6f && fabs(d) < 0.0625;
+  // C(g, n), n = 1 .. 7, for g = 1.0f / (1.0f - 0.2854f); Estrin's scheme keeps the
+  // dependent FP64 chain three operations deep instead of seven (Horner)
+  const double d2 = d * d, d4 = d2 * d2;
+  const double a = fma(0.2794461309425813, d, 1.3993843793869019);
+  const double b = fma(0.022387238647368683, d, -0.055946570454669185);
+  const double c = fma(0.0069876670302162856, d, -0.011644120505748048);
+  const double lo = fma(b, d2, a);
+  const double hi = fma(-0.0045925100129794545, d2, c);
+  const double s = fma(hi, d4, lo);
+  return (float)(pref * (s * d));
+}
+__device__ __forceinline__ float eos_pprime_ref(float rho, float rt, double inv_rt_ref, double pref) {
+  bool near = true;
+  const float p = eos_pprime_near(rho, rt, inv_rt_ref, pref, near);
+  return near ? p : eos_pprime_full(rho, rt, pref);
 }
 __device__ __forceinline__ float eos_pprime(float rho, float rt, const double* __restrict__ base, int k,
                                             int nz) {

@@ -189,23 +189,42 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   constexpr int NP = (DN + NT - 1) / NT;
   int pos_b[NP];
   float yrho[NP];
+  // positions whose theta (bit n) and whose p' and velocities (bit 8 + n) are read: not those of
+  // a partial tile's missing rows and columns, and beyond an open side (where rho is zero and
+  // the EOS would take its full form) only theta
+  unsigned live = 0;
 #pragma unroll
   for (int n = 0; n < NP; ++n) {
-    const int q = tid + n * NT, r = q / DW;
-    pos_b[n] = r * BW + (q - r * DW) + 3;
+    const int q = tid + n * NT, r = q / DW, c = q - r * DW;
+    pos_b[n] = r * BW + c + 3;
+    if (q < DN && r <= h + 1 && c <= w + 1) {
+      const int pi = i0 + c - 1, pj = j0 + r - 1;
+      live |= 1u << n;
+      if ((g.per_x || (pi >= 0 && pi < nx)) && (g.per_y || (pj >= 0 && pj < ny))) live |= 256u << n;
+    }
   }
   // theta of plane kk (kk < nz), and the reciprocals that derive(kk) divides by
   auto derive_theta = [&](int kk) {
     const float* sr = slot_at(kk);
     float* th = der + D_TH + (kk % 3) * DN;
+    bool near = true;
 #pragma unroll
     for (int n = 0; n < NP; ++n)
-      if ((n + 1) * NT <= DN || tid + n * NT < DN) {
+      if (live & (1u << n)) {
         const float rho = sr[R_RHO + pos_b[n]], rt = RT(sr, pos_b[n], rho), rr = fmaxf(rho, 1.0e-6f);
         yrho[n] = fp::recip(rr);
         const float t = fp::div_by(rt, rr, yrho[n]);
-        th[tid + n * NT] = fp::finite(t) ? t : fp::div(rt, rr);
+        near = near && fp::finite(t);
+        th[tid + n * NT] = t;
       }
+    if (!near) {  // a quotient that is not finite: plain divisions
+#pragma unroll
+      for (int n = 0; n < NP; ++n)
+        if (live & (1u << n)) {
+          const float rho = sr[R_RHO + pos_b[n]];
+          th[tid + n * NT] = fp::theta(rho, RT(sr, pos_b[n], rho));
+        }
+    }
   };
   // p', uc, vc, wc of plane k (after derive_theta(k))
   auto derive = [&](int k) {
@@ -215,26 +234,43 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     float* vc = der + D_VC + (k % 3) * DN;
     float* wc = der + D_WC + (k & 1) * DN;
     float* pp = der + D_P + (k & 1) * DN;
+    const double binv = s_binv[k], bpr = s_bpr[k];
+    bool near = true;
+    auto momenta = [&](int b, float& mu, float& mv, float& mw) {
+      mu = fp::avg(U(sr, b), U(sr, b + 1));
+      mv = fp::avg(V(sr, b), V(sr, b + BW));
+      mw = fp::avg(W(sr, b), W(sn, b));
+    };
 #pragma unroll
     for (int n = 0; n < NP; ++n)
-      if ((n + 1) * NT <= DN || tid + n * NT < DN) {
+      if (live & (256u << n)) {
         const int b = pos_b[n], q = tid + n * NT;
         const float rho = sr[R_RHO + b];
-        pp[q] = eos_pprime_ref(rho, RT(sr, b, rho), s_binv[k], s_bpr[k]);
+        pp[q] = eos_pprime_near(rho, RT(sr, b, rho), binv, bpr, near);
         // cell-centred velocities: dry_momentum_flux.cu:36-73
         const float rr = fmaxf(rho, 1.0e-6f), y = yrho[n];
-        const float mu = fp::avg(U(sr, b), U(sr, b + 1)), mv = fp::avg(V(sr, b), V(sr, b + BW)),
-                    mw = fp::avg(W(sr, b), W(sn, b));
-        float cu = fp::div_by(mu, rr, y), cv = fp::div_by(mv, rr, y), cw = fp::div_by(mw, rr, y);
-        if (!fp::finite(fabsf(cu) + fabsf(cv) + fabsf(cw))) {
-          cu = fp::div(mu, rr);
-          cv = fp::div(mv, rr);
-          cw = fp::div(mw, rr);
-        }
+        float mu, mv, mw;
+        momenta(b, mu, mv, mw);
+        const float cu = fp::div_by(mu, rr, y), cv = fp::div_by(mv, rr, y), cw = fp::div_by(mw, rr, y);
+        near = near && fp::finite(fabsf(cu) + fabsf(cv) + fabsf(cw));
         uc[q] = cu;
         vc[q] = cv;
         wc[q] = cw;
       }
+    if (!near) {  // far from the base state, or a quotient that is not finite: the plain forms
+#pragma unroll 1
+      for (int n = 0; n < NP; ++n) {
+        if (!(live & (256u << n))) continue;
+        const int q = tid + n * NT, r = q / DW, b = r * BW + (q - r * DW) + 3;
+        const float rho = sr[R_RHO + b], rr = fmaxf(rho, 1.0e-6f);
+        pp[q] = eos_pprime_ref(rho, RT(sr, b, rho), binv, bpr);
+        float mu, mv, mw;
+        momenta(b, mu, mv, mw);
+        uc[q] = fp::div(mu, rr);
+        vc[q] = fp::div(mv, rr);
+        wc[q] = fp::div(mw, rr);
+      }
+    }
   };
 
   // Values of the thread's columns carried up: the stage input at plane k, theta and rho of
@@ -361,7 +397,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     }
     // ---- cells: K2 compute_cell_tendencies_kernel (dry_core.cu:62-144)
     {
-      float gy[ROWS + 1];
+      float gy[ROWS + 1], ro[ROWS], to[ROWS];
 #pragma unroll
       for (int r = 0; r <= ROWS; ++r) gy[r] = fp::upwind(r < ROWS ? v_c[r] : v_t, tc[r], tc[r + 1]);
 #pragma unroll
@@ -384,17 +420,31 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         const float th1 = fp::theta(r1, q1);
         put(a.o_rho, kCell, r, 0, r1);
         put(a.o_th, kCell, r, 0, a.out_rt ? q1 : th1);
-        if (IN || own_rt[r]) {
-          if (a.acc_mode == 1) {
-            // p' of the output: the level sums, and (stored) the first substep's input
-            const float pv = eos_pprime_ref(r1, fp::mul(r1, th1), s_binv[k], s_bpr[k]);
-            ra += fx(r1, kFxRho);
-            rb += fx(pv, kFxP);
-            if (a.p_out) put(a.p_out, kCell, r, 0, pv);
-          } else if (a.acc_mode == 2) {
-            ra += fx(th1, kFxTheta);
-          }
+        ro[r] = r1;
+        to[r] = th1;
+      }
+      if (a.acc_mode == 1) {
+        // p' of the output: the level sums, and (stored) the first substep's input
+        const double binv = s_binv[k], bpr = s_bpr[k];
+        float pv[ROWS];
+        bool near = true;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) pv[r] = eos_pprime_near(ro[r], fp::mul(ro[r], to[r]), binv, bpr, near);
+        if (!near) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) pv[r] = eos_pprime_ref(ro[r], fp::mul(ro[r], to[r]), binv, bpr);
         }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+          if (IN || own_rt[r]) {
+            ra += fx(ro[r], kFxRho);
+            rb += fx(pv[r], kFxP);
+            if (a.p_out) put(a.p_out, kCell, r, 0, pv[r]);
+          }
+      } else if (a.acc_mode == 2) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+          if (IN || own_rt[r]) ra += fx(to[r], kFxTheta);
       }
     }
     // ---- X faces: K17 (dry_momentum_flux.cu:79-156) + K21 (dry_pressure_gradient.cu:75-123)
@@ -469,7 +519,10 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
           if (sx0) flw = 0.0f;
           if (sx1) fle = 0.0f;
           t_w = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_w[r], idx, idy, kc.idzf);
-          t_w = fp::add_buoyancy_ref(t_w, th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r], a.gravity);
+          bool near = true;
+          const float t = fp::add_buoyancy_ref(t_w, th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r],
+                                               a.gravity, near);
+          t_w = near ? t : fp::add_buoyancy(t_w, th_l[r], tc[r + 1], s_trf[k], rho_l[r], rho_c[r], a.gravity);
           if (a.damp_c) t_w = fp::add_damping(t_w, kc.damp_f, qc, 0.0f);
         }
         fz_w[r] = flt;

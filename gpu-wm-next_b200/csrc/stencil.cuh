@@ -132,24 +132,27 @@ __device__ __forceinline__ V add_pgf_terrain(V t, V pr, V pl, V zr, V zl, V dpdz
 template <class V> __device__ __forceinline__ V add_damping(V t, float rate, V q, float qref) {
   return fma(sc<V>(-rate), sub(q, sc<V>(qref)), t);
 }
-// K3 buoyancy at a Z face: t + rho_f g (theta_f - theta_ref_f) / max(theta_ref_f, 1e-6)
-// with face means of the two cells and of the two level means.
+// K3 buoyancy at a Z face: t + rho_f g (theta_f - trf) / max(trf, 1e-6) with face means of the
+// two cells and trf the face mean of the two level means theta_ref.
+template <class V>
+__device__ __forceinline__ V add_buoyancy(V t, V th_l, V th_u, float trf, V rho_l, V rho_u, float gravity) {
+  const V b = div(mul(sc<V>(gravity), sub(avg(th_l, th_u), sc<V>(trf))), sc<V>(fmaxf(trf, 1.0e-6f)));
+  return fma(avg(rho_l, rho_u), b, t);
+}
+// With the level means themselves.
 template <class V>
 __device__ __forceinline__ V add_buoyancy(V t, V th_l, V th_u, float tref_l, float tref_u, V rho_l, V rho_u,
                                           float gravity) {
-  const float trf = __fmul_rn(0.5f, __fadd_rn(tref_l, tref_u));
-  const V tf = avg(th_l, th_u);
-  const V b = div(mul(sc<V>(gravity), sub(tf, sc<V>(trf))), sc<V>(fmaxf(trf, 1.0e-6f)));
-  return fma(avg(rho_l, rho_u), b, t);
+  return add_buoyancy(t, th_l, th_u, __fmul_rn(0.5f, __fadd_rn(tref_l, tref_u)), rho_l, rho_u, gravity);
 }
 
 // The same with the face mean of the level means, trf, and the reciprocal of its floored
-// value at hand (one pair per level).
+// value at hand (one pair per level); `near` is cleared where the plain form is due.
 __device__ __forceinline__ float add_buoyancy_ref(float t, float th_l, float th_u, float trf, float ytrf, float rho_l,
-                                                  float rho_u, float gravity) {
+                                                  float rho_u, float gravity, bool& near) {
   const float n = mul(gravity, sub(avg(th_l, th_u), trf)), d = fmaxf(trf, 1.0e-6f);
-  float b = div_by(n, d, ytrf);
-  if (!finite(b)) b = div(n, d);
+  const float b = div_by(n, d, ytrf);
+  near = near && finite(b);
   return fma(avg(rho_l, rho_u), b, t);
 }
 
