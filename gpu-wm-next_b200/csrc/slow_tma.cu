@@ -165,11 +165,11 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     off[r] = gidx(g, gi, gj + r, kb);
     own_rt[r] = tx < w && r0 + r < h;
   }
-  // blend partner at plane k (off) or k + 1 (up = 1) of the thread's row r
-  auto load_q0 = [&](int r, int kk, int up) {
+  // blend partner at the current plane of the thread's row r
+  auto load_q0 = [&](int r) {
     SlowBlend q{0.f, 0.f, 0.f, 0.f, 0.f};
-    if (!BLEND || !own_rt[r] || kk >= nz) return q;
-    const int o = off[r] + up * g.plane;
+    if (!BLEND || !own_rt[r]) return q;
+    const int o = off[r];
     q.rho = __ldg(a.rho0 + o);
     q.rt = __ldg(a.rt0 + o);
     q.u = __ldg(a.u0 + o);
@@ -180,10 +180,6 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
 
   if (tid == ISSUER)
     for (int kk = kg; kk <= kb + 1; ++kk) { issue(kk); issued = kk; }
-  SlowBlend q0[ROWS];
-#pragma unroll
-  for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(r, kb, 0);
-
   // ---- derived planes: the thread's positions of the 34 x 18 (a third one in the first
   // warps), their box indices and the reciprocal of their floored density
   constexpr int NP = (DN + NT - 1) / NT;
@@ -339,7 +335,8 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   };
 
   // cells, X faces, Y faces and Z faces of plane k in the thread's rows (+ the top faces)
-  auto columns = [&](auto tile_class, int k, long long& ra, long long& rb, const PlaneConst& kc) {
+  auto columns = [&](auto tile_class, int k, const SlowBlend* q0, long long& ra, long long& rb,
+                     const PlaneConst& kc) {
     constexpr bool IN = decltype(tile_class)::value;  // an interior tile
     // store of an owned value at plane k + up: a plain store in interior tiles, else with the
     // periodic mirrors
@@ -557,12 +554,12 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     for (int k = kb; k < ke; ++k) {
       const int pb = k & 1;
       const PlaneConst kc = plane_const(k);
+      SlowBlend q0[ROWS];  // the derive phase covers the loads
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(r);
       wait_plane(k + 1, k);
       derive(k);
       if (k + 1 < nz) derive_theta(k + 1);
-      SlowBlend n0[ROWS];
-#pragma unroll
-      for (int r = 0; r < ROWS; ++r) n0[r] = load_q0(r, k + 1, 1);
       __syncthreads();  // publishes plane k's derived values; slot (k-1) is free
       if (s_abort[pb]) return true;
       if (tid == ISSUER) {
@@ -576,7 +573,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
       }
       // ---- cells and faces of plane k
       long long ra = 0, rb = 0;
-      columns(tile_class, k, ra, rb, kc);
+      columns(tile_class, k, q0, ra, rb, kc);
       if (!IN && xf) {  // open east boundary: X face nx of row j0+tx
         const float* sr = slot_at(k);
         const float uf = U(sr, (tx + 1) * BW + w + 4);
@@ -596,10 +593,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         if (tx == 0) { s_red[pb][ty][0] = ta; s_red[pb][ty][1] = tb; }
       }
 #pragma unroll
-      for (int r = 0; r < ROWS; ++r) {
-        q0[r] = n0[r];
-        off[r] += g.plane;
-      }
+      for (int r = 0; r < ROWS; ++r) off[r] += g.plane;
     }
     return false;
   };
