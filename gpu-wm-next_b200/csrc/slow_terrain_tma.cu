@@ -27,7 +27,7 @@ namespace gwmb {
 namespace {
 
 namespace st {
-constexpr int TX = 32, TY = 16, RY = 8, NT = 256, NW = NT / 32;
+constexpr int TX = 32, TY = 16, ROWS = 2, NT = 256, NW = NT / 32;  // two adjacent rows per thread
 // the thread that issues the TMA loads and folds the level sums: lane 0 of the last warp
 constexpr int ISSUER = NT - 32;
 constexpr int BW = 40, BH = 18, BHV = 19;  // boxes: cells, X and Z faces / Y faces
@@ -36,8 +36,9 @@ constexpr int DW = TX + 2, DH = TY + 2, DN = DW * DH;  // derived plane: 34 x 18
 constexpr int R_RHO = 0, R_TH = 736, R_U = 1472, R_W = 2208, R_V = 2944, R_Z = 3712, R_DU = 4448, R_DW = 5184,
               R_DV = 5920, SLOT = 6688, SLOT_SHORT = 4448, NSLOT = 3;
 constexpr unsigned B_BOX = BW * BH * 4, B_BOXV = BW * BHV * 4;
-// derived arrays (floats): uc, vc, wc [2][DN] (planes k-1, k); theta, dp/dz [DN]; p [3][DN]
-constexpr int D_UC = 0, D_VC = 2 * DN, D_WC = 4 * DN, D_TH = 6 * DN, D_DZ = 7 * DN, D_P = 8 * DN, DERIVED = 11 * DN;
+// derived arrays (floats): uc, vc [2][DN] (planes k-1, k); theta [2][DN] (planes k, k+1); wc, dp/dz,
+// p [DN]
+constexpr int D_UC = 0, D_VC = 2 * DN, D_TH = 4 * DN, D_WC = 6 * DN, D_DZ = 7 * DN, D_P = 8 * DN, DERIVED = 9 * DN;
 static_assert(R_TH % 32 == 0 && R_U % 32 == 0 && R_W % 32 == 0 && R_V % 32 == 0 && R_Z % 32 == 0 &&
                   R_DU % 32 == 0 && R_DW % 32 == 0 && R_DV % 32 == 0 && SLOT % 32 == 0 && SLOT_SHORT == R_DU,
               "128-byte aligned sub-buffers");
@@ -50,26 +51,26 @@ constexpr size_t smem_bytes(bool inc) {
 }
 }  // namespace st
 
-// Values of one owned column carried from plane k-1 to plane k.
-struct TerrCarry {
-  float rho, th, uf, vf, wf;
-};
-// Blend partner q0 at a column's owned positions of one plane.
-struct TerrBlend {
+// Blend partner q0 at an owned position of one plane.
+struct SlowBlend {
   float rho, rt, u, v, w;
 };
+
 // Metric values of one owned column at one plane: inverse layer depth of the cell, of its
 // west and south neighbours (the X and Y faces average two cells) and of the Z face.
 struct TerrMetric {
   float c, w, s, f;
 };
 
-template <bool INC>
+// FIRST: a step's first stage (rho*theta in, no blend); INC: acoustic increments are added to
+// the momenta (stages 2 and 3 behind the fast modes).
+template <bool FIRST, bool INC>
 __global__ void __launch_bounds__(st::NT, 2)
     k_slow_terrain_tma(const SlowArgs a, const __grid_constant__ SlowMaps m, ZSplit zs) {
   using namespace st;
+  constexpr bool BLEND = !FIRST;
   extern __shared__ unsigned char s_dyn[];
-  __shared__ float s_thref[kMaxNz];
+  __shared__ float s_trf[kMaxNz], s_ytrf[kMaxNz];   // theta_ref at Z face k, reciprocal of its floored value
   __shared__ long long s_red[2][NW];
   __shared__ __align__(8) uint64_t s_bar[NSLOT];
   __shared__ int s_abort[2];
@@ -82,16 +83,18 @@ __global__ void __launch_bounds__(st::NT, 2)
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int w = min(TX, nx - i0), h = min(TY, ny - j0);
-  const bool own0 = tx < w && ty < h, own1 = tx < w && ty + RY < h;
-  const int gi = i0 + tx, gj0 = j0 + ty, gj1 = j0 + ty + RY;
+  const int r0 = ty * ROWS, gi = i0 + tx, gj = j0 + r0;  // the thread's column and first row
   const bool open_x = !g.per_x, open_y = !g.per_y;
   const bool edge = (g.per_x && (i0 <= 1 || i0 + w >= nx - 1)) || (g.per_y && (j0 <= 1 || j0 + h >= ny - 1));
   const float idx = g.inv_dx, idy = g.inv_dy, dt = a.dt;
-  const bool blend = a.rho0 != nullptr;
   // open boundaries: X face nx and Y face ny belong to the last tiles; their tendency
-  // is zero (dry_momentum_flux.cu:79-235 skips them), so they are blends of the stage value
+  // is zero (dry_momentum_flux.cu:79-235 skips them), so they are blends of the stage
+  // value.  Under periodic wrap they are the mirrors of faces 0 written by store_tile.
   const bool xf = open_x && i0 + w == nx && ty == 0 && tx < h;  // X face nx, row j0+tx
   const bool yf = open_y && j0 + h == ny && ty == 1 && tx < w;  // Y face ny, column i0+tx
+  // the CTA's planes are kb .. ke-1; it also loads plane ke and (above the ground) the plane
+  // below, kb-1, whose derived values its lowest faces read
+  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0;
 
   if (tid == 0) {
     for (int s = 0; s < NSLOT; ++s) mbar_init(&s_bar[s], 1);
@@ -101,17 +104,20 @@ __global__ void __launch_bounds__(st::NT, 2)
   }
   if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && a.clr_a)
     for (int q = tid; q < nz; q += NT) { a.clr_a[q] = 0ull; a.clr_b[q] = 0ull; }
-  for (int q = tid; q < nz; q += NT) s_thref[q] = (float)(acc_read(a.th_acc + q, kScaleTheta) * a.inv_count);
+  for (int q = kg + tid; q < ke; q += NT) {
+    const float tu = (float)(acc_read(a.th_acc + q, kScaleTheta) * a.inv_count);
+    const float tl = q > 0 ? (float)(acc_read(a.th_acc + q - 1, kScaleTheta) * a.inv_count) : tu;
+    const float trf = fp::avg(tl, tu);
+    s_trf[q] = trf;
+    s_ytrf[q] = fp::recip(fmaxf(trf, 1.0e-6f));
+  }
   __syncthreads();
 
-  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads
-  // of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
+  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads of
+  // one of its planes unissued, so that CTA's bounded wait runs out
   int stall = -1;
   if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
-  // the CTA's planes are kb .. ke-1; it also loads plane ke and (above the ground) the plane
-  // below, kb-1, whose derived values its lowest faces read
-  const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0;
-  if (stall >= 0) stall = kg + stall % (ke - kg + 1);  // a plane that this CTA loads
+  if (stall >= 0) stall = kg + stall % (ke - kg + 1);
   auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * slot; };
   auto issue = [&](int kk) {  // plane kk in [kg, ke] into its slot
     float* sr = slot_at(kk);
@@ -150,16 +156,23 @@ __global__ void __launch_bounds__(st::NT, 2)
   auto U = [&](const float* sr, int b) { return INC ? fp::add(sr[R_U + b], sr[R_DU + b]) : sr[R_U + b]; };
   auto V = [&](const float* sr, int b) { return INC ? fp::add(sr[R_V + b], sr[R_DV + b]) : sr[R_V + b]; };
   auto W = [&](const float* sr, int b) { return INC ? fp::add(sr[R_W + b], sr[R_DW + b]) : sr[R_W + b]; };
-  auto RT = [&](const float* sr, int b) {
+  auto RT = [&](const float* sr, int b, float rho) {
     const float t = sr[R_TH + b];
-    return a.th_is_rt ? t : fp::mul(sr[R_RHO + b], t);
+    return FIRST ? t : fp::mul(rho, t);
   };
 
-  // blend partner of plane kk at the thread's owned positions
-  auto load_q0 = [&](int gj, bool own, int kk) {
-    TerrBlend q{0.f, 0.f, 0.f, 0.f, 0.f};
-    if (!blend || !own || kk >= nz) return q;
-    const int o = gidx(g, gi, gj, kk);
+  int off[ROWS];  // the owned cells of the current plane
+  bool own_rt[ROWS];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    off[r] = gidx(g, gi, gj + r, kb);
+    own_rt[r] = tx < w && r0 + r < h;
+  }
+  // blend partner at the current plane of the thread's row r
+  auto load_q0 = [&](int r) {
+    SlowBlend q{0.f, 0.f, 0.f, 0.f, 0.f};
+    if (!BLEND || !own_rt[r]) return q;
+    const int o = off[r];
     q.rho = __ldg(a.rho0 + o);
     q.rt = __ldg(a.rt0 + o);
     q.u = __ldg(a.u0 + o);
@@ -167,223 +180,415 @@ __global__ void __launch_bounds__(st::NT, 2)
     q.w = __ldg(a.w0 + o);
     return q;
   };
-  // metric values of plane kk at the thread's owned positions
-  auto load_metric = [&](int gj, bool own, int kk) {
-    TerrMetric t{0.f, 0.f, 0.f, 0.f};
-    if (!own || kk >= nz) return t;
-    const int o = gidx(g, gi, gj, kk);
-    t.c = __ldg(a.idz_c + o);
-    t.w = __ldg(a.idz_c + o - 1);
-    t.s = __ldg(a.idz_c + o - g.pitch);
-    t.f = __ldg(a.idz_f + o);
-    return t;
-  };
 
   if (tid == ISSUER)
     for (int kk = kg; kk <= kb + 1; ++kk) { issue(kk); issued = kk; }
-  TerrBlend q0a = load_q0(gj0, own0, kb), q0b = load_q0(gj1, own1, kb);
-  TerrMetric m0a = load_metric(gj0, own0, kb), m0b = load_metric(gj1, own1, kb);
-  TerrCarry ca{0.f, 0.f, 0.f, 0.f, 0.f}, cb{0.f, 0.f, 0.f, 0.f, 0.f};
-  wait_plane(kg, kb);
-
-  // store of an owned value: a plain store in interior tiles, else with the periodic mirrors
-  auto put = [&](bool in, float* f, const Geom& gg, int o, int i, int j, int kk, float v) {
-    if (in) f[gidx(gg, i, j, kk)] = v;
-    else store_tile(f, gg, o, i, j, kk, v, edge);
+  // metric values at the current plane of the thread's rows
+  auto load_metric = [&](TerrMetric* t) {
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      t[r] = TerrMetric{0.f, 0.f, 0.f, 0.f};
+      if (!own_rt[r]) continue;
+      const int o = off[r];
+      t[r].c = __ldg(a.idz_c + o);
+      t[r].w = __ldg(a.idz_c + o - 1);
+      t[r].s = r > 0 ? t[r > 0 ? r - 1 : 0].c : __ldg(a.idz_c + o - g.pitch);
+      t[r].f = __ldg(a.idz_f + o);
+    }
   };
-  // one owned column: cell, X face, Y face and Z face of plane k (+ the top face)
-  auto column = [&](auto tile_class, int k, int r, int gj, bool own_rt, TerrCarry& cy, const TerrBlend& q0,
-                    const TerrMetric& mt, FxAcc& ra) {
-    constexpr bool IN = decltype(tile_class)::value;  // an interior tile
-    const bool own = IN || own_rt;
-    const float* sr = slot_at(k);
-    const float* sn = slot_at(k + 1);
-    const float* uc = der + D_UC + (k & 1) * DN;
-    const float* vc = der + D_VC + (k & 1) * DN;
-    const float* wc = der + D_WC + (k & 1) * DN;
-    const float* ucm = der + D_UC + ((k + 1) & 1) * DN;  // plane k-1
-    const float* vcm = der + D_VC + ((k + 1) & 1) * DN;
-    const float* wcm = der + D_WC + ((k + 1) & 1) * DN;
-    const float* th = der + D_TH;
-    const float* dz = der + D_DZ;
-    const float* pp = der + D_P + (k % 3) * DN;
-    const int c = tx + 1;
-    const int d = r * DW + c;   // derived index
-    const int b = r * BW + c + 3;  // raw box index
-    const bool top = k + 1 == nz;
-    // values of the column at planes k and k+1
-    const float rho = sr[R_RHO + b], rt = RT(sr, b);
-    const float tc = th[d], pc = pp[d];
-    const float uf = U(sr, b), vf = V(sr, b), wf = W(sr, b);
-    const float wft = W(sn, b);  // face k+1 (plane nz holds the top faces)
-    float uft = uf, vft = vf, tt = tc;
-    if (!top) {
-      uft = U(sn, b);
-      vft = V(sn, b);
-      tt = fp::theta(sn[R_RHO + b], RT(sn, b));
+
+  // ---- derived planes: the thread's positions of the 34 x 18 (a third one in the first
+  // warps), their box indices and the reciprocal of their floored density
+  constexpr int NP = (DN + NT - 1) / NT;
+  int pos_b[NP];
+  float yrho[NP], p_m[NP], p_c[NP];  // the reciprocal at plane k; the pressure at planes k-1 and k
+  // positions whose theta (bit n) and whose p, dp/dz and velocities (bit 8 + n) are read: not
+  // those of a partial tile's missing rows and columns, and beyond an open side only theta
+  unsigned live = 0;
+#pragma unroll
+  for (int n = 0; n < NP; ++n) {
+    const int q = tid + n * NT, r = q / DW, c = q - r * DW;
+    pos_b[n] = r * BW + c + 3;
+    if (q < DN && r <= h + 1 && c <= w + 1) {
+      const int pi = i0 + c - 1, pj = j0 + r - 1;
+      live |= 1u << n;
+      if ((g.per_x || (pi >= 0 && pi < nx)) && (g.per_y || (pj >= 0 && pj < ny))) live |= 256u << n;
     }
-    const float tb = k > 0 ? cy.th : tc;
-    // ---- cell: K2 compute_cell_tendencies_kernel (dry_core.cu:62-144)
-    {
-      const float fw = uf, fe = U(sr, b + 1), fs = vf, fn = V(sr, b + BW);
-      const float fb = wf, ft = wft;
-      const float t_rho = -fp::divergence(fe, fw, fn, fs, ft, fb, idx, idy, mt.c);
-      const float tw = th[d - 1], te = th[d + 1], ts = th[d - DW], tn = th[d + DW];
-      const float gw = fp::upwind(fw, tw, tc), ge = fp::upwind(fe, tc, te);
-      const float gs = fp::upwind(fs, ts, tc), gn = fp::upwind(fn, tc, tn);
-      const float gb = fp::upwind(fb, tb, tc), gt = fp::upwind(ft, tc, tt);
-      const float t_rt = -fp::divergence(ge, gw, gn, gs, gt, gb, idx, idy, mt.c);
-      float r1 = fp::update(rho, dt, t_rho, 1.0e-6f);
-      float q1 = fp::update(rt, dt, t_rt, 1.0e-6f);
-      if (blend) {
-        r1 = fp::blend(a.wa, q0.rho, a.wb, r1);
-        q1 = fp::blend(a.wa, q0.rt, a.wb, q1);
-      }
-      const float th1 = fp::theta(r1, q1);
-      if (own) {
-        put(IN, a.o_rho, g, kCell, gi, gj, k, r1);
-        put(IN, a.o_th, g, kCell, gi, gj, k, a.out_rt ? q1 : th1);
-        if (a.acc_mode == 2) ra.add(th1, kFxTheta);
+  }
+  // K20 (dry_pressure_gradient.cu:27-35): eos_pressure with theta at hand
+  auto pressure = [&](float rho, float th, bool& near) {
+    const float x = fp::div_by(rho * kRd * th, kP0, 1.0f / kP0);
+    near = near && fp::finite(x);
+    return kP0 * powf(fmaxf(x, 1.0e-6f), 1.0f / (1.0f - kKappa));
+  };
+  // theta and pressure of plane kk (kk < nz), and the reciprocals that derive(kk) divides by:
+  // the pressure becomes p_c, the one before it p_m
+  auto derive_theta = [&](int kk) {
+    const float* sr = slot_at(kk);
+    float* th = der + D_TH + (kk & 1) * DN;
+    bool near = true;
+#pragma unroll
+    for (int n = 0; n < NP; ++n) {
+      p_m[n] = p_c[n];
+      if (live & (1u << n)) {
+        const float rho = sr[R_RHO + pos_b[n]], rt = RT(sr, pos_b[n], rho), rr = fmaxf(rho, 1.0e-6f);
+        yrho[n] = fp::recip(rr);
+        const float t = fp::div_by(rt, rr, yrho[n]);
+        near = near && fp::finite(t);
+        th[tid + n * NT] = t;
+        if (live & (256u << n)) p_c[n] = pressure(rho, t, near);
       }
     }
-    // ---- X face: K17 (dry_momentum_flux.cu:79-156) + K21 (dry_pressure_gradient.cu:75-123)
-    {
-      float t_u = 0.0f;
-      if ((IN || !(gi == 0 && open_x))) {
-        const float qw = U(sr, b - 1), qc = uf, qe = U(sr, b + 1);
-        const float qs = U(sr, b - BW), qn = U(sr, b + BW);
-        const float qb = k > 0 ? cy.uf : qc;
-        const float qt = top ? qc : uft;
-        const float flw = fp::upwind(uc[d - 1], qw, qc);
-        const float fle = fp::upwind(uc[d], qc, qe);
-        float fls = 0.0f, fln = 0.0f, flb = 0.0f, flt = 0.0f;
-        if ((IN || !(gj == 0 && open_y))) fls = fp::upwind(fp::avg(vc[d - DW - 1], vc[d - DW]), qs, qc);
-        if ((IN || !(gj + 1 == ny && open_y))) fln = fp::upwind(fp::avg(vc[d - 1], vc[d]), qc, qn);
-        if (k > 0) flb = fp::upwind(fp::avg(wcm[d - 1], wcm[d]), qb, qc);
-        if (!top) flt = fp::upwind(fp::avg(wc[d - 1], wc[d]), qc, qt);
-        t_u = -fp::divergence(fle, flw, fln, fls, flt, flb, idx, idy, fp::avg(mt.w, mt.c));
-        t_u = fp::add_pgf_terrain(t_u, pc, pp[d - 1], sr[R_Z + b], sr[R_Z + b - 1], dz[d - 1], dz[d], idx);
-        if (a.damp_c) t_u = fp::add_damping(t_u, __ldg(a.damp_c + k), qc, __ldg(a.uref + k));
-      }
-      float u1 = fp::update(uf, dt, t_u, -1.0e30f);
-      if (blend) u1 = fp::blend(a.wa, q0.u, a.wb, u1);
-      if (own) put(IN, a.o_u, g, kFaceX, gi, gj, k, u1);
-    }
-    // ---- Y face: K18 (dry_momentum_flux.cu:158-235) + K22 (dry_pressure_gradient.cu:125-173)
-    {
-      float t_v = 0.0f;
-      if ((IN || !(gj == 0 && open_y))) {
-        const float qw = V(sr, b - 1), qc = vf, qe = V(sr, b + 1);
-        const float qs = V(sr, b - BW), qn = V(sr, b + BW);
-        const float qb = k > 0 ? cy.vf : qc;
-        const float qt = top ? qc : vft;
-        float flw = 0.0f, fle = 0.0f, flb = 0.0f, flt = 0.0f;
-        if ((IN || !(gi == 0 && open_x))) flw = fp::upwind(fp::avg(uc[d - DW - 1], uc[d - 1]), qw, qc);
-        if ((IN || !(gi + 1 == nx && open_x))) fle = fp::upwind(fp::avg(uc[d - DW], uc[d]), qc, qe);
-        const float fls = fp::upwind(vc[d - DW], qs, qc);
-        const float fln = fp::upwind(vc[d], qc, qn);
-        if (k > 0) flb = fp::upwind(fp::avg(wcm[d - DW], wcm[d]), qb, qc);
-        if (!top) flt = fp::upwind(fp::avg(wc[d - DW], wc[d]), qc, qt);
-        t_v = -fp::divergence(fle, flw, fln, fls, flt, flb, idx, idy, fp::avg(mt.s, mt.c));
-        t_v = fp::add_pgf_terrain(t_v, pc, pp[d - DW], sr[R_Z + b], sr[R_Z + b - BW], dz[d - DW], dz[d], idy);
-        if (a.damp_c) t_v = fp::add_damping(t_v, __ldg(a.damp_c + k), qc, __ldg(a.vref + k));
-      }
-      float v1 = fp::update(vf, dt, t_v, -1.0e30f);
-      if (blend) v1 = fp::blend(a.wa, q0.v, a.wb, v1);
-      if (own) put(IN, a.o_v, g, kFaceY, gi, gj, k, v1);
-    }
-    // ---- Z face k: K19 (dry_momentum_flux.cu:237-312) + K3 buoyancy (dry_core.cu:146-187)
-    {
-      float t_w = 0.0f;
-      if (k > 0) {
-        const float qw = W(sr, b - 1), qc = wf, qe = W(sr, b + 1);
-        const float qs = W(sr, b - BW), qn = W(sr, b + BW);
-        const float qb = cy.wf, qt = wft;
-        float flw = 0.0f, fle = 0.0f, fls = 0.0f, fln = 0.0f;
-        if ((IN || !(gi == 0 && open_x))) flw = fp::upwind(fp::avg(ucm[d - 1], uc[d - 1]), qw, qc);
-        if ((IN || !(gi + 1 == nx && open_x))) fle = fp::upwind(fp::avg(ucm[d], uc[d]), qc, qe);
-        if ((IN || !(gj == 0 && open_y))) fls = fp::upwind(fp::avg(vcm[d - DW], vc[d - DW]), qs, qc);
-        if ((IN || !(gj + 1 == ny && open_y))) fln = fp::upwind(fp::avg(vcm[d], vc[d]), qc, qn);
-        const float flb = fp::upwind(wcm[d], qb, qc);
-        const float flt = fp::upwind(wc[d], qc, qt);
-        t_w = -fp::divergence(fle, flw, fln, fls, flt, flb, idx, idy, mt.f);
-        t_w = fp::add_buoyancy(t_w, cy.th, tc, s_thref[k - 1], s_thref[k], cy.rho, rho, a.gravity);
-        if (a.damp_c) t_w = fp::add_damping(t_w, __ldg(a.damp_f + k), qc, 0.0f);
-      }
-      float w1 = fp::update(wf, dt, t_w, -1.0e30f);
-      if (blend) w1 = fp::blend(a.wa, q0.w, a.wb, w1);
-      if (own) {
-        put(IN, a.o_w, g, kFaceZ, gi, gj, k, w1);
-        if (top) {  // top face: zero tendency
-          float wt = fmaxf(-1.0e30f, wft);
-          if (blend) wt = fp::blend(a.wa, __ldg(a.w0 + gidx(g, gi, gj, nz)), a.wb, wt);
-          put(IN, a.o_w, g, kFaceZ, gi, gj, nz, wt);
+    if (!near) {  // a value that is not finite: the plain forms
+#pragma unroll
+      for (int n = 0; n < NP; ++n)
+        if (live & (1u << n)) {
+          const float rho = sr[R_RHO + pos_b[n]], rt = RT(sr, pos_b[n], rho);
+          th[tid + n * NT] = fp::theta(rho, rt);
+          if (live & (256u << n)) p_c[n] = eos_pressure(rho, rt);
         }
-      }
     }
-    cy.rho = rho;
-    cy.th = tc;
-    cy.uf = uf;
-    cy.vf = vf;
-    cy.wf = wf;
   };
-
-  // derive plane k at the 34 x 18 positions: theta, uc, vc, wc, the pressure of plane k+1
-  // (first: of plane k too, nothing below it being derived) and, with grad, dp/dz of plane k
-  auto derive = [&](int k, bool first, bool grad) {
+  // uc, vc, wc, p and dp/dz of plane k, with derive_theta(k) done; does derive_theta(k + 1).  grad:
+  // p and dp/dz are wanted (not for the plane below a chunk)
+  auto derive = [&](int k, bool grad) {
     const float* sm = slot_at(k > kg ? k - 1 : kg);  // plane k-1 (its slot is intact)
     const float* sr = slot_at(k);
     const float* sn = slot_at(k + 1);
     float* uc = der + D_UC + (k & 1) * DN;
     float* vc = der + D_VC + (k & 1) * DN;
-    float* wc = der + D_WC + (k & 1) * DN;
-    float* th = der + D_TH;
+    float* wc = der + D_WC;
+    float* pp = der + D_P;
     float* dz = der + D_DZ;
-    float* pm = der + D_P + ((k + 2) % 3) * DN;
-    float* pc = der + D_P + (k % 3) * DN;
-    float* pn = der + D_P + ((k + 1) % 3) * DN;
-    for (int q = tid; q < DN; q += NT) {
-      const int r = q / DW, c = q - r * DW;
-      const int b = r * BW + c + 3;
-      const float rho = sr[R_RHO + b], rt = RT(sr, b);
-      // K20: the full pressure (dry_pressure_gradient.cu:27-35)
-      if (first) pc[q] = eos_pressure(rho, rt);
-      if (k + 1 < nz) pn[q] = eos_pressure(sn[R_RHO + b], RT(sn, b));
-      if (grad) {
-        th[q] = fp::theta(rho, rt);
-        dz[q] = column_dpdz(k, nz, k > 0 ? pm[q] : 0.f, pc[q], k + 1 < nz ? pn[q] : 0.f,
-                            k > 0 ? sm[R_Z + b] : 0.f, sr[R_Z + b], k + 1 < nz ? sn[R_Z + b] : 0.f);
+    bool near = true;
+    auto momenta = [&](int b, float& mu, float& mv, float& mw) {
+      mu = fp::avg(U(sr, b), U(sr, b + 1));
+      mv = fp::avg(V(sr, b), V(sr, b + BW));
+      mw = fp::avg(W(sr, b), W(sn, b));
+    };
+#pragma unroll
+    for (int n = 0; n < NP; ++n)
+      if (live & (256u << n)) {
+        const int b = pos_b[n], q = tid + n * NT;
+        // cell-centred velocities: dry_momentum_flux.cu:36-73
+        const float rr = fmaxf(sr[R_RHO + b], 1.0e-6f), y = yrho[n];
+        float mu, mv, mw;
+        momenta(b, mu, mv, mw);
+        const float cu = fp::div_by(mu, rr, y), cv = fp::div_by(mv, rr, y), cw = fp::div_by(mw, rr, y);
+        near = near && fp::finite(fabsf(cu) + fabsf(cv) + fabsf(cw));
+        uc[q] = cu;
+        vc[q] = cv;
+        wc[q] = cw;
       }
-      // cell-centred velocities: dry_momentum_flux.cu:36-73
-      const float rr = fmaxf(rho, 1.0e-6f);
-      uc[q] = fp::centred(U(sr, b), U(sr, b + 1), rr);
-      vc[q] = fp::centred(V(sr, b), V(sr, b + BW), rr);
-      wc[q] = fp::centred(W(sr, b), W(sn, b), rr);
+    if (!near) {  // a quotient that is not finite: plain divisions
+#pragma unroll 1
+      for (int n = 0; n < NP; ++n) {
+        if (!(live & (256u << n))) continue;
+        const int q = tid + n * NT, r = q / DW, b = r * BW + (q - r * DW) + 3;
+        const float rr = fmaxf(sr[R_RHO + b], 1.0e-6f);
+        float mu, mv, mw;
+        momenta(b, mu, mv, mw);
+        uc[q] = fp::div(mu, rr);
+        vc[q] = fp::div(mv, rr);
+        wc[q] = fp::div(mw, rr);
+      }
+    }
+    float below[NP];  // the pressure at plane k-1
+#pragma unroll
+    for (int n = 0; n < NP; ++n) below[n] = p_m[n];
+    if (k + 1 < nz) {  // p_m, p_c become the pressures at planes k and k+1
+      derive_theta(k + 1);
+    } else {
+#pragma unroll
+      for (int n = 0; n < NP; ++n) {
+        p_m[n] = p_c[n];
+        p_c[n] = 0.f;
+      }
+    }
+    if (!grad) return;
+#pragma unroll
+    for (int n = 0; n < NP; ++n)
+      if (live & (256u << n)) {
+        const int b = pos_b[n], q = tid + n * NT;
+        pp[q] = p_m[n];
+        dz[q] = column_dpdz(k, nz, below[n], p_m[n], p_c[n], k > 0 ? sm[R_Z + b] : 0.f, sr[R_Z + b],
+                            k + 1 < nz ? sn[R_Z + b] : 0.f);
+      }
+  };
+
+  // Values of the thread's columns carried up: the stage input at plane k, theta and rho of
+  // plane k-1, and the vertical fluxes through the faces between planes k-1 and k (the flux
+  // out of a plane's top is the one into the next plane's bottom)
+  float rho_c[ROWS], u_c[ROWS], v_c[ROWS], w_c[ROWS], th_l[ROWS], rho_l[ROWS];
+  float fz_th[ROWS], fz_u[ROWS], fz_v[ROWS], fz_w[ROWS];
+  const int d0 = (r0 + 1) * DW + tx + 1, b0 = (r0 + 1) * BW + tx + 4;  // derived and box index of row 0
+  auto load_column = [&](int kk) {
+    const float* sr = slot_at(kk);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      rho_c[r] = sr[R_RHO + b0 + r * BW];
+      u_c[r] = U(sr, b0 + r * BW);
+      v_c[r] = V(sr, b0 + r * BW);
+      w_c[r] = W(sr, b0 + r * BW);
     }
   };
-  if (kb > 0) {  // the plane below the chunk: its derived values, and the column's own
+#pragma unroll
+  for (int n = 0; n < NP; ++n) p_c[n] = 0.f;
+  wait_plane(kg, kb);
+  derive_theta(kg);
+  load_column(kg);
+  if (kb > 0) {  // the plane below the chunk: its derived values and the fluxes out of its top
     wait_plane(kb, kb);
-    derive(kg, true, false);
-    const float* sr = slot_at(kg);
-    auto carry = [&](int r) {
-      const int b = r * BW + tx + 4;
-      return TerrCarry{sr[R_RHO + b], fp::theta(sr[R_RHO + b], RT(sr, b)), U(sr, b), V(sr, b), W(sr, b)};
-    };
-    ca = carry(ty + 1);
-    cb = carry(ty + RY + 1);
+    derive(kg, false);
+    __syncthreads();
+    const float* wc = der + D_WC;
+    const float* tl = der + D_TH + (kg & 1) * DN;
+    const float* tu = der + D_TH + (kb & 1) * DN;
+    float u[ROWS], v[ROWS], ww[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      u[r] = u_c[r];
+      v[r] = v_c[r];
+      ww[r] = w_c[r];
+      rho_l[r] = rho_c[r];
+    }
+    load_column(kb);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int d = d0 + r * DW;
+      th_l[r] = tl[d];
+      fz_th[r] = fp::upwind(w_c[r], tl[d], tu[d]);
+      fz_u[r] = fp::upwind(fp::avg(wc[d - 1], wc[d]), u[r], u_c[r]);
+      fz_v[r] = fp::upwind(fp::avg(wc[d - DW], wc[d]), v[r], v_c[r]);
+      fz_w[r] = fp::upwind(wc[d], ww[r], w_c[r]);
+    }
+    __syncthreads();  // wc is derived anew for plane kb
+  } else {
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) th_l[r] = rho_l[r] = fz_th[r] = fz_u[r] = fz_v[r] = fz_w[r] = 0.f;
   }
 
-  // Interior tiles (full, away from every periodic edge ring and open side) run a copy of
-  // the plane loop compiled without the edge logic; both copies do the same arithmetic.
-  const bool interior = !edge && (g.per_x || (i0 > 0 && i0 + TX < nx)) && (g.per_y || (j0 > 0 && j0 + TY < ny));
+  // damping constants of the plane
+  struct PlaneConst {
+    float damp_c, damp_f, uref, vref;
+  };
+  auto plane_const = [&](int k) {
+    PlaneConst pc{0.0f, 0.0f, 0.0f, 0.0f};
+    if (a.damp_c) {
+      pc.damp_c = __ldg(a.damp_c + k);
+      pc.damp_f = __ldg(a.damp_f + k);
+      pc.uref = __ldg(a.uref + k);
+      pc.vref = __ldg(a.vref + k);
+    }
+    return pc;
+  };
+
+  // cells, X faces, Y faces and Z faces of plane k in the thread's rows (+ the top faces)
+  auto columns = [&](auto tile_class, int k, const SlowBlend* q0, const TerrMetric* mt, long long& ra,
+                     const PlaneConst& kc) {
+    constexpr bool IN = decltype(tile_class)::value;  // an interior tile
+    // store of an owned value at plane k + up: a plain store in interior tiles, else with the
+    // periodic mirrors
+    auto put = [&](float* f, int o, int r, int up, float v) {
+      if (IN) f[off[r] + up * g.plane] = v;
+      else if (own_rt[r]) store_tile(f, g, o, gi, gj + r, k + up, v, edge);
+    };
+    const float* sr = slot_at(k);
+    const float* sn = slot_at(k + 1);
+    const float* uc = der + D_UC + (k & 1) * DN;
+    const float* vc = der + D_VC + (k & 1) * DN;
+    const float* wc = der + D_WC;
+    const float* ucm = der + D_UC + ((k + 1) & 1) * DN;  // plane k-1
+    const float* vcm = der + D_VC + ((k + 1) & 1) * DN;
+    const float* th = der + D_TH + (k & 1) * DN;
+    const float* thn = der + D_TH + ((k + 1) & 1) * DN;  // plane k+1
+    const float* pp = der + D_P;
+    const float* dz = der + D_DZ;
+    const bool top = k + 1 == nz;
+    const bool sx0 = !IN && gi == 0 && open_x, sx1 = !IN && gi + 1 == nx && open_x;  // no flux through the side
+    bool sy[ROWS + 1];  // the Y face below row r lies on an open side
+#pragma unroll
+    for (int r = 0; r <= ROWS; ++r) sy[r] = !IN && open_y && (gj + r == 0 || gj + r == ny);
+    // column values of plane k+1 (plane nz holds the top faces only)
+    float rho_n[ROWS], u_n[ROWS], v_n[ROWS], w_n[ROWS], tc[ROWS + 2], tt[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS + 2; ++r) tc[r] = th[d0 + (r - 1) * DW];  // rows -1 .. ROWS
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      const int b = b0 + r * BW;
+      w_n[r] = W(sn, b);
+      if (!top) {
+        rho_n[r] = sn[R_RHO + b];
+        u_n[r] = U(sn, b);
+        v_n[r] = V(sn, b);
+        tt[r] = thn[d0 + r * DW];
+      } else {
+        rho_n[r] = 0.f;
+        u_n[r] = u_c[r];
+        v_n[r] = v_c[r];
+        tt[r] = tc[r + 1];
+      }
+    }
+    const float u_s = U(sr, b0 - BW), u_t = U(sr, b0 + ROWS * BW);  // rows -1 and ROWS
+    const float v_s = V(sr, b0 - BW), v_t = V(sr, b0 + ROWS * BW);
+    // the wind in the rows -1 .. ROWS-1: at the column and (vc) averaged onto its X face, (uc)
+    // its two cells
+    float uw[ROWS + 1], ue[ROWS + 1], vx[ROWS + 1], vv[ROWS + 1];
+#pragma unroll
+    for (int r = 0; r <= ROWS; ++r) {
+      const int d = d0 + (r - 1) * DW;
+      uw[r] = uc[d - 1];
+      ue[r] = uc[d];
+      vv[r] = vc[d];
+      vx[r] = fp::avg(vc[d - 1], vv[r]);
+    }
+    // ---- cells: K2 compute_cell_tendencies_kernel (dry_core.cu:62-144)
+    {
+      float gy[ROWS + 1];
+#pragma unroll
+      for (int r = 0; r <= ROWS; ++r) gy[r] = fp::upwind(r < ROWS ? v_c[r] : v_t, tc[r], tc[r + 1]);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int d = d0 + r * DW, b = b0 + r * BW;
+        const float fw = u_c[r], fe = U(sr, b + 1), fs = v_c[r], fn = r + 1 < ROWS ? v_c[r + 1] : v_t;
+        const float fb = w_c[r], ft = w_n[r], rho = rho_c[r], rt = RT(sr, b, rho);
+        const float t_rho = -fp::divergence(fe, fw, fn, fs, ft, fb, idx, idy, mt[r].c);
+        const float gw = fp::upwind(fw, th[d - 1], tc[r + 1]), ge = fp::upwind(fe, tc[r + 1], th[d + 1]);
+        const float gb = k > 0 ? fz_th[r] : fp::upwind(fb, tc[r + 1], tc[r + 1]);
+        const float gt = fp::upwind(ft, tc[r + 1], tt[r]);
+        fz_th[r] = gt;
+        const float t_rt = -fp::divergence(ge, gw, gy[r + 1], gy[r], gt, gb, idx, idy, mt[r].c);
+        float r1 = fp::update(rho, dt, t_rho, 1.0e-6f);
+        float q1 = fp::update(rt, dt, t_rt, 1.0e-6f);
+        if (BLEND) {
+          r1 = fp::blend(a.wa, q0[r].rho, a.wb, r1);
+          q1 = fp::blend(a.wa, q0[r].rt, a.wb, q1);
+        }
+        const float th1 = fp::theta(r1, q1);
+        put(a.o_rho, kCell, r, 0, r1);
+        put(a.o_th, kCell, r, 0, a.out_rt ? q1 : th1);
+        if (a.acc_mode == 2 && (IN || own_rt[r])) ra += fx(th1, kFxTheta);
+      }
+    }
+    // ---- X faces: K17 (dry_momentum_flux.cu:79-156) + K21 (dry_pressure_gradient.cu:75-123)
+    {
+      float fy[ROWS + 1];
+#pragma unroll
+      for (int r = 0; r <= ROWS; ++r) {
+        fy[r] = fp::upwind(vx[r], r > 0 ? u_c[r - 1] : u_s, r < ROWS ? u_c[r] : u_t);
+        if (sy[r]) fy[r] = 0.0f;
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int d = d0 + r * DW, b = b0 + r * BW;
+        const float qc = u_c[r];
+        const float flw = fp::upwind(uw[r + 1], U(sr, b - 1), qc), fle = fp::upwind(ue[r + 1], qc, U(sr, b + 1));
+        const float flt = top ? 0.0f : fp::upwind(fp::avg(wc[d - 1], wc[d]), qc, u_n[r]);
+        float t_u = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_u[r], idx, idy,
+                                    fp::avg(mt[r].w, mt[r].c));
+        fz_u[r] = flt;
+        t_u = fp::add_pgf_terrain(t_u, pp[d], pp[d - 1], sr[R_Z + b], sr[R_Z + b - 1], dz[d - 1], dz[d], idx);
+        if (a.damp_c) t_u = fp::add_damping(t_u, kc.damp_c, qc, kc.uref);
+        if (sx0) t_u = 0.0f;
+        float u1 = fp::update(qc, dt, t_u, -1.0e30f);
+        if (BLEND) u1 = fp::blend(a.wa, q0[r].u, a.wb, u1);
+        put(a.o_u, kFaceX, r, 0, u1);
+      }
+    }
+    // ---- Y faces: K18 (dry_momentum_flux.cu:158-235) + K22 (dry_pressure_gradient.cu:125-173)
+    {
+      float fy[ROWS + 1];
+#pragma unroll
+      for (int r = 0; r <= ROWS; ++r)
+        fy[r] = fp::upwind(vv[r], r > 0 ? v_c[r - 1] : v_s, r < ROWS ? v_c[r] : v_t);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int d = d0 + r * DW, b = b0 + r * BW;
+        const float qc = v_c[r];
+        float flw = fp::upwind(fp::avg(uw[r], uw[r + 1]), V(sr, b - 1), qc);
+        float fle = fp::upwind(fp::avg(ue[r], ue[r + 1]), qc, V(sr, b + 1));
+        if (sx0) flw = 0.0f;
+        if (sx1) fle = 0.0f;
+        const float flt = top ? 0.0f : fp::upwind(fp::avg(wc[d - DW], wc[d]), qc, v_n[r]);
+        float t_v = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_v[r], idx, idy,
+                                    fp::avg(mt[r].s, mt[r].c));
+        fz_v[r] = flt;
+        t_v = fp::add_pgf_terrain(t_v, pp[d], pp[d - DW], sr[R_Z + b], sr[R_Z + b - BW], dz[d - DW], dz[d], idy);
+        if (a.damp_c) t_v = fp::add_damping(t_v, kc.damp_c, qc, kc.vref);
+        if (!IN && gj + r == 0 && open_y) t_v = 0.0f;
+        float v1 = fp::update(qc, dt, t_v, -1.0e30f);
+        if (BLEND) v1 = fp::blend(a.wa, q0[r].v, a.wb, v1);
+        put(a.o_v, kFaceY, r, 0, v1);
+      }
+    }
+    // ---- Z faces k: K19 (dry_momentum_flux.cu:237-312) + K3 buoyancy (dry_core.cu:146-187)
+    {
+      float fy[ROWS + 1];
+      if (k > 0) {
+        const float w_s = W(sr, b0 - BW), w_t = W(sr, b0 + ROWS * BW);
+#pragma unroll
+        for (int r = 0; r <= ROWS; ++r) {
+          fy[r] = fp::upwind(fp::avg(vcm[d0 + (r - 1) * DW], vv[r]), r > 0 ? w_c[r - 1] : w_s, r < ROWS ? w_c[r] : w_t);
+          if (sy[r]) fy[r] = 0.0f;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int d = d0 + r * DW, b = b0 + r * BW;
+        const float qc = w_c[r];
+        const float flt = fp::upwind(wc[d], qc, w_n[r]);
+        float t_w = 0.0f;
+        if (k > 0) {
+          float flw = fp::upwind(fp::avg(ucm[d - 1], uw[r + 1]), W(sr, b - 1), qc);
+          float fle = fp::upwind(fp::avg(ucm[d], ue[r + 1]), qc, W(sr, b + 1));
+          if (sx0) flw = 0.0f;
+          if (sx1) fle = 0.0f;
+          t_w = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_w[r], idx, idy, mt[r].f);
+          bool near = true;
+          const float t = fp::add_buoyancy_ref(t_w, th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r],
+                                               a.gravity, near);
+          t_w = near ? t : fp::add_buoyancy(t_w, th_l[r], tc[r + 1], s_trf[k], rho_l[r], rho_c[r], a.gravity);
+          if (a.damp_c) t_w = fp::add_damping(t_w, kc.damp_f, qc, 0.0f);
+        }
+        fz_w[r] = flt;
+        float w1 = fp::update(qc, dt, t_w, -1.0e30f);
+        if (BLEND) w1 = fp::blend(a.wa, q0[r].w, a.wb, w1);
+        put(a.o_w, kFaceZ, r, 0, w1);
+        if (top) {  // top face: zero tendency
+          float wt = fmaxf(-1.0e30f, w_n[r]);
+          if (BLEND && own_rt[r]) wt = fp::blend(a.wa, __ldg(a.w0 + off[r] + g.plane), a.wb, wt);
+          put(a.o_w, kFaceZ, r, 1, wt);
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      th_l[r] = tc[r + 1];
+      rho_l[r] = rho_c[r];
+      rho_c[r] = rho_n[r];
+      u_c[r] = u_n[r];
+      v_c[r] = v_n[r];
+      w_c[r] = w_n[r];
+    }
+  };
+
+  // Interior tiles (full, away from every periodic edge ring and open side) run a copy
+  // of the plane loop compiled without the edge logic: plain stores, none of the
+  // open-boundary flux tests.  Both copies do the same arithmetic on the same values.
+  const bool interior = !edge && i0 + TX <= nx && j0 + TY <= ny && (g.per_x || (i0 > 0 && i0 + TX < nx)) &&
+                        (g.per_y || (j0 > 0 && j0 + TY < ny));
   auto plane_loop = [&](auto tile_class) -> bool {  // true when a bounded wait gave up
     constexpr bool IN = decltype(tile_class)::value;
     for (int k = kb; k < ke; ++k) {
       const int pb = k & 1;
+      const PlaneConst kc = plane_const(k);
+      SlowBlend q0[ROWS];  // the derive phase covers the loads
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(r);
+      TerrMetric mt[ROWS];
+      load_metric(mt);
       wait_plane(k + 1, k);
-      derive(k, k == 0, true);
-      const TerrBlend n0a = load_q0(gj0, own0, k + 1), n0b = load_q0(gj1, own1, k + 1);
-      const TerrMetric nma = load_metric(gj0, own0, k + 1), nmb = load_metric(gj1, own1, k + 1);
+      derive(k, true);
       __syncthreads();  // publishes plane k's derived values; slot (k-1) is free
       if (s_abort[pb]) return true;
       if (tid == ISSUER) {
@@ -395,31 +600,28 @@ __global__ void __launch_bounds__(st::NT, 2)
         if (k + 2 <= ke) { issue(k + 2); issued = k + 2; }
       }
       // ---- cells and faces of plane k
-      FxAcc ra;
-      column(tile_class, k, ty + 1, gj0, own0, ca, q0a, m0a, ra);
-      column(tile_class, k, ty + RY + 1, gj1, own1, cb, q0b, m0b, ra);
+      long long ra = 0;
+      columns(tile_class, k, q0, mt, ra, kc);
       if (!IN && xf) {  // open east boundary: X face nx of row j0+tx
         const float* sr = slot_at(k);
         const float uf = U(sr, (tx + 1) * BW + w + 4);
         float u1 = fp::update(uf, dt, 0.0f, -1.0e30f);
-        if (blend) u1 = fp::blend(a.wa, __ldg(a.u0 + gidx(g, nx, j0 + tx, k)), a.wb, u1);
-        put(false, a.o_u, g, kFaceX, nx, j0 + tx, k, u1);
+        if (BLEND) u1 = fp::blend(a.wa, __ldg(a.u0 + gidx(g, nx, j0 + tx, k)), a.wb, u1);
+        store_tile(a.o_u, g, kFaceX, nx, j0 + tx, k, u1, edge);
       }
       if (!IN && yf) {  // open north boundary: Y face ny of column i0+tx
         const float* sr = slot_at(k);
         const float vf = V(sr, (h + 1) * BW + tx + 4);
         float v1 = fp::update(vf, dt, 0.0f, -1.0e30f);
-        if (blend) v1 = fp::blend(a.wa, __ldg(a.v0 + gidx(g, i0 + tx, ny, k)), a.wb, v1);
-        put(false, a.o_v, g, kFaceY, i0 + tx, ny, k, v1);
+        if (BLEND) v1 = fp::blend(a.wa, __ldg(a.v0 + gidx(g, i0 + tx, ny, k)), a.wb, v1);
+        store_tile(a.o_v, g, kFaceY, i0 + tx, ny, k, v1, edge);
       }
       if (a.acc_mode) {
-        const long long ta = ra.warp_total();
+        const long long ta = warp_total_fx(ra);
         if (tx == 0) s_red[pb][ty] = ta;
       }
-      q0a = n0a;
-      q0b = n0b;
-      m0a = nma;
-      m0b = nmb;
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) off[r] += g.plane;
       __syncthreads();  // every thread is done with plane k's derived values
     }
     return false;
@@ -438,25 +640,34 @@ __global__ void __launch_bounds__(st::NT, 2)
   }
 }
 
+template <bool FIRST, bool INC>
+cudaError_t allow_smem() {
+  return cudaFuncSetAttribute(k_slow_terrain_tma<FIRST, INC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)st::smem_bytes(INC));
+}
+
 }  // namespace
 
 cudaError_t init_slow_terrain_tma() {
-  cudaError_t e = cudaFuncSetAttribute(k_slow_terrain_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)st::smem_bytes(true));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_slow_terrain_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)st::smem_bytes(false));
+  cudaError_t e = allow_smem<true, false>();
+  if (e == cudaSuccess) e = allow_smem<false, false>();
+  if (e == cudaSuccess) e = allow_smem<false, true>();
+  return e;
 }
 
 cudaError_t launch_slow_terrain_tma(const SlowArgs& a, const SlowMaps& m, cudaStream_t s) {
-  if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || a.tend_only || a.acc_mode == 1 || !a.idz_c || !a.idz_f)
+  // a step's first stage takes rho*theta and no blend, the others theta and q0
+  const bool first = a.th_is_rt != 0;
+  if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || a.tend_only || a.acc_mode == 1 || !a.idz_c || !a.idz_f ||
+      first != !a.rho0 || (first && a.du))
     return cudaErrorInvalidValue;
-  const dim3 block(st::TX, st::RY);
+  const dim3 block(st::TX, st::NW);
   dim3 grid((a.g.nx + st::TX - 1) / st::TX, (a.g.ny + st::TY - 1) / st::TY);
   const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 2, 1.2f);
   grid.z = zs.chunks;
-  if (a.du) k_slow_terrain_tma<true><<<grid, block, st::smem_bytes(true), s>>>(a, m, zs);
-  else k_slow_terrain_tma<false><<<grid, block, st::smem_bytes(false), s>>>(a, m, zs);
+  if (first) k_slow_terrain_tma<true, false><<<grid, block, st::smem_bytes(false), s>>>(a, m, zs);
+  else if (a.du) k_slow_terrain_tma<false, true><<<grid, block, st::smem_bytes(true), s>>>(a, m, zs);
+  else k_slow_terrain_tma<false, false><<<grid, block, st::smem_bytes(false), s>>>(a, m, zs);
   return cudaGetLastError();
 }
 
