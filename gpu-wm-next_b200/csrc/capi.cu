@@ -530,6 +530,8 @@ bool fast_terrain_maps(const Member& M, const FastArgs& f, bool first, FastTerra
 cudaError_t launch_substep(gwm_b200_ctx* c, const Member& M, const FastArgs& f, bool first, bool terr,
                            bool p_ready = false) {
   if (terr && fast_tma_path(c)) {
+    // the TMA kernel updates momenta and density; without one of them the overlapped tiles run
+    if (!f.hmom || !f.dens) return launch_fast(f, first, terr, c->stream, 8);
     FastTerrainMaps m{};
     if (!fast_terrain_maps(M, f, first, m)) return cudaErrorInvalidValue;
     return launch_fast_terrain_tma(f, m, first, c->stream);

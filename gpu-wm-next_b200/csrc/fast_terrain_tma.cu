@@ -6,7 +6,7 @@
 // hydrostatic reference of :108-158, which k_column_reference builds before the
 // substep), with the data path of k_fast_tma: one elected thread per CTA fetches every
 // plane's tiles with cp.async.bulk.tensor.3d into a five-slot shared-memory ring, and a
-// CTA owns a 32 x 16 tile, two rows per thread.  Per plane kk the slot holds
+// CTA owns a 32 x 16 tile, two adjacent rows per thread.  Per plane kk the slot holds
 //   rho(kk), theta(kk)   first substep of a stage: 40 x 18 boxes (the tile and its halo
 //                        ring, from which the full pressure is derived); otherwise the
 //                        owned 32 x 16 box
@@ -20,7 +20,8 @@
 // The vertical pressure derivative of the tile and its ring takes p at three levels; it
 // is derived one plane ahead (plane k+1 while plane k's faces are computed, from the
 // slots of planes k, k+1, k+2), so one barrier per plane publishes it together with the
-// new face increments.  The owned cells' metric columns, column reference and (last
+// new face increments.  A thread carries p, z and dp/dz of its rows up, so it reads each once,
+// and computes the Y face between its rows itself.  The owned cells' metric columns, column reference and (last
 // substep of the step) stage base momenta are per-thread coalesced loads issued one
 // plane ahead.
 #include <type_traits>
@@ -34,7 +35,7 @@ namespace gwmb {
 namespace {
 
 namespace fz {
-constexpr int TX = 32, TY = 16, RY = 8, NT = 256, NW = NT / 32;
+constexpr int TX = 32, TY = 16, ROWS = 2, NT = 256, NW = NT / 32;
 constexpr int CBW = 40, CBH = 18;  // cell box: tile + halo ring, x from i0-4 (16-byte aligned)
 constexpr int FBW = 36, FBH = 17;  // face box: owned faces + the tile's east/north face
 constexpr int OBW = 32, OBH = 16;  // owned box
@@ -77,41 +78,39 @@ constexpr size_t dyn_smem() {
 template <bool FIRST>
 struct TerrainShared {
   float p[FIRST ? 3 : 1][fz::PH][fz::PW];
-  float dz[2][fz::PH][fz::PW];     // dp/dz of the tile and its ring (column_dpdz)
-  float du[2][fz::TY][fz::TX + 1];  // new X-face increments (own + east face)
-  float dv[2][fz::TY + 1][fz::TX];  // new Y-face increments (own + north face)
-  long long red[2][fz::NW][2];
+  float dz[2][fz::PH][fz::PW];               // dp/dz of the tile and its ring (column_dpdz)
+  float du[2][fz::TY][fz::TX + 1];           // new X-face increments (own + east face)
+  float dv[2][fz::TY / fz::ROWS + 1][fz::TX];  // new Y-face increments below each thread's rows, and the north face
+  long long red[2][fz::NW];
   __align__(8) uint64_t bar[fz::NSLOT];
   int abort[2];
 };
 
-// Owned-cell columns of one plane, loaded a plane ahead of their use.
+// Owned-cell columns of one row at one plane, loaded a plane ahead of their use.
 struct TerrainCol {
   float idzc, idzf, pref, rref, bu, bv, bw;  // idzf, bw: face k+1; pref, rref: level k+1
 };
 
-template <bool FIRST>
+template <bool FIRST, int KIND>  // KIND: FastArgs::final_kind
 __global__ void __launch_bounds__(fz::NT, 2)
     k_fast_terrain_tma(const FastArgs a, const __grid_constant__ FastTerrainMaps m, ZSplit zs) {
   using namespace fz;
   using L = Slot<FIRST>;
   constexpr int O_RHO = L::O_RHO, O_TH = L::O_TH, O_Z = L::O_Z, O_P = L::O_P, O_DU = L::O_DU, O_DV = L::O_DV,
                 O_DW = L::O_DW, RW = L::RW, R0 = L::R0, C0 = L::C0, SLOT = L::SIZE;
+  constexpr bool FINAL = KIND == 2;
   extern __shared__ unsigned char s_dyn[];
   __shared__ TerrainShared<FIRST> S;
   float* const ring = reinterpret_cast<float*>(align_smem_128(s_dyn));
 
   const Geom& g = a.g;
   const int nz = g.nz;
-  const bool final_step = a.final_kind == 2;
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const int i0 = blockIdx.x * TX, j0 = blockIdx.y * TY;
   const int nx = g.nx, ny = g.ny;
   const int w = min(TX, nx - i0), h = min(TY, ny - j0);
-  const bool own0 = tx < w && ty < h, own1 = tx < w && ty + RY < h;
-  const int gi = i0 + tx, gj0 = j0 + ty, gj1 = j0 + ty + RY;
-  const bool skip_u = gi == 0 && !g.per_x;  // open west face (never changes)
-  const bool skip_v0 = gj0 == 0 && !g.per_y;
+  const int r0 = ty * ROWS, gi = i0 + tx, gj = j0 + r0;  // the thread's column and first row
+  const bool own_rt[ROWS] = {tx < w && r0 < h, tx < w && r0 + 1 < h};
   const bool edge = (g.per_x && (i0 <= 1 || i0 + w >= nx - 1)) || (g.per_y && (j0 <= 1 || j0 + h >= ny - 1));
   // halo roles (threads 0-95, whole warps): 0 west column, 1 east column, 2 south row,
   // 3 north row; (hr, hc) in derived-plane coordinates (row 0 = j0-1, column 0 = i0-1)
@@ -122,10 +121,9 @@ __global__ void __launch_bounds__(fz::NT, 2)
   else if (tid < 2 * TY + 2 * TX) { if (tid - 2 * TY - TX < w) { role = 3; hr = h + 1; hc = tid - 2 * TY - TX + 1; } }
   const int hi = i0 + hc - 1, hj = j0 + hr - 1;  // global cell of the halo role
   const bool h_skip = (role == 1 && hi == nx && !g.per_x) || (role == 3 && hj == ny && !g.per_y);
-  const float idx = g.inv_dx, idy = g.inv_dy, dtf = a.dtf;
+  const float idx = g.inv_dx, idy = g.inv_dy, dtf = a.dtf, gravity = a.gravity;
   // terrain: no reference level sums; theta level sums of a stage's result
-  const int acc_mode = (a.acc_off || a.final_kind == 0) ? 0 : 2;
-  const bool hm = a.hmom != 0, dn = a.dens != 0;
+  const bool acc = KIND != 0 && !a.acc_off;
 
   if (tid == 0) {
     for (int s = 0; s < NSLOT; ++s) mbar_init(&S.bar[s], 1);
@@ -137,14 +135,14 @@ __global__ void __launch_bounds__(fz::NT, 2)
     for (int q = tid; q < nz; q += NT) { a.clr_a[q] = 0ull; a.clr_b[q] = 0ull; }
   __syncthreads();
 
-  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads
-  // of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
+  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads of
+  // one of its planes unissued, so that CTA's bounded wait runs out
   int stall = -1;
   if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
   // the CTA's planes are kb .. ke-1; it also loads the planes around them: the one below for
   // its lowest Z face and dp/dz, the one above for its highest
   const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0, kl = min(ke, nz - 1);
-  if (stall >= 0) stall = kg + stall % (kl - kg + 1);  // a plane that this CTA loads
+  if (stall >= 0) stall = kg + stall % (kl - kg + 1);
   auto slot_of = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
   auto issue = [&](int kk) {
     float* st = slot_of(kk);
@@ -185,219 +183,253 @@ __global__ void __launch_bounds__(fz::NT, 2)
     else return slot_of(kk)[O_P + r * CBW + c + 3];
   };
   auto Zv = [&](int kk, int r, int c) { return slot_of(kk)[O_Z + r * CBW + c + 3]; };
-  // K10 + K20 (first substep): the full pressure of plane kk at the thread's positions
-  auto derive_p = [&](int kk) {
+  // p and z of plane kk in the thread's rows.  First substep, K10 + K20: the full pressure is
+  // derived, at the thread's halo role too, and published.
+  auto load_level = [&](int kk, float* p, float* z) {
+    const float* st = slot_of(kk);
+    auto derive = [&](int r, int c) {
+      const float rho = st[O_RHO + r * CBW + c + 3], th = st[O_TH + r * CBW + c + 3];
+      return eos_pressure(rho, fp::mul(rho, th));
+    };
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      z[r] = Zv(kk, r0 + r + 1, tx + 1);
+      if constexpr (FIRST) {
+        p[r] = derive(r0 + r + 1, tx + 1);
+        if (own_rt[r]) S.p[kk % 3][r0 + r + 1][tx + 1] = p[r];
+      } else {
+        p[r] = Pv(kk, r0 + r + 1, tx + 1);
+      }
+    }
     if constexpr (FIRST) {
-      const float* st = slot_of(kk);
-      auto one = [&](int r, int c) {
-        const float rho = st[O_RHO + r * CBW + c + 3], th = st[O_TH + r * CBW + c + 3];
-        S.p[kk % 3][r][c] = eos_pressure(rho, fp::mul(rho, th));
-      };
-      if (own0) one(ty + 1, tx + 1);
-      if (own1) one(ty + RY + 1, tx + 1);
-      if (role >= 0) one(hr, hc);
+      if (role >= 0) S.p[kk % 3][hr][hc] = derive(hr, hc);
     }
   };
-  // dp/dz of plane kk at the thread's positions (planes kk-1 .. kk+1 resident)
-  auto derive_dz = [&](int kk) {
-    auto one = [&](int r, int c) {
-      const float pc = Pv(kk, r, c), zc = Zv(kk, r, c);
-      const float pm = kk > 0 ? Pv(kk - 1, r, c) : 0.f, zm = kk > 0 ? Zv(kk - 1, r, c) : 0.f;
-      const float pn = kk + 1 < nz ? Pv(kk + 1, r, c) : 0.f, zn = kk + 1 < nz ? Zv(kk + 1, r, c) : 0.f;
-      S.dz[kk & 1][r][c] = column_dpdz(kk, nz, pm, pc, pn, zm, zc, zn);
-    };
-    if (own0) one(ty + 1, tx + 1);
-    if (own1) one(ty + RY + 1, tx + 1);
-    if (role >= 0) one(hr, hc);
+  // dp/dz of plane kk at the thread's halo role (planes kk-1 .. kk+1 resident)
+  auto role_dz = [&](int kk) {
+    if (role < 0) return;
+    const float pm = kk > 0 ? Pv(kk - 1, hr, hc) : 0.f, zm = kk > 0 ? Zv(kk - 1, hr, hc) : 0.f;
+    const float pn = kk + 1 < nz ? Pv(kk + 1, hr, hc) : 0.f, zn = kk + 1 < nz ? Zv(kk + 1, hr, hc) : 0.f;
+    S.dz[kk & 1][hr][hc] = column_dpdz(kk, nz, pm, Pv(kk, hr, hc), pn, zm, Zv(kk, hr, hc), zn);
   };
-  // owned-cell columns of plane kk (zeros above the top)
-  auto load_col = [&](bool own, int gj, int kk) {
+  int off[ROWS];  // the owned cells of the current plane
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) off[r] = gidx(g, gi, gj + r, kb);
+  // owned-cell columns of plane kk, `up` planes above the current one (zeros above the top)
+  auto load_col = [&](int r, int kk, int up) {
     TerrainCol c{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (!own || kk >= nz) return c;
-    const int o = gidx(g, gi, gj, kk);
+    if (!own_rt[r] || kk >= nz) return c;
+    const int o = off[r] + up * g.plane;
     c.idzc = __ldg(a.idz_c + o);
     if (kk + 1 < nz) {
       c.idzf = __ldg(a.idz_f + o + g.plane);
       c.pref = __ldg(a.col_pref + o + g.plane);
       c.rref = __ldg(a.col_rref + o + g.plane);
     }
-    if (final_step) {
+    if (FINAL) {
       c.bu = __ldg(a.bu + o);
       c.bv = __ldg(a.bv + o);
       c.bw = __ldg(a.bw + o + g.plane);
     }
     return c;
   };
+  auto rho_at = [&](int kk, int r) { return slot_of(kk)[O_RHO + (r0 + r + R0) * RW + tx + C0]; };
 
   if (tid == ISSUER)
     for (int kk = kg; kk < kb + AHEAD && kk <= kl; ++kk) { issue(kk); issued = kk; }
-  // the column reference at the chunk's lowest level and the step's bottom face
-  float prc0 = 0.f, rrc0 = 0.f, prc1 = 0.f, rrc1 = 0.f, bwz0 = 0.f, bwz1 = 0.f;
-  float dwc0 = 0.f, dwc1 = 0.f;  // increment at face k (face 0 never changes)
-  if (own0) {
-    const int o = gidx(g, gi, gj0, kb);
-    prc0 = __ldg(a.col_pref + o); rrc0 = __ldg(a.col_rref + o);
-    if (final_step && kb == 0) bwz0 = __ldg(a.bw + o);
+  // Carried up the thread's rows: p and z of planes k and k+1, dp/dz of plane k, rho and the
+  // perturbations about the column reference at plane k, the increment of face k
+  float p0[ROWS], z0[ROWS], p1[ROWS], z1[ROWS], dz0[ROWS], rc[ROWS], pa[ROWS], ra[ROWS], dwc[ROWS], bwz[ROWS];
+  TerrainCol col[ROWS];
+  float prk[ROWS], rrk[ROWS];  // the column reference at plane kb
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    prk[r] = rrk[r] = bwz[r] = dwc[r] = 0.f;  // face 0 never changes
+    if (own_rt[r]) {
+      prk[r] = __ldg(a.col_pref + off[r]);
+      rrk[r] = __ldg(a.col_rref + off[r]);
+      if (FINAL && kb == 0) bwz[r] = __ldg(a.bw + off[r]);
+    }
+    col[r] = load_col(r, kb, 0);
   }
-  if (own1) {
-    const int o = gidx(g, gi, gj1, kb);
-    prc1 = __ldg(a.col_pref + o); rrc1 = __ldg(a.col_rref + o);
-    if (final_step && kb == 0) bwz1 = __ldg(a.bw + o);
-  }
-  TerrainCol c0 = load_col(own0, gj0, kb), c1 = load_col(own1, gj1, kb);
-  wait_plane(kg, kb);
-  derive_p(kg);
-  if (kb > 0) {  // the chunk's lowest Z face, from the plane below
+  {
+    float pm[ROWS] = {0.f, 0.f}, zm[ROWS] = {0.f, 0.f};
+    if (kb > 0) {
+      wait_plane(kg, kb);
+      load_level(kg, pm, zm);
+    }
     wait_plane(kb, kb);
-    derive_p(kb);
-    const float* s0 = slot_of(kg);
-    const float* s1 = slot_of(kb);
-    auto face = [&](bool own, int row, int gj, float pru, float rru) {
-      if (!own) return 0.f;
-      const int o = gidx(g, gi, gj, kg), q = O_RHO + (row + R0) * RW + tx + C0;
-      return fp::wmom(FIRST ? 0.f : s0[O_DW + row * OBW + tx], Pv(kb, row + 1, tx + 1), pru, Pv(kg, row + 1, tx + 1),
-                      __ldg(a.col_pref + o), s0[q], __ldg(a.col_rref + o), s1[q], rru, __ldg(a.idz_f + o + g.plane),
-                      a.gravity, dtf);
-    };
-    dwc0 = face(own0, ty, gj0, prc0, rrc0);
-    dwc1 = face(own1, ty + RY, gj1, prc1, rrc1);
+    load_level(kb, p0, z0);
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      rc[r] = rho_at(kb, r);
+      pa[r] = fp::sub(p0[r], prk[r]);
+      ra[r] = fp::sub(rc[r], rrk[r]);
+      if (kb > 0 && own_rt[r]) {  // the chunk's lowest Z face, from the plane below
+        const int o = off[r] - g.plane;
+        const float dw = FIRST ? 0.f : slot_of(kg)[O_DW + (r0 + r) * OBW + tx];
+        dwc[r] = fp::wmom_pert(dw, pa[r], fp::sub(pm[r], __ldg(a.col_pref + o)),
+                               fp::sub(rho_at(kg, r), __ldg(a.col_rref + o)), ra[r], __ldg(a.idz_f + off[r]), gravity,
+                               dtf);
+      }
+      p1[r] = z1[r] = 0.f;
+    }
+    if (kb + 1 <= kl) {
+      wait_plane(kb + 1, kb);
+      load_level(kb + 1, p1, z1);
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+      dz0[r] = column_dpdz(kb, nz, pm[r], p0[r], p1[r], zm[r], z0[r], z1[r]);
+      if (own_rt[r]) S.dz[kb & 1][r0 + r + 1][tx + 1] = dz0[r];
+    }
+    role_dz(kb);
   }
-  if (kb + 1 <= kl) {
-    wait_plane(kb + 1, kb);
-    derive_p(kb + 1);
-  }
-  derive_dz(kb);
   __syncthreads();
 
   // Interior tiles (full, away from every periodic edge ring and open side) run a copy
   // of the plane loop compiled without the edge logic; both copies do the same arithmetic.
-  const bool interior = !edge && (g.per_x || (i0 > 0 && i0 + TX < nx)) && (g.per_y || (j0 > 0 && j0 + TY < ny));
+  const bool interior = !edge && i0 + TX <= nx && j0 + TY <= ny && (g.per_x || (i0 > 0 && i0 + TX < nx)) &&
+                        (g.per_y || (j0 > 0 && j0 + TY < ny));
   auto plane_loop = [&](auto tile_class) -> bool {  // true when a bounded wait gave up
     constexpr bool IN = decltype(tile_class)::value;
-    const bool o0 = IN || own0, o1 = IN || own1;
-    const bool su = !IN && skip_u, sv = !IN && skip_v0, hs = !IN && h_skip;
-    auto put = [&](float* f, const Geom& gg, int o, int i, int j, int kk, float v) {
-      if (IN) f[gidx(gg, i, j, kk)] = v;
-      else store_tile(f, gg, o, i, j, kk, v, edge);
+    const bool su = !IN && !g.per_x && gi == 0, hs = !IN && h_skip;  // faces of open sides never change
+    bool sv[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) sv[r] = !IN && !g.per_y && (gj + r == 0 || gj + r == ny);
+    // store at plane k + up of the thread's row r
+    auto put = [&](float* f, int o, int r, int k, int up, float v) {
+      if (IN) f[off[r] + up * g.plane] = v;
+      else store_tile(f, g, o, gi, gj + r, k + up, v, edge);
     };
     for (int k = kb; k < ke; ++k) {
       const int pb = k & 1;
       const float* st = slot_of(k);
-      const float* stn = slot_of(k + 1);
-      const TerrainCol n0 = load_col(o0, gj0, k + 1), n1 = load_col(o1, gj1, k + 1);
+      const bool up = k + 1 < nz;
+      TerrainCol ncol[ROWS];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) ncol[r] = load_col(r, k + 1, 1);
       // ---- dp/dz of plane k+1 (plane k+2 arrives first)
+      float p2[ROWS] = {0.f, 0.f}, z2[ROWS] = {0.f, 0.f}, dz1[ROWS] = {0.f, 0.f};
       if (k + 2 <= kl) {
         wait_plane(k + 2, k);
-        derive_p(k + 2);
+        load_level(k + 2, p2, z2);
       }
-      if (k + 1 < ke) derive_dz(k + 1);
-      // ---- faces of plane k: K12/K13 horizontal momenta, K14 vertical momentum at face k+1
-      auto P0 = [&](int r, int c) { return Pv(k, r, c); };
-      auto Z0 = [&](int r, int c) { return st[O_Z + r * CBW + c + 3]; };
-      auto D0 = [&](int r, int c) { return S.dz[pb][r][c]; };
-      float du0 = 0.f, dv0 = 0.f, du1 = 0.f, dv1 = 0.f, dw0 = 0.f, dw1 = 0.f;
-      if (!FIRST) {
-        du0 = st[O_DU + ty * FBW + tx];
-        dv0 = st[O_DV + ty * FBW + tx];
-        du1 = st[O_DU + (ty + RY) * FBW + tx];
-        dv1 = st[O_DV + (ty + RY) * FBW + tx];
-        if (k + 1 < nz) { dw0 = st[O_DW + ty * OBW + tx]; dw1 = st[O_DW + (ty + RY) * OBW + tx]; }
-      }
-      const int r0 = ty + 1, r1 = ty + RY + 1, cc = tx + 1;
-      const float pc0 = P0(r0, cc), pc1 = P0(r1, cc);
-      float un0 = du0, vn0 = dv0, un1 = du1, vn1 = dv1;
-      if (hm) {
-        if (!su) {
-          un0 = fp::hmom_terrain(du0, pc0, P0(r0, cc - 1), Z0(r0, cc), Z0(r0, cc - 1), D0(r0, cc - 1), D0(r0, cc), idx,
-                                 dtf);
-          un1 = fp::hmom_terrain(du1, pc1, P0(r1, cc - 1), Z0(r1, cc), Z0(r1, cc - 1), D0(r1, cc - 1), D0(r1, cc), idx,
-                                 dtf);
+      if (k + 1 < ke) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          dz1[r] = column_dpdz(k + 1, nz, p0[r], p1[r], p2[r], z0[r], z1[r], z2[r]);
+          if (IN || own_rt[r]) S.dz[pb ^ 1][r0 + r + 1][tx + 1] = dz1[r];
         }
-        if (!sv)
-          vn0 = fp::hmom_terrain(dv0, pc0, P0(r0 - 1, cc), Z0(r0, cc), Z0(r0 - 1, cc), D0(r0 - 1, cc), D0(r0, cc), idy,
-                                 dtf);
-        vn1 = fp::hmom_terrain(dv1, pc1, P0(r1 - 1, cc), Z0(r1, cc), Z0(r1 - 1, cc), D0(r1 - 1, cc), D0(r1, cc), idy,
-                               dtf);
+        role_dz(k + 1);
       }
-      if (o0) { S.du[pb][ty][tx] = un0; S.dv[pb][ty][tx] = vn0; }
-      if (o1) { S.du[pb][ty + RY][tx] = un1; S.dv[pb][ty + RY][tx] = vn1; }
+      // ---- faces of plane k: K12/K13 horizontal momenta, K14 vertical momentum at face k+1
+      float un[ROWS], vn[ROWS], wn[ROWS], rn[ROWS], pu[ROWS], ru[ROWS];
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int row = r0 + r + 1;
+        const float du = FIRST ? 0.f : st[O_DU + (r0 + r) * FBW + tx];
+        const float dv = FIRST ? 0.f : st[O_DV + (r0 + r) * FBW + tx];
+        un[r] = su ? du
+                   : fp::hmom_terrain(du, p0[r], Pv(k, row, tx), z0[r], Zv(k, row, tx), S.dz[pb][row][tx], dz0[r], idx,
+                                      dtf);
+        if (r == 0)
+          vn[r] = sv[r] ? dv
+                        : fp::hmom_terrain(dv, p0[r], Pv(k, row - 1, tx + 1), z0[r], Zv(k, row - 1, tx + 1),
+                                           S.dz[pb][row - 1][tx + 1], dz0[r], idy, dtf);
+        else
+          vn[r] = sv[r] ? dv
+                        : fp::hmom_terrain(dv, p0[r], p0[r > 0 ? r - 1 : 0], z0[r], z0[r > 0 ? r - 1 : 0],
+                                           dz0[r > 0 ? r - 1 : 0], dz0[r], idy, dtf);
+        if (IN || own_rt[r]) S.du[pb][r0 + r][tx] = un[r];
+      }
+      if (IN || own_rt[0]) S.dv[pb][ty][tx] = vn[0];
       if (role == 1) {  // the tile's east X face
         float d = FIRST ? 0.f : st[O_DU + (hr - 1) * FBW + w];
-        if (hm && !hs)
-          d = fp::hmom_terrain(d, P0(hr, hc), P0(hr, hc - 1), Z0(hr, hc), Z0(hr, hc - 1), D0(hr, hc - 1), D0(hr, hc),
-                               idx, dtf);
+        if (!hs)
+          d = fp::hmom_terrain(d, Pv(k, hr, hc), Pv(k, hr, hc - 1), Zv(k, hr, hc), Zv(k, hr, hc - 1),
+                               S.dz[pb][hr][hc - 1], S.dz[pb][hr][hc], idx, dtf);
         S.du[pb][hr - 1][w] = d;
         // open east boundary: face nx belongs to no tile; its step value is base + increment
-        if (final_step && hs) {
+        if (FINAL && hs) {
           const int o = gidx(g, hi, hj, k);
           a.f_u[o] = fp::add(__ldg(a.bu + o), d);
         }
       } else if (role == 3) {  // the tile's north Y face
         float d = FIRST ? 0.f : st[O_DV + h * FBW + hc - 1];
-        if (hm && !hs)
-          d = fp::hmom_terrain(d, P0(hr, hc), P0(hr - 1, hc), Z0(hr, hc), Z0(hr - 1, hc), D0(hr - 1, hc), D0(hr, hc),
-                               idy, dtf);
-        S.dv[pb][h][hc - 1] = d;
-        if (final_step && hs) {
+        if (!hs)
+          d = fp::hmom_terrain(d, Pv(k, hr, hc), Pv(k, hr - 1, hc), Zv(k, hr, hc), Zv(k, hr - 1, hc),
+                               S.dz[pb][hr - 1][hc], S.dz[pb][hr][hc], idy, dtf);
+        if (IN || h % ROWS == 0) S.dv[pb][h / ROWS][hc - 1] = d;  // else a thread's own second face
+        if (FINAL && hs) {
           const int o = gidx(g, hi, hj, k);
           a.f_v[o] = fp::add(__ldg(a.bv + o), d);
         }
       }
-      const float rc0 = st[O_RHO + (ty + R0) * RW + tx + C0], rc1 = st[O_RHO + (ty + RY + R0) * RW + tx + C0];
-      float wn0 = dw0, wn1 = dw1;
-      if (k + 1 < nz) {
-        const float pn0 = Pv(k + 1, r0, cc), pn1 = Pv(k + 1, r1, cc);
-        const float rn0 = stn[O_RHO + (ty + R0) * RW + tx + C0], rn1 = stn[O_RHO + (ty + RY + R0) * RW + tx + C0];
-        wn0 = fp::wmom(dw0, pn0, c0.pref, pc0, prc0, rc0, rrc0, rn0, c0.rref, c0.idzf, a.gravity, dtf);
-        wn1 = fp::wmom(dw1, pn1, c1.pref, pc1, prc1, rc1, rrc1, rn1, c1.rref, c1.idzf, a.gravity, dtf);
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        wn[r] = rn[r] = pu[r] = ru[r] = 0.f;  // face nz never changes
+        if (up) {
+          const float dw = FIRST ? 0.f : st[O_DW + (r0 + r) * OBW + tx];
+          rn[r] = rho_at(k + 1, r);
+          pu[r] = fp::sub(p1[r], col[r].pref);
+          ru[r] = fp::sub(rn[r], col[r].rref);
+          wn[r] = fp::wmom_pert(dw, pu[r], pa[r], ra[r], ru[r], col[r].idzf, gravity, dtf);
+        }
       }
       __syncthreads();  // publishes dz(k+1), p(k+2), du(k), dv(k); the slot of plane k-1 is free
       if (S.abort[pb]) return true;
       if (tid == ISSUER) {
-        if (acc_mode && k > kb) {  // level sums of plane k-1 (warp totals published above)
+        if (acc && k > kb) {  // level sums of plane k-1 (warp totals published above)
           long long sa = 0;
-          for (int q = 0; q < NW; ++q) sa += S.red[pb ^ 1][q][0];
+          for (int q = 0; q < NW; ++q) sa += S.red[pb ^ 1][q];
           acc_add(a.acc_a + k - 1, sa);
         }
         if (k + AHEAD <= kl) { issue(k + AHEAD); issued = k + AHEAD; }
       }
       // ---- K15 density of plane k, K10 rho*theta, stores
-      FxAcc sa;
-      auto cell = [&](bool o, int row, int gj, float rc, float un, float vn, float wn, float dwc, const TerrainCol& cl,
-                      float bwz) {
-        if (!o) return;
-        float rn = rc;
-        if (dn) rn = fp::density(rc, S.du[pb][row][tx + 1], un, S.dv[pb][row + 1][tx], vn, wn, dwc, idx, idy, cl.idzc, dtf);
-        const float rt = fp::mul(rn, st[O_TH + (row + R0) * RW + tx + C0]);
-        if (final_step) {
-          put(a.f_rho, g, kCell, gi, gj, k, rn);
-          put(a.f_rt, g, kCell, gi, gj, k, rt);
-          put(a.f_u, g, kFaceX, gi, gj, k, fp::add(cl.bu, un));
-          put(a.f_v, g, kFaceY, gi, gj, k, fp::add(cl.bv, vn));
-          if (k == 0) put(a.f_w, g, kFaceZ, gi, gj, 0, bwz);
-          put(a.f_w, g, kFaceZ, gi, gj, k + 1, fp::add(cl.bw, wn));
+      long long sum = 0;
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        if (!(IN || own_rt[r])) continue;
+        const float ue = S.du[pb][r0 + r][tx + 1], vnorth = r + 1 < ROWS ? vn[r + 1 < ROWS ? r + 1 : r] : S.dv[pb][ty + 1][tx];
+        const float rnew = fp::density(rc[r], ue, un[r], vnorth, vn[r], wn[r], dwc[r], idx, idy, col[r].idzc, dtf);
+        const float rt = fp::mul(rnew, st[O_TH + (r0 + r + R0) * RW + tx + C0]);
+        if (FINAL) {
+          put(a.f_rho, kCell, r, k, 0, rnew);
+          put(a.f_rt, kCell, r, k, 0, rt);
+          put(a.f_u, kFaceX, r, k, 0, fp::add(col[r].bu, un[r]));
+          put(a.f_v, kFaceY, r, k, 0, fp::add(col[r].bv, vn[r]));
+          if (k == 0) put(a.f_w, kFaceZ, r, 0, 0, bwz[r]);
+          put(a.f_w, kFaceZ, r, k, 1, fp::add(col[r].bw, wn[r]));
         } else {
-          put(a.rho_out, g, kCell, gi, gj, k, rn);
-          put(a.du_out, g, kFaceX, gi, gj, k, un);
-          put(a.dv_out, g, kFaceY, gi, gj, k, vn);
-          if (k + 1 < nz) put(a.dw_out, g, kFaceZ, gi, gj, k + 1, wn);
+          put(a.rho_out, kCell, r, k, 0, rnew);
+          put(a.du_out, kFaceX, r, k, 0, un[r]);
+          put(a.dv_out, kFaceY, r, k, 0, vn[r]);
+          if (up) put(a.dw_out, kFaceZ, r, k, 1, wn[r]);
           // the next substep's pressure, loaded with its ring
-          if (a.final_kind == 0) put(a.p_out, g, kCell, gi, gj, k, eos_pressure(rn, rt));
+          if (KIND == 0) put(a.p_out, kCell, r, k, 0, eos_pressure(rnew, rt));
         }
-        if (acc_mode == 2) sa.add(fp::theta(rn, rt), kFxTheta);
-      };
-      cell(o0, ty, gj0, rc0, un0, vn0, wn0, dwc0, c0, bwz0);
-      cell(o1, ty + RY, gj1, rc1, un1, vn1, wn1, dwc1, c1, bwz1);
-      if (acc_mode) {
-        const long long ta = sa.warp_total();
-        if (tx == 0) S.red[pb][ty][0] = ta;
+        if (acc) sum += fx(fp::theta(rnew, rt), kFxTheta);
       }
-      dwc0 = wn0;
-      dwc1 = wn1;
-      prc0 = c0.pref; rrc0 = c0.rref;
-      prc1 = c1.pref; rrc1 = c1.rref;
-      c0 = n0;
-      c1 = n1;
+      if (acc) {
+        const long long t = warp_total_fx(sum);
+        if (tx == 0) S.red[pb][ty] = t;
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        dwc[r] = wn[r];
+        rc[r] = rn[r];
+        pa[r] = pu[r];
+        ra[r] = ru[r];
+        p0[r] = p1[r];
+        z0[r] = z1[r];
+        p1[r] = p2[r];
+        z1[r] = z2[r];
+        dz0[r] = dz1[r];
+        col[r] = ncol[r];
+        off[r] += g.plane;
+      }
     }
     return false;
   };
@@ -408,38 +440,52 @@ __global__ void __launch_bounds__(fz::NT, 2)
       for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&S.bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1);
     return;
   }
-  if (acc_mode) {
+  if (acc) {
     __syncthreads();  // the last plane's warp totals
     if (tid == ISSUER) {
       const int pb = (ke - 1) & 1;
       long long sa = 0;
-      for (int q = 0; q < NW; ++q) sa += S.red[pb][q][0];
+      for (int q = 0; q < NW; ++q) sa += S.red[pb][q];
       acc_add(a.acc_a + ke - 1, sa);
     }
   }
 }
 
+template <bool FIRST, int KIND>
+cudaError_t allow_smem() {
+  return cudaFuncSetAttribute(k_fast_terrain_tma<FIRST, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)fz::dyn_smem<FIRST>());
+}
+
+template <bool FIRST>
+void launch(const FastArgs& a, const FastTerrainMaps& m, dim3 grid, const ZSplit& zs, cudaStream_t s) {
+  const dim3 block(fz::TX, fz::NW);
+  if (a.final_kind == 0) k_fast_terrain_tma<FIRST, 0><<<grid, block, fz::dyn_smem<FIRST>(), s>>>(a, m, zs);
+  else if (a.final_kind == 1) k_fast_terrain_tma<FIRST, 1><<<grid, block, fz::dyn_smem<FIRST>(), s>>>(a, m, zs);
+  else k_fast_terrain_tma<FIRST, 2><<<grid, block, fz::dyn_smem<FIRST>(), s>>>(a, m, zs);
+}
+
 }  // namespace
 
 cudaError_t init_fast_terrain_tma() {
-  cudaError_t e = cudaFuncSetAttribute(k_fast_terrain_tma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)fz::dyn_smem<true>());
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_fast_terrain_tma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)fz::dyn_smem<false>());
+  cudaError_t e = allow_smem<true, 0>();
+  if (e == cudaSuccess) e = allow_smem<true, 1>();
+  if (e == cudaSuccess) e = allow_smem<true, 2>();
+  if (e == cudaSuccess) e = allow_smem<false, 0>();
+  if (e == cudaSuccess) e = allow_smem<false, 1>();
+  if (e == cudaSuccess) e = allow_smem<false, 2>();
   return e;
 }
 
 cudaError_t launch_fast_terrain_tma(const FastArgs& a, const FastTerrainMaps& m, bool first, cudaStream_t s) {
-  if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || !a.col_pref || !a.col_rref || !a.idz_c || !a.idz_f ||
-      (a.final_kind == 0 && !a.p_out) || (a.final_kind == 2 && (!a.bu || !a.bv || !a.bw)))
+  if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || !a.hmom || !a.dens || !a.col_pref || !a.col_rref || !a.idz_c ||
+      !a.idz_f || (a.final_kind == 0 && !a.p_out) || (a.final_kind == 2 && (!a.bu || !a.bv || !a.bw)))
     return cudaErrorInvalidValue;
-  const dim3 block(fz::TX, fz::RY);
   dim3 grid((a.g.nx + fz::TX - 1) / fz::TX, (a.g.ny + fz::TY - 1) / fz::TY);
   const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 2, 3.0f);
   grid.z = zs.chunks;
-  if (first) k_fast_terrain_tma<true><<<grid, block, fz::dyn_smem<true>(), s>>>(a, m, zs);
-  else k_fast_terrain_tma<false><<<grid, block, fz::dyn_smem<false>(), s>>>(a, m, zs);
+  if (first) launch<true>(a, m, grid, zs, s);
+  else launch<false>(a, m, grid, zs, s);
   return cudaGetLastError();
 }
 
