@@ -13,7 +13,7 @@ SPLIT_MAIN = r"""
 #include <cstdio>
 int main() {
   const int tiles[] = {1, 2, 12, 77, 128, 288, 425, 512, 2048, 9000};
-  const float extra[] = {0.7f, 1.0f, 3.0f};
+  const float extra[] = {0.7f, 1.0f, 1.5f, 3.0f};
   for (int t : tiles)
     for (int nz = 1; nz <= 256; ++nz)
       for (int ctas = 2; ctas <= 4; ++ctas)
