@@ -138,7 +138,8 @@ struct gwm_b200_ctx {
   bool use_graph = false;
   cudaGraphExec_t graph = nullptr;
   long long graph_launches = 0;
-  int fast_tile_rows = 0;  // acoustic substep: 0 owned-tile flat kernel, 8/16 overlapped tiles
+  // tiles without tensor maps; gwm_b200_create sets 3 (TMA-fed) where every member has them
+  int fast_tile_rows = 0;     // acoustic substep: 0 owned-tile flat kernel, 8/16 overlapped tiles
   int slow_tile_rows = 16;    // slow stage: overlapped tiles of 8 or 16 rows
   int tracer_tile_rows = 16;  // tracer stage: overlapped tiles of 8 or 16 rows
   long long launches = 0;
@@ -366,7 +367,13 @@ int alloc_member(gwm_b200_ctx* c, Member& M) {
                        3 * 4 * (kMaxNz + 1) * sizeof(float) + 3 * kMaxNz * sizeof(double) + 512 +
                        4 * (kMaxNz + 1) * sizeof(float) + 256 + 256;
   const size_t total = nfields * fbytes + extra;
-  CK(cudaMalloc(&M.block, total));
+  cudaError_t em = cudaMalloc(&M.block, total);
+  if (em == cudaErrorMemoryAllocation) {  // once more without the scratch kept between calls
+    cudaGetLastError();
+    trim_scalar_scratch();
+    em = cudaMalloc(&M.block, total);
+  }
+  CK(em);
   CK(cudaMemsetAsync(M.block, 0, total, c->stream));
   char* p = M.block;
   auto take = [&](size_t bytes) { char* r = p; p += ((bytes + 255) / 256) * 256; return r; };
@@ -1019,6 +1026,7 @@ void gwm_b200_destroy(gwm_b200_ctx* c) {
   for (auto ev : c->mjoin) cudaEventDestroy(ev);
   if (c->mfork) cudaEventDestroy(c->mfork);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
+  trim_scalar_scratch();
   delete c;
 }
 

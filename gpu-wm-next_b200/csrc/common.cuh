@@ -51,10 +51,6 @@ __device__ __forceinline__ float eos_pressure(float rho, float rt) {
   const float ratio = fmaxf(rho * kRd * th / kP0, 1.0e-6f);
   return kP0 * powf(ratio, 1.0f / (1.0f - kKappa));
 }
-__device__ __forceinline__ float eos_rho(float p, float th) {
-  const float ex = powf(fmaxf(p / kP0, 1.0e-6f), kKappa);
-  return p / fmaxf(kRd * th * ex, 1.0e-6f);
-}
 __device__ __forceinline__ float dry_cp() { return kRd / kKappa; }
 // One-sided / centred dp/dz of a column (terrain pressure gradient):
 // dry_pressure_gradient.cu:37-73.

@@ -21,6 +21,7 @@
 
 #include "../../include/gwm_b200.h"
 #include "common.cuh"
+#include "physics.cuh"
 #include "stencil.cuh"
 
 namespace gwmb {
@@ -107,17 +108,18 @@ __global__ void __launch_bounds__(32 * kSWarps) k_scalar_step(const ScalarStep a
 // Scratch of the calls, from a pool of the library per device that keeps up to 256 MB between
 // calls (larger scratch goes back to the device at the next synchronisation): the default
 // pool gives everything back at each call's end, and mapping it again cost more than the
-// steps.  Allocations are stream-ordered, so threads and streams share the pool safely.
+// steps.  Allocations are stream-ordered, so threads and streams share the pool safely.  What
+// is kept goes back when a context is destroyed or finds no room (trim_scalar_scratch).
 constexpr uint64_t kKeptScratch = 256ull << 20;
+std::mutex pools_lock;
+std::map<int, cudaMemPool_t> pools;
 cudaError_t scratch_alloc(float** p, size_t bytes, cudaStream_t s) {
-  static std::mutex lock;
-  static std::map<int, cudaMemPool_t> pools;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   cudaMemPool_t pool = nullptr;
   {
-    std::lock_guard<std::mutex> hold(lock);
+    std::lock_guard<std::mutex> hold(pools_lock);
     auto it = pools.find(dev);
     if (it == pools.end()) {
       cudaMemPoolProps props{};
@@ -138,13 +140,22 @@ cudaError_t scratch_alloc(float** p, size_t bytes, cudaStream_t s) {
     e = cudaMallocFromPoolAsync((void**)p, bytes, pool, s);
     if (e == cudaSuccess || e == cudaErrorMemoryAllocation) return e;
     cudaGetLastError();  // a pool of a context that is gone (cudaDeviceReset): forget it
-    std::lock_guard<std::mutex> hold(lock);
+    std::lock_guard<std::mutex> hold(pools_lock);
     pools.erase(dev);
   }
   return cudaMallocAsync((void**)p, bytes, s);
 }
 
 }  // namespace
+
+void trim_scalar_scratch() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::lock_guard<std::mutex> hold(pools_lock);
+  auto it = pools.find(dev);
+  if (it != pools.end() && cudaMemPoolTrimTo(it->second, 0) != cudaSuccess) cudaGetLastError();
+}
+
 }  // namespace gwmb
 
 extern "C" int gwm_b200_scalar_ssprk3(const gwm_b200_scalar_desc* d, float* q, int nsteps, void* stream) {

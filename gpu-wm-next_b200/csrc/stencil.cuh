@@ -164,7 +164,7 @@ __device__ __forceinline__ float add_buoyancy_ref(float t, float th_l, float th_
 // repeats, and the final density is then the one just evaluated, so the third iteration and
 // the fourth stop there with the same result (the iterations contract by about
 // g dz / (2 c^2) ~ 1e-2, so the first two are never the last).
-__device__ __forceinline__ float eos_rho_of(float p, float rdth) {  // eos_rho with Rd*theta at hand
+__device__ __forceinline__ float eos_rho_of(float p, float rdth) {  // density of p with Rd*theta at hand
   const float x = div_by(p, kP0, 1.0f / kP0);
   return p / fmaxf(rdth * powf(fmaxf(x, 1.0e-6f), kKappa), 1.0e-6f);
 }
