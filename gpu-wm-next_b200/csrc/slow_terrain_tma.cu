@@ -4,18 +4,22 @@
 // K21/K22 tendencies of compute_slow_tendencies, src/dycore/dry_core.cu:400-539, with
 // the terrain pressure gradient of dry_pressure_gradient.cu:37-240 and the hybrid-height
 // metric columns; the update K4 and blend K5 of :189-205), with the data path of
-// k_slow_tma: a CTA owns a 32 x 16 tile, two columns per thread, and one elected thread
+// k_slow_tma: a CTA owns a 32 x 16 tile, two adjacent rows per thread, and one elected thread
 // fetches each plane's boxes with cp.async.bulk.tensor.3d into a three-slot shared-memory
 // ring two planes ahead:
 //   rho, theta (or rho*theta), u, w, z (+ du, dw)   40 x 18 boxes: tile, halo ring, corners
 //   v (+ dv)                                        40 x 19 (one more Y-face row)
 // Plane nz carries only w (+ dw), the top faces.  Per plane the CTA derives, at all 34 x 18
 // positions of the tile and its ring, theta, the cell velocities uc, vc, wc, the full
-// pressure of the plane above (three pressure planes are kept) and dp/dz of the plane; one
-// barrier publishes them, every thread computes its cells and faces, and a second barrier
+// pressure and dp/dz of the plane (a position's pressures of three planes stay in its thread's
+// registers); one barrier publishes them, every thread computes its cells and faces, and a second barrier
 // frees the derived planes for the next one (the terrain planes would not fit a CTA pair
 // per SM double-buffered).  The owned columns' metric values (the cell and face inverse
 // layer depths) and the blend partner q0 are per-thread coalesced loads a plane ahead.
+// Bounds: issue and the two barriers of a plane, as in the flat stage, whose shared and carried
+// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.716 ms a stage against 0.998 with
+// separate rows, 201 x 163 x 40: 88 us against 119 (27 fields of 4 B per cell at the copy
+// bandwidth: 0.35 ms and 22 us).
 #include <type_traits>
 
 #include "dycore.cuh"
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(st::NT, 2)
 
   // ---- derived planes: the thread's positions of the 34 x 18 (a third one in the first
   // warps), their box indices and the reciprocal of their floored density
-  constexpr int NP = (DN + NT - 1) / NT;
+  constexpr int NP = (DN + NT - 1) / NT, FULL = DN / NT;  // FULL: positions every thread has
   int pos_b[NP];
   float yrho[NP], p_m[NP], p_c[NP];  // the reciprocal at plane k; the pressure at planes k-1 and k
   // positions whose theta (bit n) and whose p, dp/dz and velocities (bit 8 + n) are read: not
@@ -223,20 +227,21 @@ __global__ void __launch_bounds__(st::NT, 2)
   };
   // theta and pressure of plane kk (kk < nz), and the reciprocals that derive(kk) divides by:
   // the pressure becomes p_c, the one before it p_m
-  auto derive_theta = [&](int kk) {
+  auto derive_theta = [&](auto tile_class, int kk) {
+    constexpr bool IN = decltype(tile_class)::value;
     const float* sr = slot_at(kk);
     float* th = der + D_TH + (kk & 1) * DN;
     bool near = true;
 #pragma unroll
     for (int n = 0; n < NP; ++n) {
       p_m[n] = p_c[n];
-      if (live & (1u << n)) {
+      if ((IN && n < FULL) || live & (1u << n)) {
         const float rho = sr[R_RHO + pos_b[n]], rt = RT(sr, pos_b[n], rho), rr = fmaxf(rho, 1.0e-6f);
         yrho[n] = fp::recip(rr);
         const float t = fp::div_by(rt, rr, yrho[n]);
         near = near && fp::finite(t);
         th[tid + n * NT] = t;
-        if (live & (256u << n)) p_c[n] = pressure(rho, t, near);
+        if ((IN && n < FULL) || live & (256u << n)) p_c[n] = pressure(rho, t, near);
       }
     }
     if (!near) {  // a value that is not finite: the plain forms
@@ -251,7 +256,8 @@ __global__ void __launch_bounds__(st::NT, 2)
   };
   // uc, vc, wc, p and dp/dz of plane k, with derive_theta(k) done; does derive_theta(k + 1).  grad:
   // p and dp/dz are wanted (not for the plane below a chunk)
-  auto derive = [&](int k, bool grad) {
+  auto derive = [&](auto tile_class, int k, bool grad) {
+    constexpr bool IN = decltype(tile_class)::value;
     const float* sm = slot_at(k > kg ? k - 1 : kg);  // plane k-1 (its slot is intact)
     const float* sr = slot_at(k);
     const float* sn = slot_at(k + 1);
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(st::NT, 2)
     };
 #pragma unroll
     for (int n = 0; n < NP; ++n)
-      if (live & (256u << n)) {
+      if ((IN && n < FULL) || live & (256u << n)) {
         const int b = pos_b[n], q = tid + n * NT;
         // cell-centred velocities: dry_momentum_flux.cu:36-73
         const float rr = fmaxf(sr[R_RHO + b], 1.0e-6f), y = yrho[n];
@@ -297,7 +303,7 @@ __global__ void __launch_bounds__(st::NT, 2)
 #pragma unroll
     for (int n = 0; n < NP; ++n) below[n] = p_m[n];
     if (k + 1 < nz) {  // p_m, p_c become the pressures at planes k and k+1
-      derive_theta(k + 1);
+      derive_theta(tile_class, k + 1);
     } else {
 #pragma unroll
       for (int n = 0; n < NP; ++n) {
@@ -308,7 +314,7 @@ __global__ void __launch_bounds__(st::NT, 2)
     if (!grad) return;
 #pragma unroll
     for (int n = 0; n < NP; ++n)
-      if (live & (256u << n)) {
+      if ((IN && n < FULL) || live & (256u << n)) {
         const int b = pos_b[n], q = tid + n * NT;
         pp[q] = p_m[n];
         dz[q] = column_dpdz(k, nz, below[n], p_m[n], p_c[n], k > 0 ? sm[R_Z + b] : 0.f, sr[R_Z + b],
@@ -335,11 +341,11 @@ __global__ void __launch_bounds__(st::NT, 2)
 #pragma unroll
   for (int n = 0; n < NP; ++n) p_c[n] = 0.f;
   wait_plane(kg, kb);
-  derive_theta(kg);
+  derive_theta(std::false_type{}, kg);
   load_column(kg);
   if (kb > 0) {  // the plane below the chunk: its derived values and the fluxes out of its top
     wait_plane(kb, kb);
-    derive(kg, false);
+    derive(std::false_type{}, kg, false);
     __syncthreads();
     const float* wc = der + D_WC;
     const float* tl = der + D_TH + (kg & 1) * DN;
@@ -588,7 +594,7 @@ __global__ void __launch_bounds__(st::NT, 2)
       TerrMetric mt[ROWS];
       load_metric(mt);
       wait_plane(k + 1, k);
-      derive(k, true);
+      derive(tile_class, k, true);
       __syncthreads();  // publishes plane k's derived values; slot (k-1) is free
       if (s_abort[pb]) return true;
       if (tid == ISSUER) {

@@ -3,7 +3,7 @@
 // Same operator and per-cell arithmetic as k_slow_stage<false, R>: the K2/K3/K16-K19/
 // K21/K22 tendencies of compute_slow_tendencies (src/dycore/dry_core.cu:400-539), the
 // stage update K4 (:189-197) and the SSPRK3 blend K5 (:199-205).  The data path is
-// different.  A CTA owns a 32 x 16 tile, two columns per thread, and one elected
+// different.  A CTA owns a 32 x 16 tile, two adjacent rows per thread, and one elected
 // thread fetches each plane's boxes with cp.async.bulk.tensor.3d into a three-slot
 // shared-memory ring two planes ahead:
 //   rho, theta (or rho*theta), u, w (+ du, dw)   40 x 18 boxes, columns i0-4..i0+35,
@@ -14,9 +14,21 @@
 // pressure perturbation and the cell velocities uc, vc, wc at all 34 x 18 positions
 // of the tile and its ring (corners included: the Y-face fluxes need uc there), then
 // one barrier publishes them and every thread computes its cells and faces.  uc, vc,
-// wc are triple-buffered (a face at plane k reads planes k-1 and k while the next
-// plane is derived), theta and p double-buffered, so one barrier per plane suffices.
-// The blend partner q0 is read per thread (owned positions only, coalesced).
+// theta are triple-buffered (a face at plane k reads planes k-1 and k while the next
+// plane is derived), wc and p double-buffered, so one barrier per plane suffices.
+// The blend partner q0 is read per thread (owned positions only, coalesced) at the top of
+// its plane, so the derive phase covers the loads.
+//
+// What bounds it: instruction issue and the wait between a plane's derive phase and its faces
+// (58 % of the issue slots used with 16 warps per SM, which the registers allow), not HBM: up
+// to 19 fields of 4 B per cell, 0.78 ms for 1024 x 1024 x 64 at the copy bandwidth.  So the
+// work per cell was cut: adjacent rows share the Y flux between them, the flux out of a
+// plane's top is carried as the next plane's bottom flux, the divisions of a derived position
+// take one reciprocal and residual steps (fp::div_by) with one test per plane for the forms
+// they do not cover, and positions nothing reads are skipped; interior tiles derive without a
+// test per position, so two positions' chains interleave (1.65 -> 1.57 ms).  1024 x 1024 x 64:
+// 1.57 ms a stage, 2.27 with separate rows and a division each; 128 x 128 x 64 with its columns split
+// over CTAs 64 us, 389 with whole columns; 32 x 32 x 40 16 us, 260 with whole columns.
 #include <type_traits>
 
 #include "dycore.cuh"
@@ -182,7 +194,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     for (int kk = kg; kk <= kb + 1; ++kk) { issue(kk); issued = kk; }
   // ---- derived planes: the thread's positions of the 34 x 18 (a third one in the first
   // warps), their box indices and the reciprocal of their floored density
-  constexpr int NP = (DN + NT - 1) / NT;
+  constexpr int NP = (DN + NT - 1) / NT, FULL = DN / NT;  // FULL: positions every thread has
   int pos_b[NP];
   float yrho[NP];
   // positions whose theta (bit n) and whose p' and velocities (bit 8 + n) are read: not those of
@@ -200,13 +212,14 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     }
   }
   // theta of plane kk (kk < nz), and the reciprocals that derive(kk) divides by
-  auto derive_theta = [&](int kk) {
+  auto derive_theta = [&](auto tile_class, int kk) {
+    constexpr bool IN = decltype(tile_class)::value;
     const float* sr = slot_at(kk);
     float* th = der + D_TH + (kk % 3) * DN;
     bool near = true;
 #pragma unroll
     for (int n = 0; n < NP; ++n)
-      if (live & (1u << n)) {
+      if ((IN && n < FULL) || live & (1u << n)) {
         const float rho = sr[R_RHO + pos_b[n]], rt = RT(sr, pos_b[n], rho), rr = fmaxf(rho, 1.0e-6f);
         yrho[n] = fp::recip(rr);
         const float t = fp::div_by(rt, rr, yrho[n]);
@@ -223,7 +236,8 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     }
   };
   // p', uc, vc, wc of plane k (after derive_theta(k))
-  auto derive = [&](int k) {
+  auto derive = [&](auto tile_class, int k) {
+    constexpr bool IN = decltype(tile_class)::value;
     const float* sr = slot_at(k);
     const float* sn = slot_at(k + 1);
     float* uc = der + D_UC + (k % 3) * DN;
@@ -239,7 +253,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     };
 #pragma unroll
     for (int n = 0; n < NP; ++n)
-      if (live & (256u << n)) {
+      if ((IN && n < FULL) || live & (256u << n)) {
         const int b = pos_b[n], q = tid + n * NT;
         const float rho = sr[R_RHO + b];
         pp[q] = eos_pprime_near(rho, RT(sr, b, rho), binv, bpr, near);
@@ -286,12 +300,12 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     }
   };
   wait_plane(kg, kb);
-  derive_theta(kg);
+  derive_theta(std::false_type{}, kg);
   load_column(kg);
   if (kb > 0) {  // the plane below the chunk: its derived values and the fluxes out of its top
     wait_plane(kb, kb);
-    derive(kg);
-    derive_theta(kb);
+    derive(std::false_type{}, kg);
+    derive_theta(std::false_type{}, kb);
     __syncthreads();
     const float* wc = der + D_WC + (kg & 1) * DN;
     const float* tl = der + D_TH + (kg % 3) * DN;
@@ -558,8 +572,8 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(r);
       wait_plane(k + 1, k);
-      derive(k);
-      if (k + 1 < nz) derive_theta(k + 1);
+      derive(tile_class, k);
+      if (k + 1 < nz) derive_theta(tile_class, k + 1);
       __syncthreads();  // publishes plane k's derived values; slot (k-1) is free
       if (s_abort[pb]) return true;
       if (tid == ISSUER) {
