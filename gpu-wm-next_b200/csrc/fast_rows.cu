@@ -14,7 +14,9 @@
 //   - an extra warp issues the TMA loads: a plane's slot has a full barrier (the loads'
 //     transaction count) and an empty one (an arrival per consumer warp);
 //   - p' - p'_ref and rho - rho_ref of a level are formed once and carried up;
-//   - the level sums stay in shared memory until the CTA's end: one atomic per level;
+//   - the level sums stay in shared memory until the CTA's end: one atomic per level.
+// 1024 x 1024 x 64: 0.549 ms a substep (0.82 of the copy bandwidth), 0.627 with k_fast_tma's
+// split columns, 0.654 with its whole columns; 517 x 389 x 50: 99 us, 116 with either.
 #include <type_traits>
 
 #include "dycore.cuh"

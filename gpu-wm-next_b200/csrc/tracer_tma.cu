@@ -13,8 +13,10 @@
 // A thread computes the mixing ratios of its rows one plane ahead and those of the rows around
 // them, lanes 0-7 those of the warp's two ring columns, with one reciprocal per position; the
 // Y fluxes between its rows are computed once, and the flux out of a plane's top is carried as
-// the next plane's bottom flux.  The kernel is issue-bound: 426 instructions per cell with one
-// row per eight and a block barrier per plane.
+// the next plane's bottom flux.  The kernel is issue-bound (69 % of the issue slots; 13 fields
+// of 4 B per cell would take 0.53 ms for 1024 x 1024 x 64, three tracers, at the copy
+// bandwidth): there 0.766 ms a stage, 1.045 with two rows eight apart per thread, 426
+// instructions per cell and a block barrier per plane; 517 x 389 x 50 0.141 ms against 0.184.
 #include <type_traits>
 
 #include "physics.cuh"

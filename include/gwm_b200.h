@@ -359,13 +359,16 @@ int gwm_b200_plan_view_field(int field, const char** name, const char** units);
  * gwm_b200_runtime_summary_json. */
 int gwm_b200_plan_view_json(gwm_b200_ctx* ctx, int member, int level, const char* case_kind, int steps, double dt,
                             char* buf, long long cap, long long* len);
-/* Tile shape of a kernel.  kernel 0 = slow stage: rows 3 = owned 32x16 tiles fed by
+/* Tile shape of a kernel.  The default is 3 for every kernel where each member's buffers
+ * have TMA descriptors (the driver can encode them); else 16, and 0 for the
+ * acoustic substep.  kernel 0 = slow stage: rows 3 = owned 32x16 tiles fed by
  * TMA tile loads (flat terrain and terrain; the stand-alone slow tendencies use 16),
- * 8 or 16 = overlapped 32-wide tiles (default 16).  kernel 2 = tracer stage: rows 3 =
- * owned 32x16 tiles fed by TMA (flat terrain and terrain), 8 or 16 (overlapped,
- * default 16).  kernel 1 = acoustic substep: rows 0 = owned 32x16 tiles
+ * 8 or 16 = overlapped 32-wide tiles.  kernel 2 = tracer stage: rows 3 =
+ * owned 32x16 tiles fed by TMA (flat terrain and terrain), 8 or 16 (overlapped).
+ * kernel 1 = acoustic substep: rows 0 = owned 32x16 tiles
  * (flat terrain; terrain falls back to 8), 3 = owned 32x16 tiles fed by TMA tile loads
- * (flat terrain and terrain), 4 = the same tiles with all the substeps of an RK stage in
+ * (flat terrain and terrain; on terrain without its momentum or density update, overlapped
+ * tiles of 8 rows), 4 = the same tiles with all the substeps of an RK stage in
  * one persistent cooperative launch (a bounded grid barrier between substeps; the
  * step's last substep keeps its own launch; terrain runs one launch per substep), 8 or
  * 16 = overlapped 32-wide tiles of that many rows.  The environment variable GWM_B200_FAST_TILE_ROWS sets the
@@ -432,8 +435,9 @@ typedef struct {
 /* nsteps of advance_scalar_ssprk3 (include/gwm/dycore/dry_transport.hpp:19-21,
  * src/dycore/dry_transport.cu:285-325) on q, a device array (nz, ny, nx) in the global
  * owned layout, in place; the arithmetic is the reference's, so results match it bit
- * for bit.  Two scratch copies of q are taken from the stream-ordered allocator for the
- * call.  stream: cudaStream_t as void* (NULL: the default stream); returns when done. */
+ * for bit.  One scratch copy of q is taken for the call from a stream-ordered pool of the
+ * library, which keeps up to 256 MB between calls and gives it back when a context is
+ * destroyed or finds no room.  stream: cudaStream_t as void* (NULL: the default stream); returns when done. */
 int gwm_b200_scalar_ssprk3(const gwm_b200_scalar_desc* desc, float* q, int nsteps, void* stream);
 
 /* ---- host layout helpers (no device work) --------------------------------- */
