@@ -17,8 +17,8 @@
 // per SM double-buffered).  The owned columns' metric values (the cell and face inverse
 // layer depths) and the blend partner q0 are per-thread coalesced loads a plane ahead.
 // Bounds: issue and the two barriers of a plane, as in the flat stage, whose shared and carried
-// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.716 ms a stage against 0.998 with
-// separate rows, 201 x 163 x 40: 88 us against 119 (27 fields of 4 B per cell at the copy
+// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.699 ms a stage against 0.998 with
+// separate rows, 201 x 163 x 40: 85 us against 119 (27 fields of 4 B per cell at the copy
 // bandwidth: 0.35 ms and 22 us).
 #include <type_traits>
 
@@ -68,7 +68,7 @@ struct TerrMetric {
 
 // FIRST: a step's first stage (rho*theta in, no blend); INC: acoustic increments are added to
 // the momenta (stages 2 and 3 behind the fast modes).
-template <bool FIRST, bool INC>
+template <bool FIRST, bool INC, bool DAMP>  // DAMP: with the Rayleigh layer
 __global__ void __launch_bounds__(st::NT, 2)
     k_slow_terrain_tma(const SlowArgs a, const __grid_constant__ SlowMaps m, ZSplit zs) {
   using namespace st;
@@ -173,9 +173,10 @@ __global__ void __launch_bounds__(st::NT, 2)
     own_rt[r] = tx < w && r0 + r < h;
   }
   // blend partner at the current plane of the thread's row r
-  auto load_q0 = [&](int r) {
+  auto load_q0 = [&](auto tile_class, int r) {
+    constexpr bool IN = decltype(tile_class)::value;
     SlowBlend q{0.f, 0.f, 0.f, 0.f, 0.f};
-    if (!BLEND || !own_rt[r]) return q;
+    if (!BLEND || !(IN || own_rt[r])) return q;
     const int o = off[r];
     q.rho = __ldg(a.rho0 + o);
     q.rt = __ldg(a.rt0 + o);
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(st::NT, 2)
   };
   auto plane_const = [&](int k) {
     PlaneConst pc{0.0f, 0.0f, 0.0f, 0.0f};
-    if (a.damp_c) {
+    if (DAMP) {
       pc.damp_c = __ldg(a.damp_c + k);
       pc.damp_f = __ldg(a.damp_f + k);
       pc.uref = __ldg(a.uref + k);
@@ -423,17 +424,10 @@ __global__ void __launch_bounds__(st::NT, 2)
     for (int r = 0; r < ROWS; ++r) {
       const int b = b0 + r * BW;
       w_n[r] = W(sn, b);
-      if (!top) {
-        rho_n[r] = sn[R_RHO + b];
-        u_n[r] = U(sn, b);
-        v_n[r] = V(sn, b);
-        tt[r] = thn[d0 + r * DW];
-      } else {
-        rho_n[r] = 0.f;
-        u_n[r] = u_c[r];
-        v_n[r] = v_c[r];
-        tt[r] = tc[r + 1];
-      }
+      rho_n[r] = sn[R_RHO + b];  // the top plane reads none of these
+      u_n[r] = U(sn, b);
+      v_n[r] = V(sn, b);
+      tt[r] = top ? tc[r + 1] : thn[d0 + r * DW];
     }
     const float u_s = U(sr, b0 - BW), u_t = U(sr, b0 + ROWS * BW);  // rows -1 and ROWS
     const float v_s = V(sr, b0 - BW), v_t = V(sr, b0 + ROWS * BW);
@@ -494,7 +488,7 @@ __global__ void __launch_bounds__(st::NT, 2)
                                     fp::avg(mt[r].w, mt[r].c));
         fz_u[r] = flt;
         t_u = fp::add_pgf_terrain(t_u, pp[d], pp[d - 1], sr[R_Z + b], sr[R_Z + b - 1], dz[d - 1], dz[d], idx);
-        if (a.damp_c) t_u = fp::add_damping(t_u, kc.damp_c, qc, kc.uref);
+        if (DAMP) t_u = fp::add_damping(t_u, kc.damp_c, qc, kc.uref);
         if (sx0) t_u = 0.0f;
         float u1 = fp::update(qc, dt, t_u, -1.0e30f);
         if (BLEND) u1 = fp::blend(a.wa, q0[r].u, a.wb, u1);
@@ -520,7 +514,7 @@ __global__ void __launch_bounds__(st::NT, 2)
                                     fp::avg(mt[r].s, mt[r].c));
         fz_v[r] = flt;
         t_v = fp::add_pgf_terrain(t_v, pp[d], pp[d - DW], sr[R_Z + b], sr[R_Z + b - BW], dz[d - DW], dz[d], idy);
-        if (a.damp_c) t_v = fp::add_damping(t_v, kc.damp_c, qc, kc.vref);
+        if (DAMP) t_v = fp::add_damping(t_v, kc.damp_c, qc, kc.vref);
         if (!IN && gj + r == 0 && open_y) t_v = 0.0f;
         float v1 = fp::update(qc, dt, t_v, -1.0e30f);
         if (BLEND) v1 = fp::blend(a.wa, q0[r].v, a.wb, v1);
@@ -538,26 +532,42 @@ __global__ void __launch_bounds__(st::NT, 2)
           if (sy[r]) fy[r] = 0.0f;
         }
       }
+      float flt[ROWS], t_w[ROWS];
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
-        const int d = d0 + r * DW, b = b0 + r * BW;
-        const float qc = w_c[r];
-        const float flt = fp::upwind(wc[d], qc, w_n[r]);
-        float t_w = 0.0f;
-        if (k > 0) {
+        flt[r] = fp::upwind(wc[d0 + r * DW], w_c[r], w_n[r]);
+        t_w[r] = 0.0f;
+      }
+      if (k > 0) {
+        float flux[ROWS];
+        bool near = true;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const int d = d0 + r * DW, b = b0 + r * BW;
+          const float qc = w_c[r];
           float flw = fp::upwind(fp::avg(ucm[d - 1], uw[r + 1]), W(sr, b - 1), qc);
           float fle = fp::upwind(fp::avg(ucm[d], ue[r + 1]), qc, W(sr, b + 1));
           if (sx0) flw = 0.0f;
           if (sx1) fle = 0.0f;
-          t_w = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_w[r], idx, idy, mt[r].f);
-          bool near = true;
-          const float t = fp::add_buoyancy_ref(t_w, th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r],
-                                               a.gravity, near);
-          t_w = near ? t : fp::add_buoyancy(t_w, th_l[r], tc[r + 1], s_trf[k], rho_l[r], rho_c[r], a.gravity);
-          if (a.damp_c) t_w = fp::add_damping(t_w, kc.damp_f, qc, 0.0f);
+          flux[r] = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt[r], fz_w[r], idx, idy, mt[r].f);
+          t_w[r] = fp::add_buoyancy_ref(flux[r], th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r],
+                                        a.gravity, near);
         }
-        fz_w[r] = flt;
-        float w1 = fp::update(qc, dt, t_w, -1.0e30f);
+        if (!near) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r)
+            t_w[r] = fp::add_buoyancy(flux[r], th_l[r], tc[r + 1], s_trf[k], rho_l[r], rho_c[r], a.gravity);
+        }
+        if (DAMP) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) t_w[r] = fp::add_damping(t_w[r], kc.damp_f, w_c[r], 0.0f);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const float qc = w_c[r];
+        fz_w[r] = flt[r];
+        float w1 = fp::update(qc, dt, t_w[r], -1.0e30f);
         if (BLEND) w1 = fp::blend(a.wa, q0[r].w, a.wb, w1);
         put(a.o_w, kFaceZ, r, 0, w1);
         if (top) {  // top face: zero tendency
@@ -590,7 +600,7 @@ __global__ void __launch_bounds__(st::NT, 2)
       const PlaneConst kc = plane_const(k);
       SlowBlend q0[ROWS];  // the derive phase covers the loads
 #pragma unroll
-      for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(r);
+      for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(tile_class, r);
       TerrMetric mt[ROWS];
       load_metric(mt);
       wait_plane(k + 1, k);
@@ -648,8 +658,20 @@ __global__ void __launch_bounds__(st::NT, 2)
 
 template <bool FIRST, bool INC>
 cudaError_t allow_smem() {
-  return cudaFuncSetAttribute(k_slow_terrain_tma<FIRST, INC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)st::smem_bytes(INC));
+  cudaError_t e = cudaFuncSetAttribute(k_slow_terrain_tma<FIRST, INC, false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st::smem_bytes(INC));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_slow_terrain_tma<FIRST, INC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)st::smem_bytes(INC));
+  return e;
+}
+
+template <bool FIRST, bool INC>
+void launch(const SlowArgs& a, const SlowMaps& m, dim3 grid, const ZSplit& zs, cudaStream_t s) {
+  const dim3 block(st::TX, st::NW);
+  const size_t smem = st::smem_bytes(INC);
+  if (a.damp_c) k_slow_terrain_tma<FIRST, INC, true><<<grid, block, smem, s>>>(a, m, zs);
+  else k_slow_terrain_tma<FIRST, INC, false><<<grid, block, smem, s>>>(a, m, zs);
 }
 
 }  // namespace
@@ -667,13 +689,12 @@ cudaError_t launch_slow_terrain_tma(const SlowArgs& a, const SlowMaps& m, cudaSt
   if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || a.tend_only || a.acc_mode == 1 || !a.idz_c || !a.idz_f ||
       first != !a.rho0 || (first && a.du))
     return cudaErrorInvalidValue;
-  const dim3 block(st::TX, st::NW);
   dim3 grid((a.g.nx + st::TX - 1) / st::TX, (a.g.ny + st::TY - 1) / st::TY);
   const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 2, 1.2f);
   grid.z = zs.chunks;
-  if (first) k_slow_terrain_tma<true, false><<<grid, block, st::smem_bytes(false), s>>>(a, m, zs);
-  else if (a.du) k_slow_terrain_tma<false, true><<<grid, block, st::smem_bytes(true), s>>>(a, m, zs);
-  else k_slow_terrain_tma<false, false><<<grid, block, st::smem_bytes(false), s>>>(a, m, zs);
+  if (first) launch<true, false>(a, m, grid, zs, s);
+  else if (a.du) launch<false, true>(a, m, grid, zs, s);
+  else launch<false, false>(a, m, grid, zs, s);
   return cudaGetLastError();
 }
 

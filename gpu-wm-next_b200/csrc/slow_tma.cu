@@ -20,15 +20,16 @@
 // its plane, so the derive phase covers the loads.
 //
 // What bounds it: instruction issue and the wait between a plane's derive phase and its faces
-// (58 % of the issue slots used with 16 warps per SM, which the registers allow), not HBM: up
+// (about 60 % of the issue slots used with 16 warps per SM, which the registers allow), not HBM: up
 // to 19 fields of 4 B per cell, 0.78 ms for 1024 x 1024 x 64 at the copy bandwidth.  So the
 // work per cell was cut: adjacent rows share the Y flux between them, the flux out of a
 // plane's top is carried as the next plane's bottom flux, the divisions of a derived position
 // take one reciprocal and residual steps (fp::div_by) with one test per plane for the forms
 // they do not cover, and positions nothing reads are skipped; interior tiles derive without a
-// test per position, so two positions' chains interleave (1.65 -> 1.57 ms).  1024 x 1024 x 64:
-// 1.57 ms a stage, 2.27 with separate rows and a division each; 128 x 128 x 64 with its columns split
-// over CTAs 64 us, 389 with whole columns; 32 x 32 x 40 16 us, 260 with whole columns.
+// test per position, so two positions' chains interleave (1.65 -> 1.57 ms), and what a launch
+// decides (damping, the kind of level sums) is compiled in, so a plane is few blocks of code
+// (1.57 -> 1.49 ms).  1024 x 1024 x 64: 1.49 ms a stage, 2.27 with separate rows and a division each; 128 x 128 x 64 with its columns split
+// over CTAs 59 us, 389 with whole columns; 32 x 32 x 40 16 us, 260 with whole columns.
 #include <type_traits>
 
 #include "dycore.cuh"
@@ -70,12 +71,15 @@ struct SlowBlend {
 };
 
 // FIRST: a step's first stage (rho*theta in, no blend); INC: acoustic increments are added to
-// the momenta (stages 2 and 3 behind the fast modes).
-template <bool FIRST, bool INC>
+// the momenta (stages 2 and 3 behind the fast modes); DAMP: with the Rayleigh layer; PSUM: level
+// sums of rho and p' of the output (acc_mode 1, what the substeps that follow take; else as
+// acc_mode says).
+template <bool FIRST, bool INC, bool DAMP, bool PSUM>
 __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const __grid_constant__ SlowMaps m,
                                                         ZSplit zs) {
   using namespace sl;
   constexpr bool BLEND = !FIRST;
+  const int acc_mode = PSUM ? 1 : a.acc_mode;
   extern __shared__ unsigned char s_dyn[];
   __shared__ float s_trf[kMaxNz], s_ytrf[kMaxNz];   // theta_ref at Z face k, reciprocal of its floored value
   __shared__ double s_binv[kMaxNz], s_bpr[kMaxNz];  // EOS base state: 1/rt_ref, p_ref
@@ -178,9 +182,10 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     own_rt[r] = tx < w && r0 + r < h;
   }
   // blend partner at the current plane of the thread's row r
-  auto load_q0 = [&](int r) {
+  auto load_q0 = [&](auto tile_class, int r) {
+    constexpr bool IN = decltype(tile_class)::value;
     SlowBlend q{0.f, 0.f, 0.f, 0.f, 0.f};
-    if (!BLEND || !own_rt[r]) return q;
+    if (!BLEND || !(IN || own_rt[r])) return q;
     const int o = off[r];
     q.rho = __ldg(a.rho0 + o);
     q.rt = __ldg(a.rt0 + o);
@@ -339,7 +344,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   };
   auto plane_const = [&](int k) {
     PlaneConst pc{__ldg(a.idz_c + k), k > 0 ? __ldg(a.idz_f + k) : 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-    if (a.damp_c) {
+    if (DAMP) {
       pc.damp_c = __ldg(a.damp_c + k);
       pc.damp_f = __ldg(a.damp_f + k);
       pc.uref = __ldg(a.uref + k);
@@ -381,17 +386,10 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     for (int r = 0; r < ROWS; ++r) {
       const int b = b0 + r * BW;
       w_n[r] = W(sn, b);
-      if (!top) {
-        rho_n[r] = sn[R_RHO + b];
-        u_n[r] = U(sn, b);
-        v_n[r] = V(sn, b);
-        tt[r] = thn[d0 + r * DW];
-      } else {
-        rho_n[r] = 0.f;
-        u_n[r] = u_c[r];
-        v_n[r] = v_c[r];
-        tt[r] = tc[r + 1];
-      }
+      rho_n[r] = sn[R_RHO + b];  // the top plane reads none of these
+      u_n[r] = U(sn, b);
+      v_n[r] = V(sn, b);
+      tt[r] = top ? tc[r + 1] : thn[d0 + r * DW];
     }
     const float u_s = U(sr, b0 - BW), u_t = U(sr, b0 + ROWS * BW);  // rows -1 and ROWS
     const float v_s = V(sr, b0 - BW), v_t = V(sr, b0 + ROWS * BW);
@@ -434,7 +432,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         ro[r] = r1;
         to[r] = th1;
       }
-      if (a.acc_mode == 1) {
+      if (acc_mode == 1) {
         // p' of the output: the level sums, and (stored) the first substep's input
         const double binv = s_binv[k], bpr = s_bpr[k];
         float pv[ROWS];
@@ -452,7 +450,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
             rb += fx(pv[r], kFxP);
             if (a.p_out) put(a.p_out, kCell, r, 0, pv[r]);
           }
-      } else if (a.acc_mode == 2) {
+      } else if (acc_mode == 2) {
 #pragma unroll
         for (int r = 0; r < ROWS; ++r)
           if (IN || own_rt[r]) ra += fx(to[r], kFxTheta);
@@ -475,7 +473,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         float t_u = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_u[r], idx, idy, kc.idz);
         fz_u[r] = flt;
         t_u = fp::add_pgf(t_u, pp[d], pp[d - 1], idx);
-        if (a.damp_c) t_u = fp::add_damping(t_u, kc.damp_c, qc, kc.uref);
+        if (DAMP) t_u = fp::add_damping(t_u, kc.damp_c, qc, kc.uref);
         if (sx0) t_u = 0.0f;
         float u1 = fp::update(qc, dt, t_u, -1.0e30f);
         if (BLEND) u1 = fp::blend(a.wa, q0[r].u, a.wb, u1);
@@ -500,7 +498,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         float t_v = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_v[r], idx, idy, kc.idz);
         fz_v[r] = flt;
         t_v = fp::add_pgf(t_v, pp[d], pp[d - DW], idy);
-        if (a.damp_c) t_v = fp::add_damping(t_v, kc.damp_c, qc, kc.vref);
+        if (DAMP) t_v = fp::add_damping(t_v, kc.damp_c, qc, kc.vref);
         if (!IN && gj + r == 0 && open_y) t_v = 0.0f;
         float v1 = fp::update(qc, dt, t_v, -1.0e30f);
         if (BLEND) v1 = fp::blend(a.wa, q0[r].v, a.wb, v1);
@@ -518,26 +516,42 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
           if (sy[r]) fy[r] = 0.0f;
         }
       }
+      float flt[ROWS], t_w[ROWS];
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
-        const int d = d0 + r * DW, b = b0 + r * BW;
-        const float qc = w_c[r];
-        const float flt = fp::upwind(wc[d], qc, w_n[r]);
-        float t_w = 0.0f;
-        if (k > 0) {
+        flt[r] = fp::upwind(wc[d0 + r * DW], w_c[r], w_n[r]);
+        t_w[r] = 0.0f;
+      }
+      if (k > 0) {
+        float flux[ROWS];
+        bool near = true;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          const int d = d0 + r * DW, b = b0 + r * BW;
+          const float qc = w_c[r];
           float flw = fp::upwind(fp::avg(ucm[d - 1], uw[r + 1]), W(sr, b - 1), qc);
           float fle = fp::upwind(fp::avg(ucm[d], ue[r + 1]), qc, W(sr, b + 1));
           if (sx0) flw = 0.0f;
           if (sx1) fle = 0.0f;
-          t_w = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt, fz_w[r], idx, idy, kc.idzf);
-          bool near = true;
-          const float t = fp::add_buoyancy_ref(t_w, th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r],
-                                               a.gravity, near);
-          t_w = near ? t : fp::add_buoyancy(t_w, th_l[r], tc[r + 1], s_trf[k], rho_l[r], rho_c[r], a.gravity);
-          if (a.damp_c) t_w = fp::add_damping(t_w, kc.damp_f, qc, 0.0f);
+          flux[r] = -fp::divergence(fle, flw, fy[r + 1], fy[r], flt[r], fz_w[r], idx, idy, kc.idzf);
+          t_w[r] = fp::add_buoyancy_ref(flux[r], th_l[r], tc[r + 1], s_trf[k], s_ytrf[k], rho_l[r], rho_c[r],
+                                        a.gravity, near);
         }
-        fz_w[r] = flt;
-        float w1 = fp::update(qc, dt, t_w, -1.0e30f);
+        if (!near) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r)
+            t_w[r] = fp::add_buoyancy(flux[r], th_l[r], tc[r + 1], s_trf[k], rho_l[r], rho_c[r], a.gravity);
+        }
+        if (DAMP) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) t_w[r] = fp::add_damping(t_w[r], kc.damp_f, w_c[r], 0.0f);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const float qc = w_c[r];
+        fz_w[r] = flt[r];
+        float w1 = fp::update(qc, dt, t_w[r], -1.0e30f);
         if (BLEND) w1 = fp::blend(a.wa, q0[r].w, a.wb, w1);
         put(a.o_w, kFaceZ, r, 0, w1);
         if (top) {  // top face: zero tendency
@@ -570,18 +584,18 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
       const PlaneConst kc = plane_const(k);
       SlowBlend q0[ROWS];  // the derive phase covers the loads
 #pragma unroll
-      for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(r);
+      for (int r = 0; r < ROWS; ++r) q0[r] = load_q0(tile_class, r);
       wait_plane(k + 1, k);
       derive(tile_class, k);
       if (k + 1 < nz) derive_theta(tile_class, k + 1);
       __syncthreads();  // publishes plane k's derived values; slot (k-1) is free
       if (s_abort[pb]) return true;
       if (tid == ISSUER) {
-        if (a.acc_mode && k > kb) {
+        if (acc_mode && k > kb) {
           long long sa = 0, sb = 0;
           for (int q = 0; q < NW; ++q) { sa += s_red[pb ^ 1][q][0]; sb += s_red[pb ^ 1][q][1]; }
           acc_add(a.acc_a + k - 1, sa);
-          if (a.acc_mode == 1) acc_add(a.acc_b + k - 1, sb);
+          if (acc_mode == 1) acc_add(a.acc_b + k - 1, sb);
         }
         if (k + 2 <= ke) { issue(k + 2); issued = k + 2; }
       }
@@ -602,7 +616,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         if (BLEND) v1 = fp::blend(a.wa, __ldg(a.v0 + gidx(g, i0 + tx, ny, k)), a.wb, v1);
         store_tile(a.o_v, g, kFaceY, i0 + tx, ny, k, v1, edge);
       }
-      if (a.acc_mode) {
+      if (acc_mode) {
         const long long ta = warp_total_fx(ra), tb = warp_total_fx(rb);
         if (tx == 0) { s_red[pb][ty][0] = ta; s_red[pb][ty][1] = tb; }
       }
@@ -617,22 +631,44 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
       for (int kk = waited + 1; kk <= issued; ++kk) mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1);
     return;
   }
-  if (a.acc_mode) {
+  if (acc_mode) {
     __syncthreads();
     if (tid == ISSUER) {
       const int pb = (ke - 1) & 1;
       long long sa = 0, sb = 0;
       for (int q = 0; q < NW; ++q) { sa += s_red[pb][q][0]; sb += s_red[pb][q][1]; }
       acc_add(a.acc_a + ke - 1, sa);
-      if (a.acc_mode == 1) acc_add(a.acc_b + ke - 1, sb);
+      if (acc_mode == 1) acc_add(a.acc_b + ke - 1, sb);
     }
   }
 }
 
 template <bool FIRST, bool INC>
 cudaError_t allow_smem() {
-  return cudaFuncSetAttribute(k_slow_tma<FIRST, INC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)sl::smem_bytes(INC));
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](auto* kernel) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sl::smem_bytes(INC));
+  };
+  allow(k_slow_tma<FIRST, INC, false, false>);
+  allow(k_slow_tma<FIRST, INC, false, true>);
+  allow(k_slow_tma<FIRST, INC, true, false>);
+  allow(k_slow_tma<FIRST, INC, true, true>);
+  return e;
+}
+
+template <bool FIRST, bool INC>
+void launch(const SlowArgs& a, const SlowMaps& m, dim3 grid, const ZSplit& zs, cudaStream_t s) {
+  const dim3 block(sl::TX, sl::NW);
+  const size_t smem = sl::smem_bytes(INC);
+  const bool psum = a.acc_mode == 1;
+  if (a.damp_c) {
+    if (psum) k_slow_tma<FIRST, INC, true, true><<<grid, block, smem, s>>>(a, m, zs);
+    else k_slow_tma<FIRST, INC, true, false><<<grid, block, smem, s>>>(a, m, zs);
+  } else {
+    if (psum) k_slow_tma<FIRST, INC, false, true><<<grid, block, smem, s>>>(a, m, zs);
+    else k_slow_tma<FIRST, INC, false, false><<<grid, block, smem, s>>>(a, m, zs);
+  }
 }
 
 }  // namespace
@@ -649,13 +685,12 @@ cudaError_t launch_slow_tma(const SlowArgs& a, const SlowMaps& m, cudaStream_t s
   const bool first = a.th_is_rt != 0;
   if (a.g.nz > kMaxNz || a.g.nz < 1 || !a.err || a.tend_only || first != !a.rho0 || (first && a.du))
     return cudaErrorInvalidValue;
-  const dim3 block(sl::TX, sl::NW);
   dim3 grid((a.g.nx + sl::TX - 1) / sl::TX, (a.g.ny + sl::TY - 1) / sl::TY);
   const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, 2, 1.0f);
   grid.z = zs.chunks;
-  if (first) k_slow_tma<true, false><<<grid, block, sl::smem_bytes(false), s>>>(a, m, zs);
-  else if (a.du) k_slow_tma<false, true><<<grid, block, sl::smem_bytes(true), s>>>(a, m, zs);
-  else k_slow_tma<false, false><<<grid, block, sl::smem_bytes(false), s>>>(a, m, zs);
+  if (first) launch<true, false>(a, m, grid, zs, s);
+  else if (a.du) launch<false, true>(a, m, grid, zs, s);
+  else launch<false, false>(a, m, grid, zs, s);
   return cudaGetLastError();
 }
 
