@@ -11,12 +11,14 @@
 //   u, v                              36 x 17 boxes: owned faces + the east/north face
 //   w                                 32 x 16 box: owned Z faces (plane nz: w only)
 // A thread computes the mixing ratios of its rows one plane ahead and those of the rows around
-// them, lanes 0-7 those of the warp's two ring columns, with one reciprocal per position; the
-// Y fluxes between its rows are computed once, and the flux out of a plane's top is carried as
-// the next plane's bottom flux.  The kernel is issue-bound (69 % of the issue slots; 13 fields
-// of 4 B per cell would take 0.53 ms for 1024 x 1024 x 64, three tracers, at the copy
-// bandwidth): there 0.766 ms a stage, 1.045 with two rows eight apart per thread, 426
-// instructions per cell and a block barrier per plane; 517 x 389 x 50 0.141 ms against 0.184.
+// them, and a position of the warp's two ring columns, with one reciprocal per position; all of
+// a plane's come first, with one test for the quotients that need a plain division, so their
+// chains interleave.  The Y fluxes between its rows are computed once, and the flux out of a
+// plane's top is carried as the next plane's bottom flux.  Bounds: issue, close to HBM (13
+// fields of 4 B per cell take 0.53 ms for 1024 x 1024 x 64, three tracers, at the copy
+// bandwidth): there 0.644 ms a stage, 0.767 with a test per position and the blend decided at
+// run time, 1.045 with two rows eight apart per thread, 426 instructions per cell and a block
+// barrier per plane; 517 x 389 x 50 0.115 ms, 0.141, 0.191.
 #include <type_traits>
 
 #include "physics.cuh"
@@ -42,7 +44,7 @@ static_assert(O_U % 32 == 0 && O_V % 32 == 0 && O_W % 32 == 0 && O_Q % 32 == 0 &
               "128-byte aligned boxes that fit");
 }  // namespace tt
 
-template <bool TERRAIN, int N>  // N: tracers
+template <bool TERRAIN, int N, bool BLEND>  // N: tracers; BLEND: stages 2 and 3
 __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
     k_tracer_tma(const TracerArgs a, const __grid_constant__ TracerMaps m, ZSplit zs) {
   using namespace tt;
@@ -115,7 +117,6 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
   const int gi = i0 + lane, gj = j0 + r0;  // the thread's column and first row
   const bool edge = (g.per_x && (i0 <= 1 || i0 + w >= nx - 1)) || (g.per_y && (j0 <= 1 || j0 + h >= ny - 1));
   const float idx = g.inv_dx, idy = g.inv_dy;
-  const bool blend = a.q0[0] != nullptr;
   // Interior tiles (full, away from every periodic edge ring) run a copy of the plane loop
   // with plain stores instead of the periodic mirror stores; the arithmetic is the same.
   const bool interior = !edge && i0 + TX <= nx && j0 + TY <= ny;
@@ -129,8 +130,9 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
     if (lane == 0) mbar_arrive(&s_empty[(kk - kg) % NSLOT]);
   };
   auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
-  // mixing ratios (dry_transport.cu:91-94) at position b of a plane's cell boxes
-  auto mix = [&](const float* st, int b, float* q) {
+  // mixing ratios (dry_transport.cu:91-94) at position b of a plane's cell boxes; `near` is
+  // cleared where one is not finite and the plain divisions are due
+  auto mix_near = [&](const float* st, int b, float* q, bool& near) {
     const float rr = fmaxf(st[O_RHO + b], 1.0e-6f), y = fp::recip(rr);
     float sum = 0.0f;
 #pragma unroll
@@ -138,10 +140,17 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
       q[t] = fp::div_by(st[O_Q + t * Q_STRIDE + b], rr, y);
       sum += fabsf(q[t]);
     }
-    if (!fp::finite(sum)) {
+    near = near && fp::finite(sum);
+  };
+  auto mix_plain = [&](const float* st, int b, float* q) {
+    const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
 #pragma unroll
-      for (int t = 0; t < N; ++t) q[t] = fp::div(st[O_Q + t * Q_STRIDE + b], rr);
-    }
+    for (int t = 0; t < N; ++t) q[t] = fp::div(st[O_Q + t * Q_STRIDE + b], rr);
+  };
+  auto mix = [&](const float* st, int b, float* q) {
+    bool near = true;
+    mix_near(st, b, q, near);
+    if (!near) mix_plain(st, b, q);
   };
 
   auto run = [&](auto tile_class) -> bool {  // false when a bounded wait gave up
@@ -194,24 +203,46 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
       for (int r = 0; r < ROWS; ++r) {
         idz[r] = TERRAIN ? (own[r] ? __ldg(a.idz_c + off[r]) : 0.f) : __ldg(a.idz_c + k);
 #pragma unroll
-        for (int t = 0; t < N; ++t) q0[r][t] = blend && own[r] ? __ldg(a.q0[t] + off[r]) : 0.f;
+        for (int t = 0; t < N; ++t) q0[r][t] = BLEND && own[r] ? __ldg(a.q0[t] + off[r]) : 0.f;
       }
-      // the warp's ring columns, and its rows for the neighbouring lanes
-      if (lane < 2 * ROWS) {
-        float q[N];
-        mix(st, ring_b, q);
+      // the mixing ratios of the rows around the warp's and of its ring columns (a position per
+      // lane), and of its rows at plane k+1: one test for the plain divisions
+      const bool top = k + 1 == nz;
+      float qs[N], qn[N], qr[N], qt[ROWS][N];
+      bool near = true;
+      mix_near(st, b0 - CBW, qs, near);
+      mix_near(st, b0 + ROWS * CBW, qn, near);
+      mix_near(st, ring_b, qr, near);
+      if (!wait_full(k + 1)) return false;
+      const float* sn = slot_at(k + 1);
+      if (!top) {
 #pragma unroll
-        for (int t = 0; t < N; ++t) s_q[pb][wid][t][ring_row][ring_col + 1] = q[t];
+        for (int r = 0; r < ROWS; ++r) mix_near(sn, b0 + r * CBW, qt[r], near);
+      }
+      if (!near) {
+        mix_plain(st, b0 - CBW, qs);
+        mix_plain(st, b0 + ROWS * CBW, qn);
+        mix_plain(st, ring_b, qr);
+        if (!top) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) mix_plain(sn, b0 + r * CBW, qt[r]);
+        }
+      }
+      if (top) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+          for (int t = 0; t < N; ++t) qt[r][t] = qc[r][t];
+      }
+      // the ring columns, and the warp's rows for the neighbouring lanes
+      if (lane < 2 * ROWS) {
+#pragma unroll
+        for (int t = 0; t < N; ++t) s_q[pb][wid][t][ring_row][ring_col + 1] = qr[t];
       }
 #pragma unroll
       for (int r = 0; r < ROWS; ++r)
 #pragma unroll
         for (int t = 0; t < N; ++t) s_q[pb][wid][t][r][lane + 1] = qc[r][t];
-      float qs[N], qn[N];  // the rows around the warp's
-      mix(st, b0 - CBW, qs);
-      mix(st, b0 + ROWS * CBW, qn);
-      if (!wait_full(k + 1)) return false;
-      const float* sn = slot_at(k + 1);
       __syncwarp();
       const float* su = st + O_U + r0 * FBW + lane;
       const float* sv = st + O_V + r0 * FBW + lane;
@@ -222,30 +253,26 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
       for (int r = 0; r < ROWS; ++r) {
         const float fw = su[r * FBW], fe = su[r * FBW + 1], fn = sv[(r + 1) * FBW];
         const float ft = sn[O_W + (r0 + r) * OBW + lane];
-        float qt[N];
-        if (k + 1 < nz) {
-          mix(sn, b0 + r * CBW, qt);
-        } else {
-#pragma unroll
-          for (int t = 0; t < N; ++t) qt[t] = qc[r][t];
-        }
 #pragma unroll
         for (int t = 0; t < N; ++t) {
           const float c = qc[r][t];
           const float gw = fp::upwind(fw, s_q[pb][wid][t][r][lane], c);
           const float ge = fp::upwind(fe, c, s_q[pb][wid][t][r][lane + 2]);
           const float gn = fp::upwind(fn, c, r + 1 < ROWS ? qc[r + 1 < ROWS ? r + 1 : r][t] : qn[t]);
-          const float gt = fp::upwind(ft, c, qt[t]);
+          const float gt = fp::upwind(ft, c, qt[r][t]);
           const float div = fp::divergence(ge, gw, gn, gy[t], gt, fz[r][t], idx, idy, idz[r]);
           float out = fp::update(st[O_Q + t * Q_STRIDE + b0 + r * CBW], -a.dt, div, 0.0f);
-          if (blend) out = fp::blend(a.wa, q0[r][t], a.wb, out);
+          if (BLEND) out = fp::blend(a.wa, q0[r][t], a.wb, out);
           if (IN) a.q_out[t][off[r]] = out;
           else if (own[r]) store_tile(a.q_out[t], g, kCell, gi, gj + r, k, out, edge);
           gy[t] = gn;
           fz[r][t] = gt;
         }
+      }
 #pragma unroll
-        for (int t = 0; t < N; ++t) qc[r][t] = qt[t];
+      for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+        for (int t = 0; t < N; ++t) qc[r][t] = qt[r][t];
         off[r] += g.plane;
       }
       release(k);
@@ -258,16 +285,20 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
 
 template <bool TERRAIN, int N>
 cudaError_t allow_smem() {
-  return cudaFuncSetAttribute(k_tracer_tma<TERRAIN, N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)tt::smem_bytes(N));
+  cudaError_t e = cudaFuncSetAttribute(k_tracer_tma<TERRAIN, N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)tt::smem_bytes(N));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_tracer_tma<TERRAIN, N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)tt::smem_bytes(N));
+  return e;
 }
 
-template <bool TERRAIN>
+template <bool TERRAIN, bool BLEND>
 void launch(const TracerArgs& a, const TracerMaps& m, dim3 grid, const ZSplit& zs, cudaStream_t s) {
   const size_t smem = tt::smem_bytes(a.ntracers);
-  if (a.ntracers == 1) k_tracer_tma<TERRAIN, 1><<<grid, tt::NT, smem, s>>>(a, m, zs);
-  else if (a.ntracers == 2) k_tracer_tma<TERRAIN, 2><<<grid, tt::NT, smem, s>>>(a, m, zs);
-  else k_tracer_tma<TERRAIN, 3><<<grid, tt::NT, smem, s>>>(a, m, zs);
+  if (a.ntracers == 1) k_tracer_tma<TERRAIN, 1, BLEND><<<grid, tt::NT, smem, s>>>(a, m, zs);
+  else if (a.ntracers == 2) k_tracer_tma<TERRAIN, 2, BLEND><<<grid, tt::NT, smem, s>>>(a, m, zs);
+  else k_tracer_tma<TERRAIN, 3, BLEND><<<grid, tt::NT, smem, s>>>(a, m, zs);
 }
 
 }  // namespace
@@ -287,8 +318,9 @@ cudaError_t launch_tracer_tma(const TracerArgs& a, const TracerMaps& m, cudaStre
   dim3 grid((a.g.nx + tt::TX - 1) / tt::TX, (a.g.ny + tt::TY - 1) / tt::TY);
   const ZSplit zs = z_split(grid.x * grid.y, a.g.nz, tt::MIN_CTAS, 1.0f);
   grid.z = zs.chunks;
-  if (a.terrain) launch<true>(a, m, grid, zs, s);
-  else launch<false>(a, m, grid, zs, s);
+  const bool blend = a.q0[0] != nullptr;
+  if (a.terrain) blend ? launch<true, true>(a, m, grid, zs, s) : launch<true, false>(a, m, grid, zs, s);
+  else blend ? launch<false, true>(a, m, grid, zs, s) : launch<false, false>(a, m, grid, zs, s);
   return cudaGetLastError();
 }
 
