@@ -16,7 +16,8 @@
 //   - p' - p'_ref and rho - rho_ref of a level are formed once and carried up;
 //   - the level sums stay in shared memory until the CTA's end: one atomic per level.
 // 1024 x 1024 x 64: 0.549 ms a substep (0.82 of the copy bandwidth), 0.627 with k_fast_tma's
-// split columns, 0.654 with its whole columns; 517 x 389 x 50: 99 us, 116 with either.
+// split columns, 0.654 with its whole columns; 517 x 389 x 50: 96 us (99.6 with a test for the
+// EOS's far form per row instead of one per plane), 116 with k_fast_tma.
 #include <type_traits>
 
 #include "dycore.cuh"
@@ -278,13 +279,28 @@ __global__ void __launch_bounds__(fr::NT, fr::MIN_CTAS)
         const float idzc = t_idzc[kt];
         const double binv = t_binv[kt], bpr = t_bpr[kt];
         long long sa = 0, sb = 0;
+        // the rows' new density, rho*theta and p' first, with one test for the EOS's far form
+        float nrho[ROWS], nrt[ROWS], np[ROWS];
+        bool near = true;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+          nrho[r] = fp::density(rho[r], s_ue[pb][wid][r][lane + 1], un[r], vn[r + 1], vn[r], wn[r], dwc[r], idx, idy,
+                                idzc, dtf);
+          nrt[r] = fp::mul(nrho[r], st[L::O_TH + (r0 + r) * OBW + lane]);
+          if (KIND == 0) {
+            bool n = true;
+            np[r] = eos_pprime_near(nrho[r], nrt[r], binv, bpr, n);
+            near = near && (n || !own[r]);
+          }
+        }
+        if (KIND == 0 && !near) {
+#pragma unroll
+          for (int r = 0; r < ROWS; ++r) np[r] = eos_pprime_ref(nrho[r], nrt[r], binv, bpr);
+        }
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
           if (!own[r]) continue;
-          const float ue = s_ue[pb][wid][r][lane + 1];
-          const float rn =
-              fp::density(rho[r], ue, un[r], vn[r + 1], vn[r], wn[r], dwc[r], idx, idy, idzc, dtf);
-          const float rt = fp::mul(rn, st[L::O_TH + (r0 + r) * OBW + lane]);
+          const float rn = nrho[r], rt = nrt[r];
           if (FINAL) {
             const int ob = (r0 + r) * OBW + lane;
             put(a.f_rho, kCell, r, k, 0, rn);
@@ -296,7 +312,7 @@ __global__ void __launch_bounds__(fr::NT, fr::MIN_CTAS)
             // open sides: faces nx and ny belong to no tile; their step values are base + increment
             if (!IN && !g.per_x && gi == nx - 1) {
               const int o = gidx(g, nx, gj + r, k);
-              a.f_u[o] = fp::add(__ldg(a.bu + o), ue);
+              a.f_u[o] = fp::add(__ldg(a.bu + o), s_ue[pb][wid][r][lane + 1]);
             }
             if (!IN && !g.per_y && gj + r == ny - 1) {
               const int o = gidx(g, gi, ny, k);
@@ -309,10 +325,9 @@ __global__ void __launch_bounds__(fr::NT, fr::MIN_CTAS)
             if (k + 1 < nz) put(a.dw_out, kFaceZ, r, k, 1, wn[r]);
           }
           if (KIND == 0) {
-            const float pv = eos_pprime_ref(rn, rt, binv, bpr);
             sa += fx(rn, kFxRho);
-            sb += fx(pv, kFxP);
-            put(a.p_out, kCell, r, k, 0, pv);
+            sb += fx(np[r], kFxP);
+            put(a.p_out, kCell, r, k, 0, np[r]);
           } else if (acc_mode == 2) {
             sa += fx(fp::theta(rn, rt), kFxTheta);
           }
