@@ -57,9 +57,8 @@ __device__ __forceinline__ float dry_cp() { return kRd / kKappa; }
 __device__ __forceinline__ float column_dpdz(int k, int nz, float pm, float pc, float pn, float zm,
                                              float zcc, float zn) {
   if (nz == 1) return 0.0f;
-  if (k == 0) return (pn - pc) / fmaxf(zn - zcc, 1.0e-6f);
-  if (k + 1 == nz) return (pc - pm) / fmaxf(zcc - zm, 1.0e-6f);
-  return (pn - pm) / fmaxf(zn - zm, 1.0e-6f);
+  const bool low = k == 0, top = k + 1 == nz;  // selected, not branched: one division
+  return ((top ? pc : pn) - (low ? pc : pm)) / fmaxf((top ? zcc : zn) - (low ? zcc : zm), 1.0e-6f);
 }
 
 // ---------------------------------------------------------------------------

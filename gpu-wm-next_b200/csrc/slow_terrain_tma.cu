@@ -17,8 +17,8 @@
 // per SM double-buffered).  The owned columns' metric values (the cell and face inverse
 // layer depths) and the blend partner q0 are per-thread coalesced loads a plane ahead.
 // Bounds: issue and the two barriers of a plane, as in the flat stage, whose shared and carried
-// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.699 ms a stage against 0.998 with
-// separate rows, 201 x 163 x 40: 85 us against 119 (27 fields of 4 B per cell at the copy
+// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.684 ms a stage against 0.998 with
+// separate rows, 201 x 163 x 40: 83 us against 119 (27 fields of 4 B per cell at the copy
 // bandwidth: 0.35 ms and 22 us).
 #include <type_traits>
 
