@@ -34,7 +34,7 @@ _SOURCES = ["capi.cu", "dycore.cu", "fast_tma.cu", "fast_rows.cu", "fast_terrain
             "physics.cu", "halo.cu", "plan_view.cu", "surrogate.cu", "surrogate_rain.cu", "scalar.cu", "cases.cpp"]
 _HEADERS = ["common.cuh", "stencil.cuh", "dycore.cuh", "physics.cuh", "halo.cuh", "tma.cuh", "zsplit.cuh", "plan_view.cuh", "rain_cell.cuh", "surrogate.cuh", "surrogate_rain.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-shared"]
+              "-Xcompiler", "-fPIC", "-shared", "-t", "4"]
 
 OK, ERR_ARG, ERR_CUDA, ERR_STATE, ERR_NO_DEVICE, ERR_TIMEOUT = 0, -1, -2, -3, -4, -5
 CELL, FACE_X, FACE_Y, FACE_Z = 0, 1, 2, 3
