@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(fz::NT, 2)
         if (k + AHEAD <= kl) { issue(k + AHEAD); issued = k + AHEAD; }
       }
       // ---- K15 density of plane k, K10 rho*theta, stores
-      long long sum = 0;
+      long long sum[ROWS] = {0, 0};
 #pragma unroll
       for (int r = 0; r < ROWS; ++r) {
         if (!(IN || own_rt[r])) continue;
@@ -415,10 +415,14 @@ __global__ void __launch_bounds__(fz::NT, 2)
           // the next substep's pressure, loaded with its ring
           if (KIND == 0) put(a.p_out, kCell, r, k, 0, eos_pressure(rnew, rt));
         }
-        if (acc) sum += fx(fp::theta(rnew, rt), kFxTheta);
+        if (acc) sum[r] = fx(fp::theta(rnew, rt), kFxTheta);
       }
       if (acc) {
-        const long long t = warp_total_fx(sum);
+        // row by row: a warp total wraps at 2^56 (theta of 1e8 K), so in a state that has blown
+        // up the rows a total covers show, and one row is what the other kernels' totals cover
+        long long t = 0;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) t += warp_total_fx(sum[r]);
         if (tx == 0) S.red[pb][ty] = t;
       }
 #pragma unroll
