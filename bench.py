@@ -481,7 +481,7 @@ def substep_roofline(model, g, stream, torch, steps=2):
     total = sum(v["total_ms"] for v in rep.values())
     shares = {k: round(v["total_ms"] / total, 4) for k, v in rep.items()}
     fast_tile = 3 if tile == 4 else tile  # the kernel whose launches were timed
-    kname = {0: "k_fast_flat", 3: "k_fast_tma"}.get(fast_tile, f"k_fast_substep<{fast_tile}>")
+    kname = {0: "k_fast_flat", 3: "k_fast_rows"}.get(fast_tile, f"k_fast_substep<{fast_tile}>")
     return {"bound": "hbm", "achieved": achieved, "unit": "GB/s", "traffic": read_traffic(g, fast_tile),
             "kernel": f"{kname} (one acoustic substep)",
             "algorithmic_bytes_per_launch": SUBSTEP_ALGO_BYTES_PER_CELL * cells,
@@ -490,7 +490,7 @@ def substep_roofline(model, g, stream, torch, steps=2):
 
 
 # committed ncu summaries of the acoustic-substep kernels (DRAM bytes per cell of one launch)
-TRAFFIC_PROFILES = {3: "k_fast_tma_768x768x64.txt"}
+TRAFFIC_PROFILES = {3: "k_fast_rows_768x768x64.txt"}
 
 
 def read_traffic(g, fast_tile):
