@@ -582,17 +582,18 @@ StripJob strip_job(float* padded, float* compact, const float* aux, int orient, 
 // before the boundary strips were written (mode 0: rho*theta stored, 2: theta stored)
 int recompute_theta_sums(gwm_b200_ctx* c, Member& M, const float* rho, const float* th, int mode);
 
-// Reads and clears the device error words; call after the stream has drained.
+// Reads and clears every member's device error word; call after the stream has drained.
 int check_device_errors(gwm_b200_ctx* c) {
+  bool gave_up = false;
   for (auto& M : c->m) {
     int e = 0;
     CK(cudaMemcpyAsync(&e, M.err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    if (e) {
-      CK(cudaMemsetAsync(M.err, 0, sizeof(int), c->stream));
-      return fail(c, GWM_B200_ERR_TIMEOUT, "a bounded wait in the acoustic substep gave up (tile load did not complete)");
-    }
+    if (!e) continue;
+    gave_up = true;
+    CK(cudaMemsetAsync(M.err, 0, sizeof(int), c->stream));
   }
+  if (gave_up) return fail(c, GWM_B200_ERR_TIMEOUT, "a kernel's bounded wait gave up (a load did not complete)");
   return GWM_B200_OK;
 }
 
@@ -1936,7 +1937,7 @@ int gwm_b200_advance_tracers(gwm_b200_ctx* c) {
   }
   c->launches = c->cur_launches;
   CK(cudaStreamSynchronize(c->stream));
-  return GWM_B200_OK;
+  return check_device_errors(c);
 }
 
 int gwm_b200_warm_rain(gwm_b200_ctx* c, int fallout) {
@@ -1952,7 +1953,7 @@ int gwm_b200_warm_rain(gwm_b200_ctx* c, int fallout) {
   }
   c->launches = c->cur_launches;
   CK(cudaStreamSynchronize(c->stream));
-  return GWM_B200_OK;
+  return check_device_errors(c);
 }
 
 int gwm_b200_fast_modes(gwm_b200_ctx* c) {
@@ -2009,7 +2010,7 @@ int gwm_b200_fast_modes(gwm_b200_ctx* c) {
   }
   c->launches = c->cur_launches;
   CK(cudaStreamSynchronize(c->stream));
-  return GWM_B200_OK;
+  return check_device_errors(c);
 }
 
 int gwm_b200_slow_tendencies(gwm_b200_ctx* c, int member, gwm_b200_fields* h) {

@@ -1,0 +1,49 @@
+"""The stand-alone operators run the TMA-fed kernels by default, whose bounded waits can give
+up: the call that ran such a kernel reports it, for every member, and the next call is not
+charged with it."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _member(gwm, terrain, nx=72, ny=40, nz=16):
+    hill = None
+    if terrain:
+        hill = gwm.build_terrain("cosine_mountain", nx, ny, 2000.0, 2000.0, height=300.0, half_width_x=0.3,
+                                 half_width_y=0.3)
+    flat = gwm.GridSpec(nx, ny, nz, dx=2000.0, dy=2000.0, z_top=8000.0)
+    grid = gwm.GridSpec(nx, ny, nz, dx=2000.0, dy=2000.0, z_top=8000.0, terrain=hill)
+    state = gwm.build_case("moist_sounding", flat, gwm.CaseParams(theta_ref=300.0, noise_rms_k=0.5, seed=3,
+                                                                  relative_humidity=1.02), moist=True)
+    spec = gwm.MemberSpec(step=gwm.StepConfig(dt=1.0, fast_substeps=3),
+                          rain=gwm.WarmRainConfig(dt=1.0, rain_terminal_velocity=12.0), moist=True)
+    return grid, state, spec
+
+
+OPERATORS = {"tracers": lambda m: m.advance_passive_tracers_ssprk3(), "fast_modes": lambda m: m.fast_modes()}
+
+
+@pytest.mark.parametrize("members", [1, 2])
+@pytest.mark.parametrize("terrain", [False, True])
+@pytest.mark.parametrize("op", list(OPERATORS))
+def test_operator_reports_a_wait_that_gave_up(gwm, op, terrain, members):
+    grid, state, spec = _member(gwm, terrain)
+    run = OPERATORS[op]
+    out = {}
+    for stall in (False, True):
+        with gwm.Model([grid] * members, [spec] * members) as m:
+            for q in range(members):
+                m.upload(state, member=q)
+            if stall:
+                for q in range(members):
+                    m.test_stall_tile_load(plane=2, member=q)
+                with pytest.raises(RuntimeError, match="status -5"):
+                    run(m)
+                for q in range(members):
+                    m.upload(state, member=q)
+            run(m)
+            out[stall] = [m.download(member=q) for q in range(members)]
+    for a, b in zip(out[False], out[True]):
+        for k in a:
+            np.testing.assert_array_equal(a[k], b[k], err_msg=k)
