@@ -178,8 +178,8 @@ __global__ void __launch_bounds__(fz::NT, 2)
     if (!mbar_wait(&S.bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1)) {
       S.abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
-    } else {
-      waited = kk;  // a plane whose wait gave up stays in the drain below
+    } else if (waited == kk - 1) {
+      waited = kk;  // a plane whose wait gave up stays in the drain below, with those after it
     }
   };
   // values of plane kk at derived-plane position (r, c)

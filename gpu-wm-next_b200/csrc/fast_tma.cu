@@ -221,8 +221,8 @@ __device__ __forceinline__ bool fast_tile(const FastArgs& a, const FastMaps& m, 
     if (!mbar_wait(&S.bar[(rb + kk) % NSLOT], ((rb + kk) / NSLOT) & 1)) {
       S.abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
-    } else {
-      waited = kk;  // a plane whose wait gave up stays in the drain below
+    } else if (waited == kk - 1) {
+      waited = kk;  // a plane whose wait gave up stays in the drain below, with those after it
     }
   };
   // K10 + K20: pressure perturbation of plane kk at the owned cells and the halo ring

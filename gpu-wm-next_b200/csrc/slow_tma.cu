@@ -161,8 +161,8 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
     if (!mbar_wait(&s_bar[(kk - kg) % NSLOT], ((kk - kg) / NSLOT) & 1)) {
       s_abort[epoch & 1] = 1;
       atomicExch(a.err, 1);
-    } else {
-      waited = kk;  // a plane whose wait gave up stays in the drain below
+    } else if (waited == kk - 1) {
+      waited = kk;  // a plane whose wait gave up stays in the drain below, with those after it
     }
   };
   // raw accessors: box index of derived position (r, c) is r * BW + c + 3

@@ -47,3 +47,25 @@ def test_operator_reports_a_wait_that_gave_up(gwm, op, terrain, members):
     for a, b in zip(out[False], out[True]):
         for k in a:
             np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+
+
+# The first plane that a CTA loads never arrives while the ones above it do: its wait gives up
+# in the prologue, and the planes behind it are still accounted for when the CTA leaves.
+@pytest.mark.parametrize("terrain", [False, True])
+@pytest.mark.parametrize("op", ["step", *OPERATORS])
+def test_first_plane_of_a_chunk_never_arrives(gwm, op, terrain):
+    grid, state, spec = _member(gwm, terrain)
+    run = dict(OPERATORS, step=lambda m: m.step(1))[op]
+    out = {}
+    for stall in (False, True):
+        with gwm.Model(grid, spec) as m:
+            m.upload(state)
+            if stall:
+                m.test_stall_tile_load(plane=0)
+                with pytest.raises(RuntimeError, match="status -5"):
+                    run(m)
+                m.upload(state)
+            run(m)
+            out[stall] = m.download()
+    for k in out[False]:
+        np.testing.assert_array_equal(out[True][k], out[False][k], err_msg=k)
