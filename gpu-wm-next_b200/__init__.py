@@ -695,11 +695,13 @@ class Model:
                                                 C.byref(t)), "tracer_total")
         return t.value
 
-    def test_stall_tile_load(self, plane: int, member: int = 0):
-        """Failure-path testing: the next TMA-fed stencil launch leaves one CTA's tile
+    def test_stall_tile_load(self, plane: int, member: int = 0, kernel: Optional[str] = None):
+        """Failure-path testing: the next TMA-fed stencil launch (of ``kernel``, if given:
+        slow_stage, fast_substep, last_substep or tracer_stage) leaves one CTA's tile
         loads of ``plane`` unissued, so its bounded wait runs out (the step call then
         fails with GWM_B200_ERR_TIMEOUT)."""
-        self._check(lib().gwm_b200_test_stall_tile_load(self._h, member, plane), "test_stall_tile_load")
+        kind = 0 if kernel is None else 1 + ("slow_stage", "fast_substep", "last_substep", "tracer_stage").index(kernel)
+        self._check(lib().gwm_b200_test_stall_tile_load(self._h, member, 65536 * kind + plane), "test_stall_tile_load")
 
     def apply_reference_boundaries(self, member: int = 0):
         """apply_reference_boundaries once on the current state."""

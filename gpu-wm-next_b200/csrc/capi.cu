@@ -36,6 +36,7 @@
 #include "plan_view.cuh"
 #include "surrogate.cuh"
 #include "surrogate_rain.cuh"
+#include "tma.cuh"
 
 using namespace gwmb;
 
@@ -1549,8 +1550,9 @@ int gwm_b200_test_stall_tile_load(gwm_b200_ctx* c, int member, int plane) {
   const int rc = check_member(c, member);
   if (rc) return rc;
   Member& M = c->m[member];
-  if (plane < 0 || plane > M.g.nz) return fail(c, GWM_B200_ERR_ARG, "plane out of range");
-  const int word = plane + 1;  // err[1]: 0 = no request
+  const int kind = plane >> 16, level = plane & 0xffff;
+  if (plane < 0 || kind > kStallTracer || level > M.g.nz) return fail(c, GWM_B200_ERR_ARG, "plane out of range");
+  const int word = (kind << 16) | (level + 1);  // err[1]: 0 = no request
   CK(cudaMemcpyAsync(M.err + 1, &word, sizeof(int), cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return GWM_B200_OK;

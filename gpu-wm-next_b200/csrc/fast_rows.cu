@@ -106,10 +106,7 @@ __global__ void __launch_bounds__(fr::NT, fr::MIN_CTAS)
 
   if (wid == NW) {  // ---- producer
     if (lane == 0) {
-      // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads
-      // of one of its planes unissued, so that CTA's bounded waits run out
-      int stall = -1;
-      if (*(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
+      int stall = take_stall(a.err, FINAL ? kStallLastSubstep : kStallSubstep);  // failure-path tests
       if (stall >= 0) stall = kg + stall % (kl - kg + 1);
       int issued = kg - 1;
       for (int kk = kg; kk <= kl; ++kk) {

@@ -140,10 +140,7 @@ __global__ void __launch_bounds__(fz::NT, 2)
     for (int q = tid; q < nz; q += NT) { a.clr_a[q] = 0ull; a.clr_b[q] = 0ull; }
   __syncthreads();
 
-  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads of
-  // one of its planes unissued, so that CTA's bounded wait runs out
-  int stall = -1;
-  if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
+  int stall = tid == ISSUER ? take_stall(a.err, FINAL ? kStallLastSubstep : kStallSubstep) : -1;  // failure-path tests
   // the CTA's planes are kb .. ke-1; it also loads the planes around them: the one below for
   // its lowest Z face and dp/dz, the one above for its highest
   const int kb = zs.first(blockIdx.z), ke = zs.last(blockIdx.z, nz), kg = kb > 0 ? kb - 1 : 0, kl = min(ke, nz - 1);

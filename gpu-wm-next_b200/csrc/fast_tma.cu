@@ -450,12 +450,10 @@ __device__ __forceinline__ void fast_cta_init(FastShared& S) {
   }
 }
 
-// err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads
-// of plane err[1] - 1 unissued, so that CTA's bounded wait runs out
-__device__ __forceinline__ int fast_stall_plane(const FastArgs& a) {
+__device__ __forceinline__ int fast_stall_plane(const FastArgs& a) {  // failure-path tests
   const int tid = threadIdx.y * ft::TX + threadIdx.x;
-  if (tid == ft::ISSUER && *(volatile int*)(a.err + 1) > 0) return atomicExch(a.err + 1, 0) - 1;
-  return -1;
+  if (tid != ft::ISSUER) return -1;
+  return take_stall(a.err, a.final_kind == 2 ? kStallLastSubstep : kStallSubstep);
 }
 
 // One acoustic substep: one CTA per tile and chunk of levels.

@@ -117,10 +117,7 @@ __global__ void __launch_bounds__(st::NT, 2)
   }
   __syncthreads();
 
-  // err[1] > 0 (set only by failure-path tests): the first CTA to see it leaves the loads of
-  // one of its planes unissued, so that CTA's bounded wait runs out
-  int stall = -1;
-  if (tid == ISSUER && *(volatile int*)(a.err + 1) > 0) stall = atomicExch(a.err + 1, 0) - 1;
+  int stall = tid == ISSUER ? take_stall(a.err, kStallSlow) : -1;  // failure-path tests
   if (stall >= 0) stall = kg + stall % (ke - kg + 1);
   auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * slot; };
   auto issue = [&](int kk) {  // plane kk in [kg, ke] into its slot

@@ -101,6 +101,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
   return true;
 }
 
+// Failure-path tests: a member's err[1] asks one CTA to leave the loads of one plane unissued,
+// so that its bounded wait runs out (0: no request).  The low half is the plane plus one, the
+// high half the kind of launch that is meant, or 0 for the first that looks.  The first CTA of
+// that kind takes the request; returns its plane, or -1.
+enum StallKind : int { kStallSlow = 1, kStallSubstep = 2, kStallLastSubstep = 3, kStallTracer = 4 };
+__device__ __forceinline__ int take_stall(int* err, int kind) {
+  const int word = *(volatile int*)(err + 1);
+  if (word <= 0 || ((word >> 16) != 0 && (word >> 16) != kind)) return -1;
+  return atomicCAS(err + 1, word, 0) == word ? (word & 0xffff) - 1 : -1;
+}
+
 // 3-D tiled TMA load of box (x, y, z) of `map` into shared memory `dst`,
 // completing on `bar`.  x must be a multiple of 4 (16 bytes of FP32).
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z,

@@ -282,10 +282,12 @@ int gwm_b200_surrogate_fallbacks(gwm_b200_ctx* ctx, int member, long long* count
 int gwm_b200_mlp_loss_grad(const float* params, const float* norm, const float* x, const float* y, int n,
                            float* grad, double* loss);
 /* Failure-path testing (no counterpart in the reference): the next TMA-fed stencil
- * launch of the member (slow stage, acoustic substep or tracer stage on flat terrain)
+ * launch of the member (slow stage, acoustic substep or tracer stage)
  * leaves the tile loads of `plane` unissued in one CTA, so that CTA's bounded wait runs
  * out; the step call then returns GWM_B200_ERR_TIMEOUT and the context stays usable.
- * The request is kept until a TMA-fed kernel takes it. */
+ * The request is kept until a TMA-fed kernel takes it.  65536 * kind + plane asks for a
+ * launch of one kind: 1 slow stage, 2 acoustic substep, 3 last substep of a step, 4 tracer
+ * stage. */
 int gwm_b200_test_stall_tile_load(gwm_b200_ctx* ctx, int member, int plane);
 /* FP64 budgets of the current state. */
 int gwm_b200_budgets(gwm_b200_ctx* ctx, int member, gwm_b200_budget* out);

@@ -69,3 +69,25 @@ def test_first_plane_of_a_chunk_never_arrives(gwm, op, terrain):
             out[stall] = m.download()
     for k in out[False]:
         np.testing.assert_array_equal(out[True][k], out[False][k], err_msg=k)
+
+
+# Each kernel of a step in turn: k_slow_tma, k_fast_rows (inner and last substep) and
+# k_tracer_tma on flat levels, their terrain forms on terrain.
+@pytest.mark.parametrize("plane", [0, 3])
+@pytest.mark.parametrize("terrain", [False, True])
+@pytest.mark.parametrize("kernel", ["slow_stage", "fast_substep", "last_substep", "tracer_stage"])
+def test_each_kernel_of_a_step_gives_up_and_recovers(gwm, kernel, terrain, plane):
+    grid, state, spec = _member(gwm, terrain)
+    out = {}
+    for stall in (False, True):
+        with gwm.Model(grid, spec) as m:
+            m.upload(state)
+            if stall:
+                m.test_stall_tile_load(plane=plane, kernel=kernel)
+                with pytest.raises(RuntimeError, match="status -5"):
+                    m.step(1)
+                m.upload(state)
+            m.step(1)
+            out[stall] = m.download()
+    for k in out[False]:
+        np.testing.assert_array_equal(out[True][k], out[False][k], err_msg=k)
