@@ -162,6 +162,10 @@ __device__ __forceinline__ void store_mirrored(float* __restrict__ f, const Geom
 // which kernel computed it.  Reruns, and runs with different tile choices, are
 // bitwise identical.  Scales keep the largest sums (1.6e7 cells per level) inside
 // int64.
+// The exception is a state that has blown up: a warp's total wraps at 2^56 (a mean theta of
+// 4e6 K over 32 cells, a p' of 6.7e7 Pa), so there the cells that a total covers show.  It
+// covers one row of a tile (32 cells, 30 in the overlapped tiles) in every kernel but
+// k_fast_flat and k_fast_tma, whose totals cover two rows eight apart.
 constexpr double kScaleRho = 4294967296.0;    // 2^32
 constexpr double kScaleP = 16777216.0;        // 2^24 (pressure perturbations)
 constexpr double kScaleTheta = 268435456.0;   // 2^28
@@ -206,6 +210,9 @@ __device__ __forceinline__ long long warp_total_fx(long long x) {
   const unsigned sl = __reduce_add_sync(0xffffffffu, (unsigned)(x & 0xffffffLL));
   return (long long)sh * 16777216LL + (long long)sl;
 }
+
+// A thread's sum of a few fx() that could wrap a warp total (beyond 2^49).
+__device__ __forceinline__ bool fx_wild(long long x) { return (unsigned)((int)(x >> 32) + (1 << 17)) >= (1u << 18); }
 
 __device__ __forceinline__ long long warp_sum_ll(long long v) {
 #pragma unroll

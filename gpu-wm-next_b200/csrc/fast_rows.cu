@@ -16,7 +16,7 @@
 //   - p' - p'_ref and rho - rho_ref of a level are formed once and carried up;
 //   - the level sums stay in shared memory until the CTA's end: one atomic per level.
 // 1024 x 1024 x 64: 0.549 ms a substep (0.82 of the copy bandwidth), 0.627 with k_fast_tma's
-// split columns, 0.654 with its whole columns; 517 x 389 x 50: 96 us (99.6 with a test for the
+// split columns, 0.654 with its whole columns; 517 x 389 x 50: 97 us (100 with a test for the
 // EOS's far form per row instead of one per plane), 116 with k_fast_tma.
 #include <type_traits>
 
@@ -55,6 +55,13 @@ constexpr size_t smem_bytes(int planes) {
   return size_t(Slot<FIRST, FINAL>::SIZE) * NSLOT * sizeof(float) + 128 + kLevel * size_t(planes + 2);
 }
 }  // namespace fr
+
+// A level sum's warp total row by row: in a state that has blown up the total can wrap, and the
+// cells that it covers show (common.cuh).  Rare, so a call.
+__noinline__ __device__ long long row_totals(float v0, float v1, float v2, float v3, float scale) {
+  return warp_total_fx(fx(v0, scale)) + warp_total_fx(fx(v1, scale)) + warp_total_fx(fx(v2, scale)) +
+         warp_total_fx(fx(v3, scale));
+}
 
 template <bool FIRST, int KIND>  // KIND: FastArgs::final_kind
 __global__ void __launch_bounds__(fr::NT, fr::MIN_CTAS)
@@ -331,7 +338,21 @@ __global__ void __launch_bounds__(fr::NT, fr::MIN_CTAS)
         }
         release(k);
         if (acc_mode) {
-          const long long ta = warp_total_fx(sa), tb = KIND == 0 ? warp_total_fx(sb) : 0;
+          long long ta, tb = 0;
+          if (!__any_sync(0xffffffffu, fx_wild(sa) || (KIND == 0 && fx_wild(sb)))) {
+            ta = warp_total_fx(sa);
+            if (KIND == 0) tb = warp_total_fx(sb);
+          } else {
+            float v[ROWS];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) v[r] = !own[r] ? 0.0f : KIND == 0 ? nrho[r] : fp::theta(nrho[r], nrt[r]);
+            ta = row_totals(v[0], v[1], v[2], v[3], KIND == 0 ? kFxRho : kFxTheta);
+            if (KIND == 0) {
+#pragma unroll
+              for (int r = 0; r < ROWS; ++r) v[r] = own[r] ? np[r] : 0.0f;
+              tb = row_totals(v[0], v[1], v[2], v[3], kFxP);
+            }
+          }
           if (lane == 0) {
             long long* red = t_red + 2 * (NW * (k - kb) + wid);
             red[0] = ta;

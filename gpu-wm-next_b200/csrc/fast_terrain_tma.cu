@@ -415,8 +415,7 @@ __global__ void __launch_bounds__(fz::NT, 2)
         if (acc) sum[r] = fx(fp::theta(rnew, rt), kFxTheta);
       }
       if (acc) {
-        // row by row: a warp total wraps at 2^56 (theta of 1e8 K), so in a state that has blown
-        // up the rows a total covers show, and one row is what the other kernels' totals cover
+        // row by row: in a state that has blown up a warp's total can wrap (common.cuh)
         long long t = 0;
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) t += warp_total_fx(sum[r]);

@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(st::NT, 2)
   };
 
   // cells, X faces, Y faces and Z faces of plane k in the thread's rows (+ the top faces)
-  auto columns = [&](auto tile_class, int k, const SlowBlend* q0, const TerrMetric* mt, long long& ra,
+  auto columns = [&](auto tile_class, int k, const SlowBlend* q0, const TerrMetric* mt, long long* ra,
                      const PlaneConst& kc) {
     constexpr bool IN = decltype(tile_class)::value;  // an interior tile
     // store of an owned value at plane k + up: a plain store in interior tiles, else with the
@@ -464,7 +464,7 @@ __global__ void __launch_bounds__(st::NT, 2)
         const float th1 = fp::theta(r1, q1);
         put(a.o_rho, kCell, r, 0, r1);
         put(a.o_th, kCell, r, 0, a.out_rt ? q1 : th1);
-        if (a.acc_mode == 2 && (IN || own_rt[r])) ra += fx(th1, kFxTheta);
+        if (a.acc_mode == 2 && (IN || own_rt[r])) ra[r] = fx(th1, kFxTheta);
       }
     }
     // ---- X faces: K17 (dry_momentum_flux.cu:79-156) + K21 (dry_pressure_gradient.cu:75-123)
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(st::NT, 2)
         if (k + 2 <= ke) { issue(k + 2); issued = k + 2; }
       }
       // ---- cells and faces of plane k
-      long long ra = 0;
+      long long ra[ROWS] = {0, 0};
       columns(tile_class, k, q0, mt, ra, kc);
       if (!IN && xf) {  // open east boundary: X face nx of row j0+tx
         const float* sr = slot_at(k);
@@ -630,7 +630,8 @@ __global__ void __launch_bounds__(st::NT, 2)
         store_tile(a.o_v, g, kFaceY, i0 + tx, ny, k, v1, edge);
       }
       if (a.acc_mode) {
-        const long long ta = warp_total_fx(ra);
+        // row by row: in a state that has blown up a warp's total can wrap (common.cuh)
+        const long long ta = warp_total_fx(ra[0]) + warp_total_fx(ra[1]);
         if (tx == 0) s_red[pb][ty] = ta;
       }
 #pragma unroll

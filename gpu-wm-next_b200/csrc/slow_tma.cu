@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
   };
 
   // cells, X faces, Y faces and Z faces of plane k in the thread's rows (+ the top faces)
-  auto columns = [&](auto tile_class, int k, const SlowBlend* q0, long long& ra, long long& rb,
+  auto columns = [&](auto tile_class, int k, const SlowBlend* q0, long long* ra, long long* rb,
                      const PlaneConst& kc) {
     constexpr bool IN = decltype(tile_class)::value;  // an interior tile
     // store of an owned value at plane k + up: a plain store in interior tiles, else with the
@@ -443,14 +443,14 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
 #pragma unroll
         for (int r = 0; r < ROWS; ++r)
           if (IN || own_rt[r]) {
-            ra += fx(ro[r], kFxRho);
-            rb += fx(pv[r], kFxP);
+            ra[r] = fx(ro[r], kFxRho);
+            rb[r] = fx(pv[r], kFxP);
             if (a.p_out) put(a.p_out, kCell, r, 0, pv[r]);
           }
       } else if (acc_mode == 2) {
 #pragma unroll
         for (int r = 0; r < ROWS; ++r)
-          if (IN || own_rt[r]) ra += fx(to[r], kFxTheta);
+          if (IN || own_rt[r]) ra[r] = fx(to[r], kFxTheta);
       }
     }
     // ---- X faces: K17 (dry_momentum_flux.cu:79-156) + K21 (dry_pressure_gradient.cu:75-123)
@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         if (k + 2 <= ke) { issue(k + 2); issued = k + 2; }
       }
       // ---- cells and faces of plane k
-      long long ra = 0, rb = 0;
+      long long ra[ROWS] = {0, 0}, rb[ROWS] = {0, 0};
       columns(tile_class, k, q0, ra, rb, kc);
       if (!IN && xf) {  // open east boundary: X face nx of row j0+tx
         const float* sr = slot_at(k);
@@ -614,7 +614,9 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         store_tile(a.o_v, g, kFaceY, i0 + tx, ny, k, v1, edge);
       }
       if (acc_mode) {
-        const long long ta = warp_total_fx(ra), tb = warp_total_fx(rb);
+        // row by row: in a state that has blown up a warp's total can wrap (common.cuh)
+        const long long ta = warp_total_fx(ra[0]) + warp_total_fx(ra[1]);
+        const long long tb = acc_mode == 1 ? warp_total_fx(rb[0]) + warp_total_fx(rb[1]) : 0;
         if (tx == 0) { s_red[pb][ty][0] = ta; s_red[pb][ty][1] = tb; }
       }
 #pragma unroll

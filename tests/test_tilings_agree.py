@@ -1,0 +1,34 @@
+"""Every tiling of a kernel computes the same values, also where the values leave the range
+that a forecast lives in: there the kernels' general forms run."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = ("slow_stage", "fast_substep", "tracer_stage")
+
+
+def _step_with(gwm, grid, spec, state, rows, run=lambda m: m.step(1)):
+    with gwm.Model(grid, spec) as m:
+        for kernel in KERNELS:
+            m.set_tile(kernel, rows)
+        m.upload(state)
+        run(m)
+        return m.download()
+
+
+# Two neighbouring cells whose p' (theta of 4e5 K: 0.7 of the 2^31 Pa at which a total wraps) or
+# theta (1e8 K: 0.75 of the 2^27 K) only together leave the range of a warp's total.
+@pytest.mark.parametrize("fast", [True, False])
+@pytest.mark.parametrize("theta", [4.0e5, 1.0e8])
+@pytest.mark.parametrize("row", [4, 17])
+def test_wild_cells_in_adjacent_rows(gwm, row, theta, fast):
+    grid = gwm.GridSpec(96, 48, 12, dx=1000.0, dy=1000.0, z_top=6000.0)
+    state = gwm.build_case("moist_sounding", grid, gwm.CaseParams(theta_ref=300.0, noise_rms_k=0.5, seed=3))
+    for j in (row, row + 1):
+        state["rho_theta"][5, j, 40] = state["rho"][5, j, 40] * np.float32(theta)
+    spec = gwm.MemberSpec(step=gwm.StepConfig(dt=1.0e-4, fast_substeps=3, enable_fast_modes=fast))
+    a, b = (_step_with(gwm, grid, spec, state, rows) for rows in (16, 3))
+    assert np.isfinite(a["w"]).all()
+    for k in a:
+        np.testing.assert_array_equal(b[k], a[k], err_msg=k)
