@@ -62,7 +62,8 @@ __device__ __forceinline__ SlowCol slow_derive(const SlowArgs& a, const SlowRaw&
   if (kk < a.g.nz) {
     c.rho = r.rho;
     c.rt = a.th_is_rt ? r.t : fp::mul(c.rho, r.t);
-    c.th = fp::theta(c.rho, c.rt);
+    const float rr = fmaxf(c.rho, 1.0e-6f);
+    c.th = fp::quotient(c.rt, rr, fp::recip(rr));
     c.p = TERRAIN ? eos_pressure(c.rho, c.rt) : eos_pprime(c.rho, c.rt, a.base, kk, a.g.nz);
     c.uf = fp::add(r.u, r.du);
     c.vf = fp::add(r.v, r.dv);
@@ -151,10 +152,10 @@ __global__ void __launch_bounds__(BX * SBY) k_slow_stage(const SlowArgs a) {
     }
     // cell-centred velocities of plane k, halo included: dry_momentum_flux.cu:36-73
     {
-      const float rr = fmaxf(cc.rho, 1.0e-6f);
-      s_uc[pb][ty][tx] = (tx + 1 < BX) ? fp::centred(cc.uf, s_u[pb][ty][tx + 1], rr) : 0.0f;
-      s_vc[pb][ty][tx] = (ty + 1 < SBY) ? fp::centred(cc.vf, s_v[pb][ty + 1][tx], rr) : 0.0f;
-      s_wc[pb][ty][tx] = fp::centred(cc.wf, cn.wf, rr);
+      const float rr = fmaxf(cc.rho, 1.0e-6f), y = fp::recip(rr);
+      s_uc[pb][ty][tx] = (tx + 1 < BX) ? fp::centred(cc.uf, s_u[pb][ty][tx + 1], rr, y) : 0.0f;
+      s_vc[pb][ty][tx] = (ty + 1 < SBY) ? fp::centred(cc.vf, s_v[pb][ty + 1][tx], rr, y) : 0.0f;
+      s_wc[pb][ty][tx] = fp::centred(cc.wf, cn.wf, rr, y);
     }
     __syncthreads();
 

@@ -33,9 +33,9 @@ __device__ __forceinline__ TrCol tr_load(const TracerArgs& a, bool valid, int ba
 }
 
 __device__ __forceinline__ void tr_mix(TrCol& c) {
-  const float rr = fmaxf(c.rho, 1.0e-6f);
+  const float rr = fmaxf(c.rho, 1.0e-6f), y = fp::recip(rr);
 #pragma unroll
-  for (int t = 0; t < NTR; ++t) c.q[t] = c.rq[t] / rr;  // mixing ratio: dry_transport.cu:91-94
+  for (int t = 0; t < NTR; ++t) c.q[t] = fp::quotient(c.rq[t], rr, y);  // mixing ratio: dry_transport.cu:91-94
 }
 
 template <int TBY>
@@ -168,8 +168,7 @@ __global__ void __launch_bounds__(32 * kRW) k_warm_rain(const RainArgs a) {
         // a / max(rho, 1e-6) of several a by one reciprocal
         const float rr = fmaxf(rho_d, 1.0e-6f), y = fp::recip(rr);
         auto quotient = [&](float v) {
-          const float t = fp::div_by(v, rr, y);
-          return fp::finite(t) ? t : fp::div(v, rr);
+          return fp::quotient(v, rr, y);
         };
         if (MICRO) {  // warm_rain_kernel: warm_rain.cu:36-120
           MicroCell mc;

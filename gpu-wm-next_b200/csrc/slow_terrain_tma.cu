@@ -242,12 +242,12 @@ __global__ void __launch_bounds__(st::NT, 2)
         if ((IN && n < FULL) || live & (256u << n)) p_c[n] = pressure(rho, t, near);
       }
     }
-    if (!near) {  // a value that is not finite: the plain forms
+    if (!near) {  // a value that is not finite: each one tested
 #pragma unroll
       for (int n = 0; n < NP; ++n)
         if (live & (1u << n)) {
           const float rho = sr[R_RHO + pos_b[n]], rt = RT(sr, pos_b[n], rho);
-          th[tid + n * NT] = fp::theta(rho, rt);
+          th[tid + n * NT] = fp::quotient_far(rt, fmaxf(rho, 1.0e-6f));
           if (live & (256u << n)) p_c[n] = eos_pressure(rho, rt);
         }
     }
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(st::NT, 2)
         vc[q] = cv;
         wc[q] = cw;
       }
-    if (!near) {  // a quotient that is not finite: plain divisions
+    if (!near) {  // a quotient that is not finite: each one tested
 #pragma unroll 1
       for (int n = 0; n < NP; ++n) {
         if (!(live & (256u << n))) continue;
@@ -292,9 +292,9 @@ __global__ void __launch_bounds__(st::NT, 2)
         const float rr = fmaxf(sr[R_RHO + b], 1.0e-6f);
         float mu, mv, mw;
         momenta(b, mu, mv, mw);
-        uc[q] = fp::div(mu, rr);
-        vc[q] = fp::div(mv, rr);
-        wc[q] = fp::div(mw, rr);
+        uc[q] = fp::quotient_far(mu, rr);
+        vc[q] = fp::quotient_far(mv, rr);
+        wc[q] = fp::quotient_far(mw, rr);
       }
     }
     float below[NP];  // the pressure at plane k-1

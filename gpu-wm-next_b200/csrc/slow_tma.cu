@@ -228,12 +228,12 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         near = near && fp::finite(t);
         th[tid + n * NT] = t;
       }
-    if (!near) {  // a quotient that is not finite: plain divisions
+    if (!near) {  // a quotient that is not finite: each one tested
 #pragma unroll
       for (int n = 0; n < NP; ++n)
         if (live & (1u << n)) {
           const float rho = sr[R_RHO + pos_b[n]];
-          th[tid + n * NT] = fp::theta(rho, RT(sr, pos_b[n], rho));
+          th[tid + n * NT] = fp::quotient_far(RT(sr, pos_b[n], rho), fmaxf(rho, 1.0e-6f));
         }
     }
   };
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         vc[q] = cv;
         wc[q] = cw;
       }
-    if (!near) {  // far from the base state, or a quotient that is not finite: the plain forms
+    if (!near) {  // far from the base state, or a quotient that is not finite: each one tested
 #pragma unroll 1
       for (int n = 0; n < NP; ++n) {
         if (!(live & (256u << n))) continue;
@@ -278,9 +278,9 @@ __global__ void __launch_bounds__(sl::NT, 2) k_slow_tma(const SlowArgs a, const 
         pp[q] = eos_pprime_ref(rho, RT(sr, b, rho), binv, bpr);
         float mu, mv, mw;
         momenta(b, mu, mv, mw);
-        uc[q] = fp::div(mu, rr);
-        vc[q] = fp::div(mv, rr);
-        wc[q] = fp::div(mw, rr);
+        uc[q] = fp::quotient_far(mu, rr);
+        vc[q] = fp::quotient_far(mv, rr);
+        wc[q] = fp::quotient_far(mw, rr);
       }
     }
   };

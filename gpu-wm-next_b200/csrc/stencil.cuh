@@ -5,7 +5,8 @@
 // functions.  Each operation rounds on its own (__fadd_rn, __fmul_rn, ...) and an FMA is
 // used only where written, so the compiler cannot contract the same expression
 // differently in two kernels or two copies of a loop: the variants agree bit for bit by
-// construction.  The formulas and constants are the reference's (file:line per function);
+// construction.  (The level means of a state that has blown up are the exception, see
+// common.cuh.)  The formulas and constants are the reference's (file:line per function);
 // the FMAs are placed where a multiply feeds an add, the contraction a CUDA build of the
 // reference makes of the same expressions.
 //
@@ -35,7 +36,10 @@ __device__ __forceinline__ float div(float a, float b) { return __fdiv_rn(a, b);
 // Dev. 34, 1990, theorem 8.3): the value of div(a, b), five operations each instead of a
 // division.  It holds where the residuals neither overflow nor underflow; for b in [1e-6,
 // 1e6] that is a = 0 or 2^-79 <= |a| <= 2^100.  Smaller |a| may be one ulp off (of values
-// below 1e-18); the callers send quotients that are not finite to div().
+// below 1e-18, the tails of momenta and tracers), and -0 gives +0.  So every variant of an
+// operator takes quotient(), the residual form unless that is not finite; kernels that test
+// several quotients at once redo them all with it.  (Testing for small |a| instead costs the
+// TMA-fed slow stage 2 % and the tracer stage 1 to 4 %.)
 __device__ __forceinline__ float recip(float b) { return __frcp_rn(b); }
 __device__ __forceinline__ float div_by(float a, float b, float y) {
   const float q0 = __fmul_rn(a, y);
@@ -43,6 +47,12 @@ __device__ __forceinline__ float div_by(float a, float b, float y) {
   return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
 }
 __device__ __forceinline__ bool finite(float a) { return fabsf(a) < __int_as_float(0x7f800000); }
+__device__ __forceinline__ float quotient(float a, float b, float y) {
+  const float q = div_by(a, b, y);
+  return finite(q) ? q : div(a, b);
+}
+// The same as a call, for the paths that are rarely taken.
+static __noinline__ __device__ float quotient_far(float a, float b) { return quotient(a, b, recip(b)); }
 __device__ __forceinline__ float neg(float a) { return -a; }
 __device__ __forceinline__ float vmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float select_ge0(float a, float x, float y) { return a >= 0.0f ? x : y; }
@@ -78,8 +88,9 @@ template <class V> __device__ __forceinline__ V blend(float wa, V q0, float wb, 
 // theta = rho_theta / max(rho, 1e-6) (include/gwm/core/dry_thermo.hpp:21-24).
 template <class V> __device__ __forceinline__ V theta(V rho, V rt) { return div(rt, vmax(rho, sc<V>(1.0e-6f))); }
 
-// Cell-centred velocity 0.5 (m_a + m_b) / max(rho, 1e-6) (dry_momentum_flux.cu:36-73).
-template <class V> __device__ __forceinline__ V centred(V ma, V mb, V rr) { return div(avg(ma, mb), rr); }
+// Cell-centred velocity 0.5 (m_a + m_b) / max(rho, 1e-6) (dry_momentum_flux.cu:36-73), from the
+// floored density rr and its reciprocal y.
+template <class V> __device__ __forceinline__ V centred(V ma, V mb, V rr, V y) { return quotient(avg(ma, mb), rr, y); }
 
 // ---- acoustic substep (dry_fast_modes.cu:160-394) --------------------------------
 // K12/K13 horizontal momentum increment on flat levels: d - dtf (p_r - p_l) inv_d.
@@ -136,18 +147,20 @@ template <class V> __device__ __forceinline__ V add_damping(V t, float rate, V q
 // two cells and trf the face mean of the two level means theta_ref.
 template <class V>
 __device__ __forceinline__ V add_buoyancy(V t, V th_l, V th_u, float trf, V rho_l, V rho_u, float gravity) {
-  const V b = div(mul(sc<V>(gravity), sub(avg(th_l, th_u), sc<V>(trf))), sc<V>(fmaxf(trf, 1.0e-6f)));
+  const V b = quotient_far(mul(sc<V>(gravity), sub(avg(th_l, th_u), sc<V>(trf))), sc<V>(fmaxf(trf, 1.0e-6f)));
   return fma(avg(rho_l, rho_u), b, t);
 }
 // With the level means themselves.
 template <class V>
 __device__ __forceinline__ V add_buoyancy(V t, V th_l, V th_u, float tref_l, float tref_u, V rho_l, V rho_u,
                                           float gravity) {
-  return add_buoyancy(t, th_l, th_u, __fmul_rn(0.5f, __fadd_rn(tref_l, tref_u)), rho_l, rho_u, gravity);
+  const float trf = __fmul_rn(0.5f, __fadd_rn(tref_l, tref_u)), d = fmaxf(trf, 1.0e-6f);
+  const V b = quotient(mul(sc<V>(gravity), sub(avg(th_l, th_u), sc<V>(trf))), sc<V>(d), sc<V>(recip(d)));
+  return fma(avg(rho_l, rho_u), b, t);
 }
 
 // The same with the face mean of the level means, trf, and the reciprocal of its floored
-// value at hand (one pair per level); `near` is cleared where the plain form is due.
+// value at hand (one pair per level); `near` is cleared where the form above is due.
 __device__ __forceinline__ float add_buoyancy_ref(float t, float th_l, float th_u, float trf, float ytrf, float rho_l,
                                                   float rho_u, float gravity, bool& near) {
   const float n = mul(gravity, sub(avg(th_l, th_u), trf)), d = fmaxf(trf, 1.0e-6f);

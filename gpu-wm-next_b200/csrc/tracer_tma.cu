@@ -12,7 +12,7 @@
 //   w                                 32 x 16 box: owned Z faces (plane nz: w only)
 // A thread computes the mixing ratios of its rows one plane ahead and those of the rows around
 // them, and a position of the warp's two ring columns, with one reciprocal per position; all of
-// a plane's come first, with one test for the quotients that need a plain division, so their
+// a plane's come first, with one test for quotients that are not finite, so their
 // chains interleave.  The Y fluxes between its rows are computed once, and the flux out of a
 // plane's top is carried as the next plane's bottom flux.  Bounds: issue, close to HBM (13
 // fields of 4 B per cell take 0.53 ms for 1024 x 1024 x 64, three tracers, at the copy
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
   };
   auto slot_at = [&](int kk) { return ring + ((kk - kg) % NSLOT) * SLOT; };
   // mixing ratios (dry_transport.cu:91-94) at position b of a plane's cell boxes; `near` is
-  // cleared where one is not finite and the plain divisions are due
+  // cleared where one is not finite and each is to be tested
   auto mix_near = [&](const float* st, int b, float* q, bool& near) {
     const float rr = fmaxf(st[O_RHO + b], 1.0e-6f), y = fp::recip(rr);
     float sum = 0.0f;
@@ -139,15 +139,15 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
     }
     near = near && fp::finite(sum);
   };
-  auto mix_plain = [&](const float* st, int b, float* q) {
-    const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
+  auto mix_each = [&](const float* st, int b, float* q) {
+    const float rr = fmaxf(st[O_RHO + b], 1.0e-6f), y = fp::recip(rr);
 #pragma unroll
-    for (int t = 0; t < N; ++t) q[t] = fp::div(st[O_Q + t * Q_STRIDE + b], rr);
+    for (int t = 0; t < N; ++t) q[t] = fp::quotient(st[O_Q + t * Q_STRIDE + b], rr, y);
   };
   auto mix = [&](const float* st, int b, float* q) {
     bool near = true;
     mix_near(st, b, q, near);
-    if (!near) mix_plain(st, b, q);
+    if (!near) mix_each(st, b, q);
   };
 
   auto run = [&](auto tile_class) -> bool {  // false when a bounded wait gave up
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
         for (int t = 0; t < N; ++t) q0[r][t] = BLEND && own[r] ? __ldg(a.q0[t] + off[r]) : 0.f;
       }
       // the mixing ratios of the rows around the warp's and of its ring columns (a position per
-      // lane), and of its rows at plane k+1: one test for the plain divisions
+      // lane), and of its rows at plane k+1: one test for quotients that are not finite
       const bool top = k + 1 == nz;
       float qs[N], qn[N], qr[N], qt[ROWS][N];
       bool near = true;
@@ -217,12 +217,12 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
         for (int r = 0; r < ROWS; ++r) mix_near(sn, b0 + r * CBW, qt[r], near);
       }
       if (!near) {
-        mix_plain(st, b0 - CBW, qs);
-        mix_plain(st, b0 + ROWS * CBW, qn);
-        mix_plain(st, ring_b, qr);
+        mix_each(st, b0 - CBW, qs);
+        mix_each(st, b0 + ROWS * CBW, qn);
+        mix_each(st, ring_b, qr);
         if (!top) {
 #pragma unroll
-          for (int r = 0; r < ROWS; ++r) mix_plain(sn, b0 + r * CBW, qt[r]);
+          for (int r = 0; r < ROWS; ++r) mix_each(sn, b0 + r * CBW, qt[r]);
         }
       }
       if (top) {

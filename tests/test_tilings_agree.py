@@ -32,3 +32,31 @@ def test_wild_cells_in_adjacent_rows(gwm, row, theta, fast):
     assert np.isfinite(a["w"]).all()
     for k in a:
         np.testing.assert_array_equal(b[k], a[k], err_msg=k)
+
+
+# Tracers in the range that upwind transport's tails leave (residuals of the quotient by one
+# reciprocal underflow there), zeros of either sign, and a wind that moves a third of a cell a step.
+@pytest.mark.parametrize("low,high", [(-149.0, -130.0), (-125.0, -105.0)])
+@pytest.mark.parametrize("terrain", [False, True])
+def test_tails_of_tracers(gwm, terrain, low, high):
+    nx, ny, nz = 70, 37, 14
+    hill = None
+    if terrain:
+        hill = gwm.build_terrain("cosine_mountain", nx, ny, 1000.0, 1000.0, height=300.0, half_width_x=0.3,
+                                 half_width_y=0.3)
+    flat = gwm.GridSpec(nx, ny, nz, dx=1000.0, dy=1000.0, z_top=300.0 * nz)
+    grid = gwm.GridSpec(nx, ny, nz, dx=1000.0, dy=1000.0, z_top=300.0 * nz, terrain=hill)
+    state = gwm.build_case("moist_sounding", flat, gwm.CaseParams(theta_ref=300.0, noise_rms_k=0.5, seed=3,
+                                                                  relative_humidity=1.01), moist=True)
+    rng = np.random.default_rng(2)
+    state["u"] = (rng.uniform(50.0, 150.0, state["u"].shape)).astype(np.float32)
+    state["u"][:, :, -1] = state["u"][:, :, 0]
+    for k in ("qv", "qc", "qr"):
+        v = np.exp2(rng.uniform(low, high, state[k].shape))
+        v[rng.random(v.shape) < 0.05] = -0.0
+        state[k] = v.astype(np.float32)
+    state["precip"] = np.zeros((ny, nx))
+    spec = gwm.MemberSpec(step=gwm.StepConfig(dt=3.0, fast_substeps=3), moist=True)
+    a, b = (_step_with(gwm, grid, spec, state, rows, lambda m: m.advance_passive_tracers_ssprk3()) for rows in (16, 3))
+    for k in a:
+        np.testing.assert_array_equal(b[k], a[k], err_msg=k)
