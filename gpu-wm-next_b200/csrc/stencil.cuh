@@ -177,7 +177,11 @@ __device__ __forceinline__ float add_buoyancy_ref(float t, float th_l, float th_
 // repeats, and the final density is then the one just evaluated, so the third iteration and
 // the fourth stop there with the same result (the iterations contract by about
 // g dz / (2 c^2) ~ 1e-2, so the first two are never the last).
-__device__ __forceinline__ float eos_rho_of(float p, float rdth) {  // density of p with Rd*theta at hand
+// Density of a finite p with Rd*theta at hand.  Only the lowest level's p can be infinite: its
+// density is then NaN, and the level above takes the floor of the pressure (fmaxf takes the
+// number).  So that level divides, and the chains of the others stay short (a test here took
+// 512 x 512 x 80 from 0.326 to 0.334 ms).
+__device__ __forceinline__ float eos_rho_of(float p, float rdth) {
   const float x = div_by(p, kP0, 1.0f / kP0);
   return p / fmaxf(rdth * powf(fmaxf(x, 1.0e-6f), kKappa), 1.0e-6f);
 }
@@ -186,7 +190,7 @@ __device__ __forceinline__ void column_reference_level(int k, float rho, float r
   const float rdth = kRd * theta(rho, rt);
   if (k == 0) {
     pref = eos_pressure(rho, rt);
-    rref = eos_rho_of(pref, rdth);
+    rref = pref / fmaxf(rdth * powf(fmaxf(pref / kP0, 1.0e-6f), kKappa), 1.0e-6f);
   } else {
     const float dzk = z - zb, hg = mul(gravity, 0.5f);
     auto next = [&](float rn) { return fmaxf(fma(-mul(hg, add(rref, rn)), dzk, pref), 1.0f); };
