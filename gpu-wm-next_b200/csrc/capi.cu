@@ -445,7 +445,9 @@ int alloc_member(gwm_b200_ctx* c, Member& M) {
 constexpr int kFastTma = 3;  // fast_tile_rows value selecting the TMA-fed substep
 // fast_tile_rows value selecting the TMA-fed substeps of a stage in one persistent launch
 constexpr int kFastStage = 4;
-bool fast_tma_path(const gwm_b200_ctx* c) { return c->fast_tile_rows == kFastTma || c->fast_tile_rows == kFastStage; }
+bool fast_rows_known(long r) { return r == 0 || r == kFastTma || r == kFastStage || r == 8 || r == 16; }
+bool fast_rows_tma(int r) { return r == kFastTma || r == kFastStage; }  // these need tensor maps
+bool fast_tma_path(const gwm_b200_ctx* c) { return fast_rows_tma(c->fast_tile_rows); }
 constexpr int kSlowTma = 3;  // slow_tile_rows value selecting the TMA-fed slow stage
 constexpr int kTracerTma = 3;  // tracer_tile_rows value selecting the TMA-fed tracer stage
 
@@ -951,8 +953,12 @@ int gwm_b200_create(const gwm_b200_grid_desc* grids, const gwm_b200_member_desc*
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return GWM_B200_ERR_NO_DEVICE;
   auto* c = new gwm_b200_ctx();
-  const char* fast_rows = std::getenv("GWM_B200_FAST_TILE_ROWS");
-  if (fast_rows) { const int r = std::atoi(fast_rows); c->fast_tile_rows = (r == 8 || r == 16) ? r : 0; }
+  int fast_rows = -1;  // the acoustic tile asked for, if any
+  if (const char* text = std::getenv("GWM_B200_FAST_TILE_ROWS")) {
+    char* end = nullptr;
+    const long r = std::strtol(text, &end, 10);
+    if (end != text && fast_rows_known(r)) fast_rows = (int)r;
+  }
   cudaError_t e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) { delete c; return GWM_B200_ERR_CUDA; }
   c->stream = c->own_stream;
@@ -1001,8 +1007,9 @@ int gwm_b200_create(const gwm_b200_grid_desc* grids, const gwm_b200_member_desc*
   // split over CTAs they are the fastest form at every grid size (autotune can still choose).
   bool tma = true;
   for (const auto& M : c->m) tma = tma && !M.tmaps.empty();
+  if (fast_rows >= 0 && (tma || !fast_rows_tma(fast_rows))) c->fast_tile_rows = fast_rows;
+  else if (tma) c->fast_tile_rows = kFastTma;
   if (tma) {
-    if (!fast_rows) c->fast_tile_rows = kFastTma;
     c->slow_tile_rows = kSlowTma;
     c->tracer_tile_rows = kTracerTma;
   }
@@ -1065,11 +1072,11 @@ long long gwm_b200_launch_count(const gwm_b200_ctx* c) { return c ? c->launches 
 
 int gwm_b200_set_tile(gwm_b200_ctx* c, int kernel, int rows) {
   if (!c) return GWM_B200_ERR_ARG;
-  const bool ok = kernel == 1   ? (rows == 0 || rows == kFastTma || rows == kFastStage || rows == 8 || rows == 16)
+  const bool ok = kernel == 1   ? fast_rows_known(rows)
                   : kernel == 0 ? (rows == kSlowTma || rows == 8 || rows == 16)
                                 : kernel == 2 && (rows == kTracerTma || rows == 8 || rows == 16);
   if (!ok) return GWM_B200_ERR_ARG;
-  if ((kernel == 1 && (rows == kFastTma || rows == kFastStage)) || (kernel == 0 && rows == kSlowTma) ||
+  if ((kernel == 1 && fast_rows_tma(rows)) || (kernel == 0 && rows == kSlowTma) ||
       (kernel == 2 && rows == kTracerTma))
     for (const auto& M : c->m)
       if (M.tmaps.empty())

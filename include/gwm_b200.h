@@ -373,8 +373,9 @@ int gwm_b200_plan_view_json(gwm_b200_ctx* ctx, int member, int level, const char
  * tiles of 8 rows), 4 = the same tiles with all the substeps of an RK stage in
  * one persistent cooperative launch (a bounded grid barrier between substeps; the
  * step's last substep keeps its own launch; terrain runs one launch per substep), 8 or
- * 16 = overlapped 32-wide tiles of that many rows.  The environment variable GWM_B200_FAST_TILE_ROWS sets the
- * acoustic default at context creation.  The choice changes speed only: every tiling
+ * 16 = overlapped 32-wide tiles of that many rows.  The environment variable
+ * GWM_B200_FAST_TILE_ROWS sets the acoustic tile at context creation (0, 3, 4, 8 or 16; 3 and 4
+ * where there are descriptors; any other text leaves the default).  The choice changes speed only: every tiling
  * computes the same values.  gwm_b200_get_tile returns the current rows (or < 0). */
 int gwm_b200_set_tile(gwm_b200_ctx* ctx, int kernel, int rows);
 int gwm_b200_get_tile(const gwm_b200_ctx* ctx, int kernel);
