@@ -72,22 +72,34 @@ inline ZSplit z_split_search(unsigned tiles, int nz, int slots, float extra) {
   }
   return best;
 }
-// The same with the last results kept (they depend on the arguments alone).
-inline ZSplit z_split(unsigned tiles, int nz, int ctas_per_sm, float extra) {
+// Results kept: they depend on the arguments alone.  256 of them, in sets of four: an ensemble of
+// uneven members asks for a handful per member and step, and a search takes 2.5 to 6 us.
+struct SplitMemo {
   struct Entry {
     unsigned tiles = 0;
     int nz = 0, slots = 0;
     float extra = 0.0f;
     ZSplit s{};
   };
-  thread_local Entry memo[16];
-  thread_local unsigned next = 0;
-  const int slots = sm_count() * ctas_per_sm;
-  for (const Entry& e : memo)
-    if (e.tiles == tiles && e.nz == nz && e.slots == slots && e.extra == extra) return e.s;
-  Entry& e = memo[next++ % 16];
-  e = Entry{tiles, nz, slots, extra, z_split_search(tiles, nz, slots, extra)};
-  return e.s;
+  static constexpr unsigned kSets = 64, kWays = 4;
+  Entry entry[kSets][kWays];
+  unsigned char next[kSets] = {};  // the way of a set that is replaced next
+  unsigned searches = 0;
+  ZSplit get(unsigned tiles, int nz, int slots, float extra) {
+    const unsigned h = (tiles * 0x9e3779b1u) ^ ((unsigned)nz * 0x85ebca77u) ^ ((unsigned)slots * 0xc2b2ae3du) ^
+                       ((unsigned)(extra * 1024.0f) * 0x27d4eb2fu);
+    const unsigned set = h >> 26;
+    for (const Entry& e : entry[set])
+      if (e.tiles == tiles && e.nz == nz && e.slots == slots && e.extra == extra) return e.s;
+    ++searches;
+    Entry& e = entry[set][next[set]++ % kWays];
+    e = Entry{tiles, nz, slots, extra, z_split_search(tiles, nz, slots, extra)};
+    return e.s;
+  }
+};
+inline ZSplit z_split(unsigned tiles, int nz, int ctas_per_sm, float extra) {
+  thread_local SplitMemo memo;
+  return memo.get(tiles, nz, sm_count() * ctas_per_sm, extra);
 }
 
 }  // namespace gwmb
