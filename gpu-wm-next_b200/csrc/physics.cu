@@ -3,6 +3,7 @@
 #include "dycore.cuh"
 #include "physics.cuh"
 #include "stencil.cuh"
+#include "zsplit.cuh"
 #include "rain_cell.cuh"
 
 namespace gwmb {
@@ -264,7 +265,8 @@ cudaError_t launch_warm_rain(const RainArgs& a, cudaStream_t s, bool micro) {
   if (a.g.nz > kMaxNz) return cudaErrorInvalidValue;
   // enough CTAs for two waves of four per SM decide how much of the CTA goes along the row
   const int nseg = (a.g.nx + 31) / 32 * a.g.ny;
-  const int wx = nseg >= 4 * 148 * 8 ? 4 : nseg >= 2 * 148 * 8 ? 2 : 1;
+  const int wave = 8 * sm_count();
+  const int wx = nseg >= 4 * wave ? 4 : nseg >= 2 * wave ? 2 : 1;
   const dim3 grid((a.g.nx + 32 * wx - 1) / (32 * wx), a.g.ny);
   if (!micro && !a.fallout_mode && !a.th_acc) return cudaSuccess;
   switch (wx) {
