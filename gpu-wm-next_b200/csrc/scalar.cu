@@ -66,10 +66,11 @@ __global__ void __launch_bounds__(32 * kSWarps) k_scalar_step(const ScalarStep a
     return n < rows && inside(j) ? __ldg(col + (size_t)wrap(j, a.ny) * a.nx) : 0.0f;
   };
   const float ydx = fp::recip(a.dx), ydy = fp::recip(a.dy);
-  // 0, or a magnitude in [2^-79, 2^100]
+  // +0 (div_by loses the sign of -0), or a magnitude in [2^-79, 2^100]; on the value rotated by
+  // its sign, which costs nothing (testing it beside the magnitude: 5 % of the kernel)
   auto residual_safe = [](float e) {
-    const unsigned x = __float_as_uint(e) & 0x7fffffffu;
-    return x == 0u || x - 0x18000000u <= 0x71800000u - 0x18000000u;
+    const unsigned x = __float_as_uint(e), r = (x << 1) | (x >> 31);
+    return r == 0u || r - 0x30000000u <= 0xe3000001u - 0x30000000u;
   };
   // the reference build's contractions of q - dt*(u*dqx + v*dqy) and wa*a + wb*b
   auto stage = [&](float q, float qy) {
