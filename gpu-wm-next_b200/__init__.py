@@ -31,8 +31,9 @@ DRIVER_PATH = os.path.join(_HERE, "_build", "gwm_b200_idealized_driver")
 _DRIVER_SRC = os.path.join(_HERE, "drivers", "gwm_b200_idealized_driver.cpp")
 _SOURCES = ["capi.cu", "dycore.cu", "fast_tma.cu", "fast_rows.cu", "fast_terrain_tma.cu", "slow_tma.cu", "slow_terrain_tma.cu",
             "tracer_tma.cu",
-            "physics.cu", "halo.cu", "plan_view.cu", "surrogate.cu", "surrogate_rain.cu", "scalar.cu", "cases.cpp"]
-_HEADERS = ["common.cuh", "stencil.cuh", "dycore.cuh", "physics.cuh", "halo.cuh", "tma.cuh", "zsplit.cuh", "plan_view.cuh", "rain_cell.cuh", "surrogate.cuh", "surrogate_rain.cuh"]
+            "physics.cu", "halo.cu", "plan_view.cu", "surrogate.cu", "surrogate_rain.cu", "scalar.cu", "device_memory.cpp",
+            "cases.cpp"]
+_HEADERS = ["common.cuh", "stencil.cuh", "dycore.cuh", "physics.cuh", "halo.cuh", "tma.cuh", "zsplit.cuh", "device_memory.cuh", "plan_view.cuh", "rain_cell.cuh", "surrogate.cuh", "surrogate_rain.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "-t", "4"]
 

@@ -30,6 +30,7 @@
 
 #include "../../include/gwm_b200.h"
 #include "common.cuh"
+#include "device_memory.cuh"
 #include "dycore.cuh"
 #include "halo.cuh"
 #include "physics.cuh"
@@ -368,13 +369,7 @@ int alloc_member(gwm_b200_ctx* c, Member& M) {
                        3 * 4 * (kMaxNz + 1) * sizeof(float) + 3 * kMaxNz * sizeof(double) + 512 +
                        4 * (kMaxNz + 1) * sizeof(float) + 256 + 256;
   const size_t total = nfields * fbytes + extra;
-  cudaError_t em = cudaMalloc(&M.block, total);
-  if (em == cudaErrorMemoryAllocation) {  // once more without the scratch kept between calls
-    cudaGetLastError();
-    trim_scalar_scratch();
-    em = cudaMalloc(&M.block, total);
-  }
-  CK(em);
+  CK(device_alloc(&M.block, total));
   CK(cudaMemsetAsync(M.block, 0, total, c->stream));
   char* p = M.block;
   auto take = [&](size_t bytes) { char* r = p; p += ((bytes + 255) / 256) * 256; return r; };
@@ -1035,7 +1030,7 @@ void gwm_b200_destroy(gwm_b200_ctx* c) {
   for (auto ev : c->mjoin) cudaEventDestroy(ev);
   if (c->mfork) cudaEventDestroy(c->mfork);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
-  trim_scalar_scratch();
+  trim_scratch();
   delete c;
 }
 
@@ -1145,7 +1140,7 @@ int gwm_b200_set_boundary_state(gwm_b200_ctx* c, int member, const gwm_b200_fiel
     long long off = 0;
     for (int f = 0; f < 8; ++f) { M.boff[f] = off; off += strip_len(M.g, kStripOrient[f]); }
     M.boff[8] = off;
-    CK(cudaMalloc(&M.bstrip, 2 * off * sizeof(float)));
+    CK(device_alloc(&M.bstrip, 2 * off * sizeof(float)));
     CK(cudaMemsetAsync(M.bstrip, 0, 2 * off * sizeof(float), c->stream));
     M.bsave = M.bstrip + off;
   }
@@ -1189,14 +1184,14 @@ int gwm_b200_set_boundary_cache(gwm_b200_ctx* c, int member, int n, const int* o
     long long off = 0;
     for (int f = 0; f < 8; ++f) { M.boff[f] = off; off += strip_len(M.g, kStripOrient[f]); }
     M.boff[8] = off;
-    CK(cudaMalloc(&M.bstrip, 2 * off * sizeof(float)));
+    CK(device_alloc(&M.bstrip, 2 * off * sizeof(float)));
     CK(cudaMemsetAsync(M.bstrip, 0, 2 * off * sizeof(float), c->stream));
     M.bsave = M.bstrip + off;
   }
   if (M.bcache_block) { CK(cudaFree(M.bcache_block)); M.bcache_block = nullptr; }
   const size_t snap_bytes = ((size_t)n * M.boff[8] * sizeof(float) + 255) / 256 * 256;
   const size_t off_bytes = ((size_t)n * sizeof(int) + 255) / 256 * 256;
-  CK(cudaMalloc(&M.bcache_block, snap_bytes + off_bytes + sizeof(BoundaryClock)));
+  CK(device_alloc(&M.bcache_block, snap_bytes + off_bytes + sizeof(BoundaryClock)));
   M.bcache = (float*)M.bcache_block;
   M.bcache_off = (int*)(M.bcache_block + snap_bytes);
   M.bclock = (BoundaryClock*)(M.bcache_block + snap_bytes + off_bytes);
@@ -1337,7 +1332,7 @@ int gwm_b200_rain_record(gwm_b200_ctx* c, int member, float* x, float* y, long l
   a.x = x; a.y = y; a.capacity = capacity; a.seed = seed;
   a.p_active = p_active; a.p_inactive = p_inactive;
   unsigned long long* count = nullptr;
-  CK(cudaMallocAsync(&count, sizeof(unsigned long long), c->stream));
+  CK(device_alloc_async(&count, sizeof(unsigned long long), c->stream));
   CK(cudaMemsetAsync(count, 0, sizeof(unsigned long long), c->stream));
   a.count = count;
   CK(launch_rain_record(a, c->stream));
@@ -1359,10 +1354,10 @@ int gwm_b200_mlp_loss_grad(const float* params, const float* norm, const float* 
   double* dl = nullptr;
   auto bad = [&](cudaError_t e) { return e != cudaSuccess; };
   int rc = GWM_B200_OK;
-  if (bad(cudaMalloc(&dp, kMlpParams * 4)) || bad(cudaMalloc(&dn, kMlpNorm * 4)) ||
-      bad(cudaMalloc(&dx, (size_t)n * kMlpIn * 4)) || bad(cudaMalloc(&dy, (size_t)n * kMlpOut * 4)) ||
-      bad(cudaMalloc(&scr, mlp_scratch_floats(n) * 4)) || bad(cudaMalloc(&part, mlp_partial_floats(n) * 4)) ||
-      bad(cudaMalloc(&dg, kMlpParams * 4)) || bad(cudaMalloc(&dl, sizeof(double)))) {
+  if (bad(device_alloc(&dp, kMlpParams * 4)) || bad(device_alloc(&dn, kMlpNorm * 4)) ||
+      bad(device_alloc(&dx, (size_t)n * kMlpIn * 4)) || bad(device_alloc(&dy, (size_t)n * kMlpOut * 4)) ||
+      bad(device_alloc(&scr, mlp_scratch_floats(n) * 4)) || bad(device_alloc(&part, mlp_partial_floats(n) * 4)) ||
+      bad(device_alloc(&dg, kMlpParams * 4)) || bad(device_alloc(&dl, sizeof(double)))) {
     rc = GWM_B200_ERR_CUDA;
   } else {
     cudaMemcpy(dp, params, kMlpParams * 4, cudaMemcpyHostToDevice);
@@ -1400,7 +1395,7 @@ int gwm_b200_mlp_train(const float* x, const float* y, long long n, const gwm_b2
                o_part = place(mlp_partial_floats(batch) * 4), o_l = place(nbatch * sizeof(double)),
                o_idx = place((size_t)n * sizeof(int));
   char* block = nullptr;
-  if (cudaMalloc(&block, total) != cudaSuccess) return GWM_B200_ERR_CUDA;
+  if (device_alloc(&block, total) != cudaSuccess) return GWM_B200_ERR_CUDA;
   auto cleanup = [&](int rc) {
     cudaFree(block);
     return rc;
@@ -1485,7 +1480,7 @@ int gwm_b200_mlp_infer(const float* params, const float* norm, const float* x, f
   surrogate_operands(params, fr.data(), tail.data());
   std::copy(norm, norm + kMlpNorm, tail.begin() + kSurBias);
   char* buf = nullptr;
-  if (cudaMalloc(&buf, 65536 + 256) != cudaSuccess) return GWM_B200_ERR_CUDA;
+  if (device_alloc(&buf, 65536 + 256) != cudaSuccess) return GWM_B200_ERR_CUDA;
   cudaStream_t s = (cudaStream_t)stream;
   bool ok = cudaMemsetAsync(buf + 65536, 0, 256, s) == cudaSuccess &&
             cudaMemcpyAsync(buf, fr.data(), fr.size(), cudaMemcpyHostToDevice, s) == cudaSuccess &&
@@ -1520,7 +1515,7 @@ int gwm_b200_set_rain_surrogate(gwm_b200_ctx* c, int member, const float* params
   if (!params) { M.use_surrogate = false; return GWM_B200_OK; }
   if (!norm || !range || !M.md.moist) return fail(c, GWM_B200_ERR_ARG, "surrogate needs norm, range and a moist member");
   if (!M.sur) {
-    CK(cudaMalloc(&M.sur, 65536 + 256));
+    CK(device_alloc(&M.sur, 65536 + 256));
     CK(cudaMemset(M.sur + 65536, 0, 256));
   }
   static_assert(kSurWeightBytes + (kSurBias + kMlpNorm + kMlpRange) * sizeof(float) <= 65536, "surrogate buffer");
@@ -1583,7 +1578,7 @@ int gwm_b200_tracer_add(gwm_b200_ctx* c, int member, const char* name, const cha
     if (t.name == name) return fail(c, GWM_B200_ERR_ARG, "Tracer already exists in registry");
   const size_t fbytes = ((M.field_elems * sizeof(float) + 255) / 256) * 256;
   char* blk = nullptr;
-  CK(cudaMalloc(&blk, 3 * fbytes));
+  CK(device_alloc(&blk, 3 * fbytes));
   M.extra.push_back(blk);
   CK(cudaMemsetAsync(blk, 0, 3 * fbytes, c->stream));
   Member::Tracer tr;
@@ -1847,7 +1842,7 @@ int gwm_b200_step_host(gwm_b200_ctx* c, const gwm_b200_fields* in, gwm_b200_fiel
     c->io_ev.assign(11, nullptr);
     for (auto& ev : c->io_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
-  if (!M.io_stage) CK(cudaMalloc(&M.io_stage, 8 * owned_max * sizeof(float)));
+  if (!M.io_stage) CK(device_alloc(&M.io_stage, 8 * owned_max * sizeof(float)));
   auto stage = [&](int f) { return M.io_stage + (size_t)f * owned_max; };
   auto count = [&](int f) {
     const int o = orient[f];
@@ -2435,7 +2430,7 @@ int plan_view_fields(gwm_b200_ctx* c, Member& M, int k, int steps, double dt, st
   }
   const size_t plane = (size_t)g.nx * g.ny;
   double* dev = nullptr;
-  CK(cudaMalloc(&dev, (size_t)a.nfields * plane * sizeof(double)));
+  CK(device_alloc(&dev, (size_t)a.nfields * plane * sizeof(double)));
   a.out = dev;
   host.assign((size_t)a.nfields * plane, 0.0);
   cudaError_t e = launch_plan_view(a, c->stream);

@@ -56,7 +56,4 @@ cudaError_t init_tracer_tma();
 // was already applied.
 cudaError_t launch_warm_rain(const RainArgs& a, cudaStream_t s, bool micro = true);
 
-// Gives back the scratch that scalar transport keeps between calls (scalar.cu).
-void trim_scalar_scratch();
-
 }  // namespace gwmb

@@ -16,11 +16,9 @@
 // its golden vectors), written out so that no compiler choice can change them.  The
 // stencil's halo is the periodic image, or zero beyond an open side: what the
 // reference's halo exchange gives its virtual ranks (an absent neighbour sends zeros).
-#include <map>
-#include <mutex>
-
 #include "../../include/gwm_b200.h"
 #include "common.cuh"
+#include "device_memory.cuh"
 #include "physics.cuh"
 #include "stencil.cuh"
 
@@ -106,57 +104,7 @@ __global__ void __launch_bounds__(32 * kSWarps) k_scalar_step(const ScalarStep a
   }
 }
 
-// Scratch of the calls, from a pool of the library per device that keeps up to 256 MB between
-// calls (larger scratch goes back to the device at the next synchronisation): the default
-// pool gives everything back at each call's end, and mapping it again cost more than the
-// steps.  Allocations are stream-ordered, so threads and streams share the pool safely.  What
-// is kept goes back when a context is destroyed or finds no room (trim_scalar_scratch).
-constexpr uint64_t kKeptScratch = 256ull << 20;
-std::mutex pools_lock;
-std::map<int, cudaMemPool_t> pools;
-cudaError_t scratch_alloc(float** p, size_t bytes, cudaStream_t s) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> hold(pools_lock);
-    auto it = pools.find(dev);
-    if (it == pools.end()) {
-      cudaMemPoolProps props{};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      uint64_t keep = kKeptScratch;
-      if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
-          cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-        pools[dev] = pool;
-      else
-        pool = nullptr;
-    } else {
-      pool = it->second;
-    }
-  }
-  if (pool) {
-    e = cudaMallocFromPoolAsync((void**)p, bytes, pool, s);
-    if (e == cudaSuccess || e == cudaErrorMemoryAllocation) return e;
-    cudaGetLastError();  // a pool of a context that is gone (cudaDeviceReset): forget it
-    std::lock_guard<std::mutex> hold(pools_lock);
-    pools.erase(dev);
-  }
-  return cudaMallocAsync((void**)p, bytes, s);
-}
-
 }  // namespace
-
-void trim_scalar_scratch() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
-  std::lock_guard<std::mutex> hold(pools_lock);
-  auto it = pools.find(dev);
-  if (it != pools.end() && cudaMemPoolTrimTo(it->second, 0) != cudaSuccess) cudaGetLastError();
-}
-
 }  // namespace gwmb
 
 extern "C" int gwm_b200_scalar_ssprk3(const gwm_b200_scalar_desc* d, float* q, int nsteps, void* stream) {
@@ -164,11 +112,14 @@ extern "C" int gwm_b200_scalar_ssprk3(const gwm_b200_scalar_desc* d, float* q, i
   if (!d || !q || d->nx <= 0 || d->ny <= 0 || d->nz <= 0 || nsteps < 0 || d->nz > 65535 || !(d->dx > 0.0f) ||
       !(d->dy > 0.0f))
     return GWM_B200_ERR_ARG;
-  if (nsteps == 0) return GWM_B200_OK;
+  if (nsteps == 0) {
+    trim_scratch();
+    return GWM_B200_OK;
+  }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const size_t n = (size_t)d->nx * d->ny * d->nz;
   float* tmp = nullptr;
-  if (scratch_alloc(&tmp, n * sizeof(float), s) != cudaSuccess) return GWM_B200_ERR_CUDA;
+  if (scratch_alloc((void**)&tmp, n * sizeof(float), s) != cudaSuccess) return GWM_B200_ERR_CUDA;
   ScalarStep a{d->nx, d->ny, d->periodic_x, d->periodic_y, d->u_adv, d->v_adv, d->dt, d->dx, d->dy, q, tmp};
   auto mid = [](float x) { return x >= 9.5367431640625e-7f && x <= 1048576.0f; };
   const bool near = mid(d->dx) && mid(d->dy);

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "device_memory.cuh"
 #include "surrogate.cuh"
 
 namespace gwmb {
@@ -407,9 +408,9 @@ cudaError_t launch_rain_record(const RecordArgs& a, cudaStream_t s) {
   if (nb > (1LL << 30)) return cudaErrorInvalidValue;
   unsigned* counts = nullptr;
   unsigned long long* offsets = nullptr;
-  cudaError_t e = cudaMallocAsync(&counts, (size_t)nb * sizeof(unsigned), s);
+  cudaError_t e = device_alloc_async(&counts, (size_t)nb * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
-  e = cudaMallocAsync(&offsets, (size_t)nb * sizeof(unsigned long long), s);
+  e = device_alloc_async(&offsets, (size_t)nb * sizeof(unsigned long long), s);
   if (e != cudaSuccess) { cudaFreeAsync(counts, s); return e; }
   k_rain_record_count<<<(unsigned)nb, kRecThreads, 0, s>>>(a, n, counts);
   k_rain_record_scan<<<1, 1024, 0, s>>>(counts, (int)nb, offsets, a.count);
@@ -422,7 +423,7 @@ cudaError_t launch_rain_record(const RecordArgs& a, cudaStream_t s) {
 
 cudaError_t mlp_column_stats(const float* a, long long n, int d, double* out, double* rng, cudaStream_t s) {
   double* part = nullptr;
-  cudaError_t e = cudaMallocAsync(&part, (size_t)kStatBlocks * d * 4 * sizeof(double), s);
+  cudaError_t e = device_alloc_async(&part, (size_t)kStatBlocks * d * 4 * sizeof(double), s);
   if (e != cudaSuccess) return e;
   k_stats1<<<kStatBlocks, 256, 0, s>>>(a, n, d, part);
   k_stats2<<<1, 32, 0, s>>>(part, kStatBlocks, n, d, out, rng);

@@ -439,8 +439,9 @@ typedef struct {
  * src/dycore/dry_transport.cu:285-325) on q, a device array (nz, ny, nx) in the global
  * owned layout, in place; the arithmetic is the reference's, so results match it bit
  * for bit.  One scratch copy of q is taken for the call from a stream-ordered pool of the
- * library, which keeps up to 256 MB between calls and gives it back when a context is
- * destroyed or finds no room.  stream: cudaStream_t as void* (NULL: the default stream); returns when done. */
+ * library, which keeps up to 256 MB per device between calls.  What is kept goes back when a
+ * context is destroyed, when an allocation of the library finds no room, and at a call with
+ * nsteps = 0.  stream: cudaStream_t as void* (NULL: the default stream); returns when done. */
 int gwm_b200_scalar_ssprk3(const gwm_b200_scalar_desc* desc, float* q, int nsteps, void* stream);
 
 /* ---- host layout helpers (no device work) --------------------------------- */
