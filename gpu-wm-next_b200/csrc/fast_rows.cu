@@ -16,7 +16,7 @@
 //   - p' - p'_ref and rho - rho_ref of a level are formed once and carried up;
 //   - the level sums stay in shared memory until the CTA's end: one atomic per level.
 // 1024 x 1024 x 64: 0.549 ms a substep (0.82 of the copy bandwidth), 0.627 with k_fast_tma's
-// split columns, 0.654 with its whole columns; 517 x 389 x 50: 97 us (100 with a test for the
+// split columns, 0.654 with its whole columns; 517 x 389 x 50: 98 us (100 with a test for the
 // EOS's far form per row instead of one per plane), 116 with k_fast_tma.
 #include <type_traits>
 

@@ -26,7 +26,7 @@
 // issued one plane ahead.
 // Bounds: the chain of a plane (dp/dz, faces, barrier, density, EOS) with 16 warps per SM, and
 // issue; 16 fields of 4 B per cell would take 0.20 ms for 512 x 512 x 80 at the copy bandwidth.
-// There 0.351 ms, 0.465 with every neighbour read from shared memory and no carried values;
+// There 0.346 ms, 0.465 with every neighbour read from shared memory and no carried values;
 // independent warps of four rows as in fast_rows.cu took 0.51 to 0.58 (too few warps in flight
 // for these chains, at 168 registers).
 #include <type_traits>

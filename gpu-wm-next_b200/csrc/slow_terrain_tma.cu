@@ -15,10 +15,11 @@
 // registers); one barrier publishes them, every thread computes its cells and faces, and a second barrier
 // frees the derived planes for the next one (the terrain planes would not fit a CTA pair
 // per SM double-buffered).  The owned columns' metric values (the cell and face inverse
-// layer depths) and the blend partner q0 are per-thread coalesced loads a plane ahead.
+// layer depths) and the blend partner q0 are per-thread coalesced loads at the top of the plane
+// that uses them, so its derive phase covers them.
 // Bounds: issue and the two barriers of a plane, as in the flat stage, whose shared and carried
-// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.684 ms a stage against 0.998 with
-// separate rows, 201 x 163 x 40: 83 us against 119 (27 fields of 4 B per cell at the copy
+// fluxes and shared reciprocals it has.  512 x 512 x 80: 0.68 ms a stage against 1.00 with
+// separate rows, 201 x 163 x 40: 82 us against 119 (27 fields of 4 B per cell at the copy
 // bandwidth: 0.35 ms and 22 us).
 #include <type_traits>
 

@@ -16,9 +16,9 @@
 // chains interleave.  The Y fluxes between its rows are computed once, and the flux out of a
 // plane's top is carried as the next plane's bottom flux.  Bounds: issue, close to HBM (13
 // fields of 4 B per cell take 0.53 ms for 1024 x 1024 x 64, three tracers, at the copy
-// bandwidth): there 0.644 ms a stage, 0.767 with a test per position and the blend decided at
+// bandwidth): there 0.640 ms a stage, 0.767 with a test per position and the blend decided at
 // run time, 1.045 with two rows eight apart per thread, 426 instructions per cell and a block
-// barrier per plane; 517 x 389 x 50 0.115 ms, 0.141, 0.191.
+// barrier per plane; 517 x 389 x 50 0.113 ms, 0.141, 0.191.
 #include <type_traits>
 
 #include "physics.cuh"
@@ -139,10 +139,11 @@ __global__ void __launch_bounds__(tt::NT, tt::MIN_CTAS)
     }
     near = near && fp::finite(sum);
   };
+  // each quotient tested on its own: rare, so a call (128 x 128 x 64: 27 us a stage, 30 inlined)
   auto mix_each = [&](const float* st, int b, float* q) {
-    const float rr = fmaxf(st[O_RHO + b], 1.0e-6f), y = fp::recip(rr);
+    const float rr = fmaxf(st[O_RHO + b], 1.0e-6f);
 #pragma unroll
-    for (int t = 0; t < N; ++t) q[t] = fp::quotient(st[O_Q + t * Q_STRIDE + b], rr, y);
+    for (int t = 0; t < N; ++t) q[t] = fp::quotient_far(st[O_Q + t * Q_STRIDE + b], rr);
   };
   auto mix = [&](const float* st, int b, float* q) {
     bool near = true;
