@@ -60,3 +60,43 @@ def test_tails_of_tracers(gwm, terrain, low, high):
     a, b = (_step_with(gwm, grid, spec, state, rows, lambda m: m.advance_passive_tracers_ssprk3()) for rows in (16, 3))
     for k in a:
         np.testing.assert_array_equal(b[k], a[k], err_msg=k)
+
+
+# Cells beyond the EOS's series, infinite and not-a-number values and tracers that overflow: the
+# kernels' tests for their general forms, each in one cell of an otherwise ordinary state and all
+# together.
+ODD = {"warm": ("rho_theta", 1.2), "cold": ("rho_theta", 0.8), "dense": ("rho", 40.0), "inf_theta": ("rho_theta", np.inf),
+       "nan_u": ("u", np.nan), "inf_w": ("w", np.inf), "huge_v": ("v", 3.0e38), "inf_qr": ("qr", np.inf),
+       "huge_qc": ("qc", 3.0e38), "nan_qv": ("qv", np.nan)}
+
+
+@pytest.mark.parametrize("periodic", [True, False])
+@pytest.mark.parametrize("terrain", [False, True])
+@pytest.mark.parametrize("odd", [*ODD, "all"])
+def test_odd_cells(gwm, odd, terrain, periodic):
+    nx, ny, nz = 70, 53, 11
+    hill = None
+    if terrain:
+        hill = gwm.build_terrain("cosine_mountain", nx, ny, 1000.0, 1000.0, height=300.0, half_width_x=0.3,
+                                 half_width_y=0.3)
+    flat = gwm.GridSpec(nx, ny, nz, dx=1000.0, dy=1000.0, z_top=300.0 * nz)
+    grid = gwm.GridSpec(nx, ny, nz, dx=1000.0, dy=1000.0, z_top=300.0 * nz, terrain=hill, periodic_x=periodic,
+                        periodic_y=periodic)
+    state = gwm.build_case("moist_sounding", flat, gwm.CaseParams(theta_ref=300.0, noise_rms_k=0.5, seed=3,
+                                                                  relative_humidity=1.01), moist=True)
+    rng = np.random.default_rng(8)
+    for k in ("qc", "qr"):
+        state[k] = (state["rho"] * rng.uniform(0.0, 1e-3, state["rho"].shape)).astype(np.float32)
+    for n, name in enumerate(ODD if odd == "all" else [odd]):
+        field, value = ODD[name]
+        at = (1 + 3 * n % 9, 7 + 4 * n, 13 + 5 * n)  # n <= 9: inside
+        if np.isfinite(value) and value < 100.0:
+            state[field][at] *= np.float32(value)
+        else:
+            state[field][at] = np.float32(value)
+    state["precip"] = np.zeros((ny, nx))
+    spec = gwm.MemberSpec(step=gwm.StepConfig(dt=0.5, fast_substeps=3),
+                          rain=gwm.WarmRainConfig(dt=0.5, rain_terminal_velocity=12.0), moist=True)
+    a, b = (_step_with(gwm, grid, spec, state, rows) for rows in (16, 3))
+    for k in a:
+        np.testing.assert_array_equal(b[k], a[k], err_msg=k)
