@@ -167,11 +167,12 @@ def load_peaks():
     return 6650.0, "fallback"
 
 
-# Algorithmic bytes of one acoustic substep per cell (the dominant kernel): the
-# hot-path byte model counts 12 FP32 field accesses per cell per substep
-# (rho, theta, three momenta and three base momenta read; rho and three momenta
-# written).
-SUBSTEP_ALGO_BYTES_PER_CELL = 12 * 4
+# Algorithmic bytes of one acoustic substep per cell (the dominant kernel), an inner one:
+# rho, theta and three momentum increments in, rho and three increments out; on the TMA-fed
+# tiles p' in and out besides.  (The hot-path byte model, without increments, counts 12
+# accesses: three base momenta more, no p'.)
+def substep_bytes_per_cell(tile):
+    return 4 * (11 if tile in (3, 4) else 9)
 
 
 # CPU sample per step: the per-cell cost of the CPU restatement does not depend on the
@@ -477,14 +478,15 @@ def substep_roofline(model, g, stream, torch, steps=2):
         model.set_tile("fast_substep", 4)
     cells = g.nx * g.ny * g.nz
     fast = rep["k_fast_substep"]
-    achieved = SUBSTEP_ALGO_BYTES_PER_CELL * cells / (fast["avg_ms"] * 1e-3) / 1e9
     total = sum(v["total_ms"] for v in rep.values())
     shares = {k: round(v["total_ms"] / total, 4) for k, v in rep.items()}
     fast_tile = 3 if tile == 4 else tile  # the kernel whose launches were timed
+    nbytes = substep_bytes_per_cell(fast_tile) * cells
+    achieved = nbytes / (fast["avg_ms"] * 1e-3) / 1e9
     kname = {0: "k_fast_flat", 3: "k_fast_rows"}.get(fast_tile, f"k_fast_substep<{fast_tile}>")
     return {"bound": "hbm", "achieved": achieved, "unit": "GB/s", "traffic": read_traffic(g, fast_tile),
             "kernel": f"{kname} (one acoustic substep)",
-            "algorithmic_bytes_per_launch": SUBSTEP_ALGO_BYTES_PER_CELL * cells,
+            "algorithmic_bytes_per_launch": nbytes,
             "avg_launch_ms": fast["avg_ms"], "kernel_shares": shares,
             "kernel_avg_ms": {k: round(v["avg_ms"], 4) for k, v in rep.items()}}
 
